@@ -33,24 +33,12 @@ namespace cdd {
 // sign of both when they agree and its magnitude is never below the smaller of theirs (also after
 // rounding: fl(a + c) / 2 >= min(a, c) for a, c > 0), so the 3-way minmod equals the 2-way one:
 // min(|a|, |c|) with their common sign, 0 when the signs differ or one is zero. That is the median
-// of (a, c, 0); FP32 forms it with four min/max operations and no compares or selects:
-// max(min(a, c), min(max(a, c), 0)) (both positive: min(a, c); both negative: max(a, c); else 0).
-// FP64 keeps the compare-and-select form.
-__device__ __forceinline__ float minmod2(float a, float c) {
-    return fmaxf(fminf(a, c), fminf(fmaxf(a, c), 0.0f));
-}
-__device__ __forceinline__ double minmod2(double a, double c) {
-    const double m = fmin(fabs(a), fabs(c));
-    const bool pos = (a > 0.0) & (c > 0.0);
-    const bool neg = (a < 0.0) & (c < 0.0);
-    return pos ? m : (neg ? -m : 0.0);
-}
+// of (a, c, 0), which FP32 forms with min / max operations (minmod_pair); FP64, which has none, folds
+// the 0 into the factor 1/2 of the derivative (limited_f64).
 
-// 1/sqrt and division: FP32 uses the hardware approximations (<= 2 ulp), FP64 exact ones.
+// 1/sqrt and division of the FP32 form: the hardware approximations (<= 2 ulp).
 __device__ __forceinline__ float inv_sqrt(float x) { return rsqrtf(x); }
-__device__ __forceinline__ double inv_sqrt(double x) { return 1.0 / sqrt(x); }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
-__device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
 
 // Shared-memory tiles of the 2.5-D march: a block owns TXS x TYS cells of a plane (last axis x
 // contiguous) and walks along axis 0 (3-D). Each staged plane holds all 9 components of a box of
@@ -150,20 +138,6 @@ __device__ __forceinline__ void minmod_pair(float e0, float em1, float em2, floa
     const float lo = fminf(em1, 0.0f), hi = fmaxf(em1, 0.0f);
     dd0 = fminf(fmaxf(e0, lo), hi);
     ddm = fminf(fmaxf(em2, lo), hi);
-}
-__device__ __forceinline__ void minmod_pair(double e0, double em1, double em2, double& dd0, double& ddm) {
-    dd0 = minmod2(e0, em1);
-    ddm = minmod2(em1, em2);
-}
-
-template <typename T>
-__device__ __forceinline__ void derivs5(const T* v, T ih, T& up, T& um) {
-    const T dm2 = v[1] - v[0], dm1 = v[2] - v[1], d0 = v[3] - v[2], d1 = v[4] - v[3];
-    const T e0 = d1 - d0, em1 = d0 - dm1, em2 = dm1 - dm2;
-    T dd0, ddm;
-    minmod_pair(e0, em1, em2, dd0, ddm);
-    up = (d0 - (T)0.5 * dd0) * ih;
-    um = (dm1 + (T)0.5 * ddm) * ih;
 }
 
 // ---- FP32 flux with paired arithmetic ----
@@ -474,6 +448,228 @@ __device__ __forceinline__ void flux_f32(const TileView<float, ND>& tv, float ih
     }
 }
 
+// ---- FP64 flux ----
+// The scalar counterpart of flux_f32, with the same regrouping of the rhs per one-sided derivative.
+// The derivatives are undivided (times Dx): the velocities are ratios of two forms of the same degree in
+// them, so only the ME terms take Dx^2 and the rhs the one factor 1 / Dx.
+// Bound by the FP64 pipe (64 lanes per SM and clock: about 930 of its instructions per cell, 0.9 ms at 256^3) and
+// by 8 resident warps per SM to hide its latency. All 54 derivatives stay in registers (246, no spills), formed
+// once: forming them again for the rhs, with the five-compare minmod, 8 square roots and 8 + 4 divisions
+// of the form before it, took 4272 us per 256^3 flux, this 2704 us; with the plane copies under the cell's own
+// work (march) and 20 planes per block, 1796 us.
+// d + h minmod(e, m) for h = -1/2 or 1/2: the factor is 0 unless the signs of e and m agree (an integer test),
+// and times the smaller magnitude otherwise, so the FP64 pipe sees one compare and one multiply-add. A NaN in
+// e (two cells away) leaves m, as minmod's 0 leaves d: only the cells whose d or m is NaN become NaN.
+__device__ __forceinline__ double limited_f64(double d, double e, double m, double h) {
+    const double v = fabs(e) < fabs(m) ? e : m;
+    const bool same = (__double2hiint(e) ^ __double2hiint(m)) >= 0;
+    return fma(__hiloint2double(same ? __double2hiint(h) : 0, 0), v, d);
+}
+// (u+, u-) times Dx from u_{-2} .. u_{+2}.
+__device__ __forceinline__ void derivs5_f64(const double* v, double& up, double& um) {
+    const double dm2 = v[1] - v[0], dm1 = v[2] - v[1], d0 = v[3] - v[2], d1 = v[4] - v[3];
+    const double e0 = d1 - d0, em1 = d0 - dm1, em2 = dm1 - dm2;
+    up = limited_f64(d0, e0, em1, -0.5);
+    um = limited_f64(dm1, em2, em1, 0.5);
+}
+
+// meh: ME Dx^2. ring_read(): called once the thread has read all it needs of the ring but its cell's own
+// values; false (a plane did not arrive) ends the cell. Returns false then.
+template <int ND, bool GLIDE, class F>
+__device__ __forceinline__ bool flux_f64(const TileView<double, ND>& tv, double ih, double meh, const double (&S)[3][3],
+                                         bool lam_on, bool glide, double Lambda, double (&rhs)[9], double& spd,
+                                         const F& ring_read) {
+    constexpr int NC = 1 << ND;
+    constexpr int NP = (ND == 3) ? 3 : 1;
+    double U[ND][2][9];   // u+_d, u-_d of component c = 3 l + j, times Dx
+    const double str = lam_on ? (S[0][0] + S[1][1] + S[2][2]) / 3.0 * Lambda : 0.0;
+
+    // A_d l = sum_j (u_d)_lj S_dj (the d-th less sum_{l,j} (u_d)_lj S_lj), P_d = sum_{l != d, j} (u_d)_lj^2, one
+    // axis after the other as its derivatives are formed
+    double A[ND][2][3], Pq[ND][2], Cp[NP][2][2];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            Pq[d][s] = 0.0;
+#pragma unroll
+            for (int l = 0; l < 3; ++l) A[d][s][l] = 0.0;
+        }
+#pragma unroll
+        for (int c = 0; c < 9; ++c) {
+            const int l = c / 3, j = c - 3 * l;
+            double v5[5];
+            tv.load5(c, d, v5);
+            derivs5_f64(v5, U[d][0][c], U[d][1][c]);
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                const double u = U[d][s][c];
+                A[d][s][l] = fma(u, S[d][j], A[d][s][l]);
+                A[d][s][d] = fma(-u, S[l][j], A[d][s][d]);
+                if (l != d) Pq[d][s] = fma(u, u, Pq[d][s]);
+            }
+        }
+        if (lam_on) {
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                A[d][s][d] = fma(str, U[d][s][0] + U[d][s][4] + U[d][s][8], A[d][s][d]);
+#pragma unroll
+                for (int l = 0; l < 3; ++l) A[d][s][l] = fma(-str, U[d][s][3 * l + d], A[d][s][l]);
+            }
+        }
+    }
+    if (!ring_read()) return false;
+    // pair terms C_de[s_d][s_e] = sum_j (u_d)_ej (u_e)_dj
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                const int d = p, e = (p + 1) % 3;
+                double t = 0.0;
+#pragma unroll
+                for (int j = 0; j < 3; ++j) t = fma(U[d % ND][a][3 * e + j], U[e % ND][b][3 * d + j], t);
+                Cp[p][a][b] = t;
+            }
+
+    // corners: V = (A_x[sx] + A_y[sy] (+ A_z[sz])) / |rho|
+    double V[NC][3];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const int sx = (c >> (ND - 1)) & 1, sy = (c >> (ND - 2)) & 1;
+        const int sz = (ND == 3) ? (c & 1) : 0;
+        double r2 = fma(-2.0, Cp[0][sx][sy], meh + Pq[0][sx] + Pq[1][sy]);
+        if (ND == 3) r2 = fma(-2.0, Cp[1 % NP][sy][sz] + Cp[2 % NP][sz][sx], r2 + Pq[2 % ND][sz]);
+        const double inv = rsqrt(r2);
+        double av[3];
+#pragma unroll
+        for (int l = 0; l < 3; ++l) {
+            av[l] = A[0][sx][l] + A[1][sy][l];
+            if (ND == 3) av[l] += A[2 % ND][sz][l];
+        }
+        if (GLIDE && glide) {
+            // glide-only projection (CentralUpwindHJBetaPGlideOnlyDynamics.py L152-201, 2-D L96-129):
+            // g_d = tr(u_d) - sum_e (u_e)_{d e}, v += g (ME + v.g) / (ME + g.g), then v / |rho|
+            const int sgc[3] = {sx, sy, sz};
+            double gv[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                double Dd = 0.0;
+#pragma unroll
+                for (int e = 0; e < ND; ++e) Dd += U[e][sgc[e]][3 * d + e];
+                const double tr = (d < ND) ? U[d % ND][sgc[d]][0] + U[d % ND][sgc[d]][4] + U[d % ND][sgc[d]][8] : 0.0;
+                gv[d] = tr - Dd;
+            }
+            const double rr = meh + gv[0] * gv[0] + gv[1] * gv[1] + gv[2] * gv[2];
+            const double rv = meh + av[0] * gv[0] + av[1] * gv[1] + av[2] * gv[2];
+            const double f = rv / rr;
+#pragma unroll
+            for (int l = 0; l < 3; ++l) av[l] = fma(gv[l], f, av[l]);
+        }
+#pragma unroll
+        for (int l = 0; l < 3; ++l) V[c][l] = av[l] * inv;
+    }
+    // one-sided speeds a+_d = max(0, max V_d), a-_d = -min(0, min V_d); each axis' weights are divided by its
+    // total a+_d + a-_d + ME. A NaN in V is dropped by the compares and carried to the speed by vsum.
+    double pp[ND], pm[ND], wm[ND], wp[ND];
+    double vsum = 0.0;
+    spd = 0.0;
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+        double mx = 0.0, mn = 0.0;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            mx = V[c][d] > mx ? V[c][d] : mx;
+            mn = V[c][d] < mn ? V[c][d] : mn;
+            vsum += V[c][d];
+        }
+        pp[d] = mx;
+        pm[d] = -mn;
+        const double tot = pp[d] + pm[d] + ME;
+        spd += tot;
+        const double it = 1.0 / tot;
+        wm[d] = pm[d] * it;
+        wp[d] = pp[d] * it;
+    }
+    if (vsum != vsum) spd = vsum;
+
+    // Q^s_dl = sum over corners with s_d = s of w_c V_cl
+    double Q[ND][2][3];
+    {
+        double w[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            w[c] = ((c >> (ND - 1)) & 1) ? wp[0] : wm[0];
+#pragma unroll
+            for (int d = 1; d < ND; ++d) w[c] *= ((c >> (ND - 1 - d)) & 1) ? wp[d] : wm[d];
+        }
+#pragma unroll
+        for (int l = 0; l < 3; ++l) {
+            double T[NC];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) T[c] = w[c] * V[c][l];
+            if constexpr (ND == 3) {
+                const double y0 = T[0] + T[1], y1 = T[2] + T[3], y2 = T[4] + T[5], y3 = T[6] + T[7];   // by (sx, sy)
+                Q[0][0][l] = y0 + y1;
+                Q[0][1][l] = y2 + y3;
+                Q[1][0][l] = y0 + y2;
+                Q[1][1][l] = y1 + y3;
+                Q[2 % ND][0][l] = (T[0] + T[2]) + (T[4] + T[6]);
+                Q[2 % ND][1][l] = (T[1] + T[3]) + (T[5] + T[7]);
+            } else {
+                Q[0][0][l] = T[0] + T[1];
+                Q[0][1][l] = T[2 % NC] + T[3 % NC];
+                Q[1][0][l] = T[0] + T[2 % NC];
+                Q[1][1][l] = T[1] + T[3 % NC];
+            }
+        }
+    }
+
+    // rhs_ij = sum_d [(c_d - Q+_dd) (u+_d)_ij + (-c_d - Q-_dd) (u-_d)_ij] + [i < ND] sum_{s,l} Q^s_il (u^s_i)_lj,
+    // c_d = a+_d a-_d / tot_d
+    double G[ND][2];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+        G[d][0] = fma(pm[d], wp[d], -Q[d][0][d]);
+        G[d][1] = -fma(pm[d], wp[d], Q[d][1][d]);
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            double acc = 0.0;
+#pragma unroll
+            for (int d = 0; d < ND; ++d)
+#pragma unroll
+                for (int s = 0; s < 2; ++s) acc = fma(G[d][s], U[d][s][3 * i + j], acc);
+            if (i < ND) {
+#pragma unroll
+                for (int s = 0; s < 2; ++s)
+#pragma unroll
+                    for (int l = 0; l < 3; ++l) acc = fma(Q[i % ND][s][l], U[i % ND][s][3 * l + j], acc);
+            }
+            rhs[3 * i + j] = acc * ih;
+        }
+    if (lam_on) {
+        // the Lambda trace term enters H_ii: rhs_ii -= J, J = -Lambda/3 sum_{d,s} [Q^s_dd tr(u_d) - sum_l Q^s_dl (u_d)_ld]
+        double Jp = 0.0;
+#pragma unroll
+        for (int d = 0; d < ND; ++d)
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                Jp = fma(Q[d][s][d], U[d][s][0] + U[d][s][4] + U[d][s][8], Jp);
+#pragma unroll
+                for (int l = 0; l < 3; ++l) Jp = fma(-Q[d][s][l], U[d][s][3 * l + d], Jp);
+            }
+        const double J = -Lambda / 3.0 * Jp * ih;
+        rhs[0] -= J;
+        rhs[4] -= J;
+        rhs[8] -= J;
+    }
+    return true;
+}
+
 template <typename T>
 __device__ __forceinline__ T block_reduce_max(T v, T* red) {
 #pragma unroll
@@ -514,6 +710,7 @@ struct StageConst {
     double dt;
     double cnu;   // nu / (1 + nu) of the elastic energy density (|sigma|^2 - cnu tr^2) / (4 mu)
     float cnu_f;  // the same rounded to FP32 (the FP32 form's per-cell density)
+    double meh;   // ME Dx^2 (FP64)
     bool active;
 };
 
@@ -527,6 +724,7 @@ __device__ __forceinline__ StageConst stage_const(const InstDev& I, const InstCl
     k.dt = ck.dt;
     k.cnu = I.nu / (1.0 + I.nu);
     k.cnu_f = (float)k.cnu;
+    k.meh = ME * I.h * I.h;
     k.active = ck.active != 0;
     return k;
 }
@@ -581,24 +779,19 @@ template <> struct Stage1Acc<float> {
 // ssm: this thread's 6 shared-memory stress slots (component c at ssm[c * ST_THREADS]), filled by
 // asynchronous copies issued one cell earlier; sig_next: the stress of the thread's cell in the
 // next plane (its copies are issued as soon as this cell's values are read), or null; acc: this
-// thread's FP64 sum slots (FP32 stage 1).
-template <typename T, int ND, int MODE, int VAR>
+// thread's FP64 sum slots (FP32 stage 1); kc: the block's constants, in shared memory; early() is
+// called once the stress slots are free (FP32), ring_read() as in flux_f64 (FP64).
+template <typename T, int ND, int MODE, int VAR, class FE, class FR>
 __device__ __forceinline__ void stencil_cell(const InstDev& I, const CellCtx<T>& cx, bool valid,
-                                             const TileView<T, ND>& tv,
-                                             const StageConst& kc_block, const InstClock& ck, double t_flux,
+                                             const TileView<T, ND>& tv, const StageConst& kc,
                                              Stage1Acc<T>& sums, double* acc,
                                              const T* __restrict__ sig0, const T* __restrict__ vac,
-                                             T* ssm, const T* sig_next) {
+                                             T* ssm, const T* sig_next, const FE& early, const FR& ring_read) {
     // compile-time variant: bit 0 carries the glide-only projection, bit 1 the vacancy term
     constexpr bool GLIDE = (VAR & 1) != 0;
     constexpr bool VAC = (VAR & 2) != 0;
     const T ih = cx.ih;
     const long long cells = cx.cells;
-    // FP32 reads the block's stage constants from shared memory; FP64 (no registers to spare across
-    // the march) re-derives them per cell
-    StageConst kc_cell;
-    if constexpr (sizeof(T) == 8) kc_cell = stage_const<MODE>(I, ck, t_flux);
-    const StageConst& kc = (sizeof(T) == 8) ? kc_cell : kc_block;
     // beta_n of the stage update is loaded after the flux (no registers to hold it across; FP32
     // requested its rows into L2 one plane ahead)
     constexpr bool UPD = (MODE == M_STAGE2 || MODE == M_STAGE3);
@@ -615,6 +808,7 @@ __device__ __forceinline__ void stencil_cell(const InstDev& I, const CellCtx<T>&
             for (int c = 0; c < 6; ++c) cp_async_elem(ssm + c * st_threads<T>(), sig_next + c * cells);
             cp_async_commit();
         }
+        early();
         if (MODE == M_STAGE1 && valid) {
             // observables of the step-start state: elastic energy of the internal stress (k_dt
             // applies 1 / (4 mu) to the instance sum). FP32 forms the cell's density in FP32 (its
@@ -655,258 +849,7 @@ __device__ __forceinline__ void stencil_cell(const InstDev& I, const CellCtx<T>&
     if constexpr (sizeof(T) == 4) {
         flux_f32<ND, GLIDE>(tv, ih, S, cx.lam_on, GLIDE && cx.glide, (float)I.Lambda, rhs, spd);
     } else {
-        const bool lam_on = cx.lam_on;
-        const bool glide = GLIDE && cx.glide;   // glide-only dynamics (Lambda is 0 then)
-        const T str = lam_on ? (S[0][0] + S[1][1] + S[2][2]) / (T)3 * (T)I.Lambda : (T)0;
-
-        // ---------------- pass 1: A, P, C, trace ----------------
-        T A[ND][2][3], Sd[ND][2], Pq[ND][2], trU[ND][2];
-        constexpr int NP = (ND == 3) ? 3 : 1;
-        T Cp[NP][2][2];
-#pragma unroll
-        for (int d = 0; d < ND; ++d)
-#pragma unroll
-            for (int s = 0; s < 2; ++s) {
-                Sd[d][s] = 0; Pq[d][s] = 0; trU[d][s] = 0;
-#pragma unroll
-                for (int l = 0; l < 3; ++l) A[d][s][l] = 0;
-            }
-#pragma unroll
-        for (int p = 0; p < NP; ++p)
-#pragma unroll
-            for (int a = 0; a < 2; ++a)
-#pragma unroll
-                for (int b = 0; b < 2; ++b) Cp[p][a][b] = 0;
-
-        // the 54 one-sided derivatives are recomputed from shared memory in each pass (register
-        // budget)
-        T Dv[GLIDE ? ND : 1][2][3];   // glide-only: (u_e)_{d e} per axis e and sign
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            T U[ND][2][3];
-#pragma unroll
-            for (int l = 0; l < 3; ++l) {
-#pragma unroll
-                for (int d = 0; d < ND; ++d) {
-                    T v5[5];
-                    tv.load5(3 * l + j, d, v5);
-                    derivs5(v5, ih, U[d][0][l], U[d][1][l]);
-                }
-            }
-            T Sj[3], Sdj[3];
-#pragma unroll
-            for (int l = 0; l < 3; ++l) { Sj[l] = (j == 0) ? S[l][0] : ((j == 1) ? S[l][1] : S[l][2]); }
-#pragma unroll
-            for (int d = 0; d < ND; ++d) Sdj[d] = (j == 0) ? S[d][0] : ((j == 1) ? S[d][1] : S[d][2]);
-#pragma unroll
-            for (int d = 0; d < ND; ++d)
-#pragma unroll
-                for (int s = 0; s < 2; ++s) {
-#pragma unroll
-                    for (int l = 0; l < 3; ++l) {
-                        T v = U[d][s][l];
-                        A[d][s][l] += v * Sdj[d];
-                        Sd[d][s] += v * Sj[l];
-                        if (l != d) Pq[d][s] += v * v;
-                    }
-                    if (lam_on || glide) {
-                        // trace of u_d (components (j, j))
-                        T dj = (j == 0) ? U[d][s][0] : ((j == 1) ? U[d][s][1] : U[d][s][2]);
-                        trU[d][s] += dj;
-                    }
-                    if (lam_on && j == d) {
-                        // the -str (u_d)_{l d} terms
-#pragma unroll
-                        for (int l = 0; l < 3; ++l) A[d][s][l] -= str * U[d][s][l];
-                    }
-                }
-            if constexpr (GLIDE) {
-                if (glide && j < ND) {
-#pragma unroll
-                    for (int s = 0; s < 2; ++s)
-#pragma unroll
-                        for (int l = 0; l < 3; ++l) Dv[j % ND][s][l] = U[j % ND][s][l];
-                }
-            }
-            // pair terms C_de[s_d][s_e] = sum_j (u_d)_ej (u_e)_dj
-#pragma unroll
-            for (int a = 0; a < 2; ++a)
-#pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                    Cp[0][a][b] += U[0][a][1] * U[1][b][0];
-                    if (ND == 3) {
-                        Cp[1 % NP][a][b] += U[1 % ND][a][2] * U[2 % ND][b][1];
-                        Cp[2 % NP][a][b] += U[2 % ND][a][0] * U[0][b][2];
-                    }
-                }
-        }
-#pragma unroll
-        for (int d = 0; d < ND; ++d)
-#pragma unroll
-            for (int s = 0; s < 2; ++s) {
-                T ad = (d == 0) ? A[d][s][0] : ((d == 1) ? A[d][s][1] : A[d][s][2]);
-                ad -= Sd[d][s];
-                if (lam_on) ad += str * trU[d][s];
-                if (d == 0) A[d][s][0] = ad; else if (d == 1) A[d][s][1] = ad; else A[d][s][2] = ad;
-            }
-
-        // ---------------- corners: V, speeds, weights, Q ----------------
-        constexpr int NC = 1 << ND;
-        T V[NC][3];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            const int sx = (c >> (ND - 1)) & 1, sy = (c >> (ND - 2)) & 1;
-            const int sz = (ND == 3) ? (c & 1) : 0;
-            T rho2;
-            if (ND == 3)
-                rho2 = (T)ME + Pq[0][sx] + Pq[1][sy] + Pq[2 % ND][sz]
-                       - (T)2 * (Cp[0][sx][sy] + Cp[1 % NP][sy][sz] + Cp[2 % NP][sz][sx]);
-            else
-                rho2 = (T)ME + Pq[0][sx] + Pq[1][sy] - (T)2 * Cp[0][sx][sy];
-            T inv = inv_sqrt(rho2);
-            T av[3];
-#pragma unroll
-            for (int l = 0; l < 3; ++l) {
-                T a = A[0][sx][l] + A[1][sy][l];
-                if (ND == 3) a += A[2 % ND][sz][l];
-                av[l] = a;
-            }
-            if (glide) {
-                // glide-only projection (CentralUpwindHJBetaPGlideOnlyDynamics.py L152-201, 2-D L96-129):
-                // g_d = tr(u_d) - sum_e (u_e)_{d e}, v += g (ME + v.g) / (ME + g.g), then v / |rho|
-                const int sgc[3] = {sx, sy, sz};
-                T gv[3];
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    T Dd = (T)0;
-#pragma unroll
-                    for (int e = 0; e < ND; ++e) {
-                        if constexpr (GLIDE) Dd += Dv[e][sgc[e]][d];
-                    }
-                    const T tr = (d < ND) ? trU[d % ND][sgc[d]] : (T)0;
-                    gv[d] = tr - Dd;
-                }
-                const T rr = (T)ME + gv[0] * gv[0] + gv[1] * gv[1] + gv[2] * gv[2];
-                const T rv = (T)ME + av[0] * gv[0] + av[1] * gv[1] + av[2] * gv[2];
-                const T f = fdiv(rv, rr);
-#pragma unroll
-                for (int l = 0; l < 3; ++l) av[l] += gv[l] * f;
-            }
-#pragma unroll
-            for (int l = 0; l < 3; ++l) V[c][l] = av[l] * inv;
-        }
-        T pp[ND], pm[ND], tot[ND];
-        T vsum = 0;   // NaN anywhere in V (fmax/fmin would drop it) must reach the CFL maximum
-#pragma unroll
-        for (int d = 0; d < ND; ++d) {
-            T mx = (T)0, mn = (T)0;
-#pragma unroll
-            for (int c = 0; c < NC; ++c) { mx = fmax(mx, V[c][d]); mn = fmin(mn, V[c][d]); vsum += V[c][d]; }
-            pp[d] = mx;
-            pm[d] = -mn;
-            tot[d] = pp[d] + pm[d] + (T)ME;
-        }
-        // the reference's order: the upwind weights a-_d, a+_d are divided by a_tot b_tot c_tot at
-        // the end (the FP32 form, flux_f32, normalises each axis first)
-        T wm[ND], wp[ND];
-#pragma unroll
-        for (int d = 0; d < ND; ++d) {
-            wm[d] = pm[d];
-            wp[d] = pp[d];
-        }
-        T Q[ND][2][3];
-#pragma unroll
-        for (int d = 0; d < ND; ++d)
-#pragma unroll
-            for (int s = 0; s < 2; ++s)
-#pragma unroll
-                for (int l = 0; l < 3; ++l) Q[d][s][l] = 0;
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            int sg[3];
-            sg[0] = (c >> (ND - 1)) & 1;
-            sg[1] = (c >> (ND - 2)) & 1;
-            sg[2] = (ND == 3) ? (c & 1) : 0;
-            T w = (T)1;
-#pragma unroll
-            for (int d = 0; d < ND; ++d) w *= (sg[d] == 0) ? wm[d] : wp[d];
-#pragma unroll
-            for (int l = 0; l < 3; ++l) {
-                T wv = w * V[c][l];
-#pragma unroll
-                for (int d = 0; d < ND; ++d) Q[d][sg[d]][l] += wv;
-            }
-        }
-        const T inv_abc = fdiv((T)1, ND == 3 ? tot[0] * tot[1] * tot[2 % ND] : tot[0] * tot[1]);
-        T coef[ND];
-#pragma unroll
-        for (int d = 0; d < ND; ++d) coef[d] = fdiv(pm[d] * pp[d], tot[d]);
-        spd = tot[0] + tot[1];
-        if (ND == 3) spd += tot[2 % ND];
-        if (vsum != vsum) spd = vsum;
-
-        // ---------------- pass 2: rhs ----------------
-        T Jp = 0;   // Lambda trace term, J = -Lambda/3 * Jp
-        if (lam_on) {
-#pragma unroll
-            for (int d = 0; d < ND; ++d)
-#pragma unroll
-                for (int s = 0; s < 2; ++s) {
-                    T qdd = (d == 0) ? Q[d][s][0] : ((d == 1) ? Q[d][s][1] : Q[d][s][2]);
-                    Jp += qdd * trU[d][s];
-                }
-        }
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            T U[ND][2][3];
-#pragma unroll
-            for (int l = 0; l < 3; ++l) {
-#pragma unroll
-                for (int d = 0; d < ND; ++d) {
-                    T v5[5];
-                    tv.load5(3 * l + j, d, v5);
-                    derivs5(v5, ih, U[d][0][l], U[d][1][l]);
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                T hs = 0, vis = 0;
-#pragma unroll
-                for (int d = 0; d < ND; ++d) {
-                    T gp = (d == 0) ? Q[d][0][0] : ((d == 1) ? Q[d][0][1] : Q[d][0][2]);
-                    T gm = (d == 0) ? Q[d][1][0] : ((d == 1) ? Q[d][1][1] : Q[d][1][2]);
-                    hs += gp * U[d][0][i] + gm * U[d][1][i];
-                    vis += (U[d][0][i] - U[d][1][i]) * coef[d];
-                }
-                if (i < ND) {
-#pragma unroll
-                    for (int s = 0; s < 2; ++s)
-#pragma unroll
-                        for (int l = 0; l < 3; ++l) hs -= Q[i % ND][s][l] * U[i % ND][s][l];
-                }
-                T r = -hs * inv_abc + vis;
-                if (j == 0) { if (i == 0) rhs[0] = r; else if (i == 1) rhs[3] = r; else rhs[6] = r; }
-                else if (j == 1) { if (i == 0) rhs[1] = r; else if (i == 1) rhs[4] = r; else rhs[7] = r; }
-                else { if (i == 0) rhs[2] = r; else if (i == 1) rhs[5] = r; else rhs[8] = r; }
-            }
-            if (lam_on) {
-#pragma unroll
-                for (int d = 0; d < ND; ++d) {
-                    if (d != j) continue;
-#pragma unroll
-                    for (int s = 0; s < 2; ++s)
-#pragma unroll
-                        for (int l = 0; l < 3; ++l) Jp -= Q[d][s][l] * U[d][s][l];
-                }
-            }
-        }
-        if (lam_on) {
-            // the trace term enters H_ii, so rhs_ii gets -J / (a_tot b_tot c_tot)
-            T J = -(T)I.Lambda / (T)3 * Jp;
-            rhs[0] -= J * inv_abc;
-            rhs[4] -= J * inv_abc;
-            rhs[8] -= J * inv_abc;
-        }
+        if (!flux_f64<ND, GLIDE>(tv, ih, kc.meh, S, cx.lam_on, GLIDE && cx.glide, I.Lambda, rhs, spd, ring_read)) return;
     }
 
     // ---------------- outputs ----------------
@@ -948,80 +891,72 @@ __device__ __forceinline__ void stencil_cell(const InstDev& I, const CellCtx<T>&
 
 // The plane box of a stencil tile: RX x RY cells from (x0 - OX, y0 - 2) of the instance's field
 // (component c at src + c * cells), wrapped periodically.
+// Kept in shared memory, like StageConst, so that nothing of it stays in registers across the march.
 template <typename T> struct BoxGeomT {
     const T* src;
     long long cells;
-    int x0, y0, nX, nY;
+    int x0, y0, nX, nY, nZ, zr;   // zr: the grid plane of relative index 0
+    int chunk;                    // elements per copy
+    __device__ __forceinline__ int plane_of(int pr) const {
+        int z = zr + pr;
+        while (z < 0) z += nZ;
+        while (z >= nZ) z -= nZ;
+        return z;
+    }
 };
-template <typename T>
-__device__ __forceinline__ void stage_box(T* dst, const BoxGeomT<T>& g, int zp, bool all) {
-    constexpr int RX = TileGeom<T>::RX, OX = TileGeom<T>::OX, PP = tile_pp<T>(), ST_THREADS = st_threads<T>();
-    const T* sp0 = g.src + (long long)zp * g.nY * g.nX;
-    for (int e = threadIdx.x; e < 9 * PP; e += ST_THREADS) {
-        const int c = e / PP;
-        const int r = e - c * PP;
-        const int iy = r / RX, ix = r - iy * RX;
-        int yy = g.y0 - 2 + iy, xx = g.x0 - OX + ix;
-        if (!all && yy >= 0 && yy < g.nY && xx >= 0 && xx < g.nX) continue;
+// CH consecutive elements global -> shared (4 to 16 bytes), asynchronously.
+template <int BYTES> __device__ __forceinline__ void cp_async_chunk(void* dst, const void* src) {
+    if constexpr (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(smem_addr(dst)), "l"(src), "n"(BYTES) : "memory");
+}
+// Box of plane zp by asynchronous copies of CH elements, all in flight at once; the block's threads walk
+// the box's rows (component, y) with a fixed column each. CH divides nX, x0 and OX, so a chunk never
+// crosses the periodic boundary. The caller commits the group.
+template <typename T, int CH>
+__device__ __forceinline__ void box_async_ch(T* dst, const BoxGeomT<T>& g, int zp) {
+    constexpr int RX = TileGeom<T>::RX, OX = TileGeom<T>::OX, RY = tile_ry<T>();
+    constexpr int CPR = RX / CH, RS = st_threads<T>() / CPR;   // chunks per row, rows per sweep
+    const int r0 = threadIdx.x / CPR, col = (threadIdx.x - r0 * CPR) * CH;
+    if (r0 >= RS) return;
+    int xx = g.x0 - OX + col;
+    while (xx < 0) xx += g.nX;
+    while (xx >= g.nX) xx -= g.nX;
+    const T* sp = g.src + (long long)zp * g.nY * g.nX + xx;
+#pragma unroll 1
+    for (int r = r0; r < 9 * RY; r += RS) {
+        const int c = r / RY, iy = r - c * RY;
+        int yy = g.y0 - 2 + iy;
         while (yy < 0) yy += g.nY;
         while (yy >= g.nY) yy -= g.nY;
-        while (xx < 0) xx += g.nX;
-        while (xx >= g.nX) xx -= g.nX;
-        dst[e] = __ldg(sp0 + c * g.cells + (long long)yy * g.nX + xx);
+        cp_async_chunk<CH * (int)sizeof(T)>(dst + r * RX + col, sp + c * g.cells + yy * g.nX);
     }
 }
-// Patch after a TMA copy: only the box's out-of-grid cells, i.e. its columns outside [xl, xr) (all
-// rows) and its rows outside [yl, yr) (the in-grid columns). Tiles with more than 8 such columns or
-// 4 such rows (grids narrower than a tile) scan the whole box.
+// The widest chunk that the row length and the field's address allow (grids are even, tiles start at
+// multiples of 4 or at nX - 32): 16 bytes, 8 bytes (FP32 rows of 4 k + 2 values), one value.
+template <typename T> __device__ __forceinline__ int box_chunk(const T* src, int nX) {
+    const uintptr_t a = (uintptr_t)src | (uintptr_t)nX * sizeof(T);
+    return (a & 15) == 0 ? 16 / (int)sizeof(T) : ((a & 7) == 0 ? 8 / (int)sizeof(T) : 1);
+}
 template <typename T>
-__device__ __forceinline__ void patch_box_edges(T* dst, const BoxGeomT<T>& g, int zp) {
-    constexpr int RX = TileGeom<T>::RX, OX = TileGeom<T>::OX, PP = tile_pp<T>(), RY = tile_ry<T>();
-    constexpr int ST_THREADS = st_threads<T>();
-    const int x0 = g.x0, y0 = g.y0, nX = g.nX, nY = g.nY, tid = threadIdx.x;
-    const int xl = max(0, OX - x0), xr = max(xl, min(RX, nX - x0 + OX));
-    const int yl = max(0, 2 - y0), yr = max(yl, min(RY, nY - y0 + 2));
-    const int nxo = xl + (RX - xr), nyo = yl + (RY - yr);
-    if (nxo > 8 || nyo > 4) { stage_box<T>(dst, g, zp, false); return; }
-    const T* sp0 = g.src + (long long)zp * nY * nX;
-    auto put = [&](int c, int iy, int ix) {
-        int yy = y0 - 2 + iy, xx = x0 - OX + ix;
-        if (yy < 0) yy += nY;
-        if (yy >= nY) yy -= nY;
-        if (xx < 0) xx += nX;
-        if (xx >= nX) xx -= nX;
-        dst[c * PP + iy * RX + ix] = __ldg(sp0 + c * g.cells + (long long)yy * nX + xx);
-    };
-    if (nxo > 0) {
-        for (int e = tid; e < 9 * RY * 8; e += ST_THREADS) {
-            const int c = e / (RY * 8), r = e - c * (RY * 8), iy = r >> 3, j = r & 7;
-            if (j < nxo) put(c, iy, j < xl ? j : xr + (j - xl));
-        }
-    }
-    if (nyo > 0) {
-        for (int e = tid; e < 9 * 4 * RX; e += ST_THREADS) {
-            const int c = e / (4 * RX), r = e - c * (4 * RX), q = r / RX, ix = r - q * RX;
-            if (q < nyo && ix >= xl && ix < xr) put(c, q < yl ? q : yr + (q - yl), ix);
-        }
-    }
-}
-
-// Out-of-line copies: FP64 calls these (its march is at the 255-register limit, and keeping the
-// rarely run staging code out of it removes most of its spills: 22.3 -> 21.7 ms per 256^3 step);
-// FP32 inlines them (out of line measured 3% slower there).
-template <typename T> __device__ __noinline__ void stage_box_ool(T* dst, BoxGeomT<T> g, int zp, bool all) {
-    stage_box<T>(dst, g, zp, all);
-}
-template <typename T> __device__ __noinline__ void patch_box_edges_ool(T* dst, BoxGeomT<T> g, int zp) {
-    patch_box_edges<T>(dst, g, zp);
+__device__ __forceinline__ void box_async(T* dst, const BoxGeomT<T>& g, int zp) {
+    const int chunk = g.chunk;
+    if (chunk == 16 / (int)sizeof(T)) box_async_ch<T, 16 / (int)sizeof(T)>(dst, g, zp);
+    else if (sizeof(T) == 4 && chunk == 2) box_async_ch<T, 2>(dst, g, zp);
+    else box_async_ch<T, 1>(dst, g, zp);
 }
 
 // One block: a TXS x TYS tile of planes [z0, z0 + zc) (3-D) or of the single plane (2-D).
-// The 3-D ring holds planes z-2 .. z+2 of all 9 components of beta_s (NS slots). With TMA
-// (I.tma_slot >= 0) one 5-D bulk-tensor copy stages a whole plane box (2-D: the one plane) from
-// the tensor map of the instance's run of same-shape instances; coordinates outside the
-// grid read zeros, and tiles whose box crosses the periodic boundary patch those cells with
-// wrapped loads after the copy lands. FP32 (6 slots) prefetches plane z+3 while computing z;
-// FP64 (5 slots) refills the slot of z-2 after computing z. Otherwise threads load the box.
+// The 3-D ring holds planes z-2 .. z+2 of all 9 components of beta_s (NS slots). A tile whose box lies
+// inside the grid stages a plane by one 5-D bulk-tensor copy from the tensor map of its instance's run of
+// same-shape instances (I.tma_slot >= 0); the others, and those without a map, by asynchronous 16-byte (or
+// narrower) copies with wrapped addresses (box_async). (A TMA copy of an edge tile would need its
+// out-of-grid cells patched once it has landed, by loads whose latency nothing hides: 30% of the FP64 flux
+// at 128^3, where half of the tiles are at an edge.)
+// FP32 (6 slots) requests plane z+3 as cell z starts. FP64 (5 slots, two blocks of 110 KB) requests it into the
+// slot of plane z-2 once the whole block has formed its derivatives, so the copy runs under the
+// corner and rhs work of the same cell; that barrier also collects the verdict of the bounded waits.
 template <typename T, int ND, int MODE, int VAR>
 __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, double* red, uint64_t* bars,
                                       const StencilMapSet& maps,
@@ -1056,64 +991,44 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
     const long long cells = I.cells;
     const long long plane = (long long)nY * nX;
     const T* src = bs + I.foff;
-    const bool use_tma = maps.enabled && (I.tma_slot >= 0);
     const bool edge = (x0 - OX < 0) || (x0 - OX + RX > nX) || (y0 - 2 < 0) || (y0 - 2 + RY > nY);
+    const bool use_tma = maps.enabled && (I.tma_slot >= 0) && !edge;
 
-    auto wrapz = [&](int z) { while (z < 0) z += nZ; while (z >= nZ) z -= nZ; return z; };
-    // Fill (all = true) or patch the out-of-grid cells (all = false) of the box of plane zp; the
-    // patch after a TMA copy visits only the box's out-of-grid cells (edge tiles).
-    const BoxGeomT<T> bg{src, cells, x0, y0, nX, nY};
-    auto load_box = [&](int slot, int zp, bool all) {
-        if constexpr (sizeof(T) == 8) stage_box_ool<T>(sm + slot * 9 * PP, bg, zp, all);
-        else stage_box<T>(sm + slot * 9 * PP, bg, zp, all);
-    };
-    auto patch_box = [&](int slot, int zp) {
-        if constexpr (sizeof(T) == 8) patch_box_edges_ool<T>(sm + slot * 9 * PP, bg, zp);
-        else patch_box_edges<T>(sm + slot * 9 * PP, bg, zp);
-    };
+    __shared__ StageConst kc;   // read per cell from shared memory (keeps registers free)
+    __shared__ BoxGeomT<T> bg;
+    if (tid == 0) {
+        kc = stage_const<MODE>(I, clk[ii], t_flux);
+        bg = {src, cells, x0, y0, nX, nY, nZ, ND == 3 ? z0 - 2 : 0, box_chunk<T>(src, nX)};
+    }
+    __syncthreads();
     // plane with relative index pr (= z - (z0 - 2)) lives in slot pr % NS
-    auto issue = [&](int pr) {
+    auto issue = [&](int pr) {   // TMA, one thread
         const int slot = pr % NS;
         mbar_expect_tx(&bars[slot], PLANE_BYTES);
-        tma_load_5d(sm + slot * 9 * PP, &maps.m[I.tma_slot], &bars[slot], x0 - OX, y0 - 2,
-                    wrapz(z0 - 2 + pr), 0, I.tma_sub);
+        tma_load_5d(sm + slot * 9 * PP, &maps.m[I.tma_slot], &bars[slot], bg.x0 - OX, bg.y0 - 2,
+                    bg.plane_of(pr), 0, I.tma_sub);
     };
-    int ok = 1;
-    auto arrive = [&](int pr) {   // wait for plane pr and patch it; block-uniform result in ok
-        if (!ok) return;
-        const int slot = pr % NS;
-        bool got = mbar_wait(&bars[slot], (uint32_t)((pr / NS) & 1));
-        if (__syncthreads_or(!got)) {
-            ok = 0;
-            if (tid == 0) atomicOr(status, (int)ST_TIMEOUT);
-            return;
-        }
-        if (edge) patch_box(slot, wrapz(z0 - 2 + pr));
+    auto stage = [&](int pr) {   // asynchronous copies, all threads
+        box_async<T>(sm + (pr % NS) * 9 * PP, bg, bg.plane_of(pr));
+        cp_async_commit();
     };
+    auto landed = [&](int pr) { return mbar_wait(&bars[pr % NS], (uint32_t)((pr / NS) & 1)); };
 
+    constexpr int NPL = (ND == 3) ? 5 : 1;   // planes z0-2 .. z0+2 (3-D), the plane (2-D)
     int issued = -1;   // highest plane index handed to TMA
+    int ok = 1;        // block-uniform: every plane waited for has arrived
     if (use_tma) {
         if (tid == 0) {
 #pragma unroll 1
             for (int s = 0; s < NS; ++s) mbar_init(&bars[s], 1);
             fence_mbar_init();
-        }
-        __syncthreads();
-        constexpr int NPL = (ND == 3) ? 5 : 1;   // planes z0-2 .. z0+2 (3-D), the plane (2-D)
-        if (tid == 0)
             for (int pr = 0; pr < NPL; ++pr) issue(pr);
+        }
         issued = NPL - 1;
-#pragma unroll 1
-        for (int pr = 0; pr < NPL; ++pr) arrive(pr);
-    } else if (ND == 3) {
-#pragma unroll 1
-        for (int q = 0; q < 5; ++q) load_box(q, wrapz(z0 - 2 + q), true);
     } else {
-        load_box(0, 0, true);
+#pragma unroll 1
+        for (int pr = 0; pr < NPL; ++pr) stage(pr);
     }
-    __shared__ StageConst kc;   // FP32: read per cell from shared memory (keeps registers free)
-    if (sizeof(T) == 4 && tid == 0) kc = stage_const<MODE>(I, clk[ii], t_flux);
-    __syncthreads();
     Stage1Acc<T> sums;
     // FP32: this thread's FP64 sum slots after the stress slots
     double* acc = reinterpret_cast<double*>(sm + NS * 9 * PP + 6 * ST_THREADS) + tid;
@@ -1141,21 +1056,45 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
 #pragma unroll
     for (int c = 0; c < 6; ++c) cp_async_elem(ssm + c * ST_THREADS, cx.sig + c * cells);
     cp_async_commit();
+    // the first planes: the barrier makes the barriers' initialisation, kc and the staged copies visible
+    if (!use_tma) cp_async_wait_own();
+    __syncthreads();
+    bool got = true;   // this thread saw every plane of the coming cell arrive
+    if (use_tma) {
 #pragma unroll 1
-    for (int z = z0, k = 0; ok && z < z1; ++z, ++k) {
+        for (int pr = 0; pr < NPL; ++pr) got &= landed(pr);
+    }
+    // FP32 stage updates read beta_n of their cell after the flux (no registers to hold it across): its rows
+    // of the next plane are requested into L2 a plane ahead, one 128-byte row of 32 cells per thread for
+    // the first 9 TYS threads of tiles inside the grid
+    const bool ahead = nX >= TXS && nY >= TYS && tid < 9 * TYS;
+#pragma unroll 1
+    for (int z = z0, k = 0; z < z1; ++z, ++k) {
         const bool more = (z + 1 < z1);
-        if (use_tma && NS == 6 && more && tid == 0) {
-            fence_proxy_async();
-            issue(k + 5);
-        }
-        if (use_tma && NS == 6 && more) issued = k + 5;
+        // collects the waits' verdict; every thread has read the planes it needs
+        auto verdict = [&]() {
+            if (__syncthreads_or(!got)) {
+                ok = 0;
+                if (tid == 0) atomicOr(status, (int)ST_TIMEOUT);
+            }
+            return ok != 0;
+        };
+        auto request = [&]() {   // plane k + 5
+            if (use_tma) {
+                if (tid == 0) {
+                    fence_proxy_async();
+                    issue(k + 5);
+                }
+                issued = k + 5;
+            } else {
+                stage(k + 5);
+            }
+        };
+        if (NS != 5 && use_tma && !verdict()) break;
+        if (NS == 6 && use_tma && more) request();
         if (ND == 3) {
-            // ring planes z-2 .. z+2 live in slots (k + q) mod NS: FP32 rotates them by one plane
-            // per step; FP64 (no registers to spare across the march) recomputes them
-            if (NS != 6) {
-#pragma unroll
-                for (int q = 0; q < 5; ++q) tv.so[q] = ((k + q) % NS) * 9 * PP;
-            } else if (k == 0) {
+            // ring planes z-2 .. z+2 live in slots (k + q) mod NS, rotated by one plane per step
+            if (k == 0) {
 #pragma unroll
                 for (int q = 0; q < 5; ++q) tv.so[q] = q * 9 * PP;
             } else {
@@ -1166,47 +1105,45 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
         } else {
             tv.so[2] = 0;
         }
-        // FP32 stage updates read beta_n of their cell after the flux (no registers to hold it
-        // across): its rows of the next plane are requested into L2 now, one 128-byte row of 32
-        // cells per thread for the first 9 TYS threads (TMA-staged tiles lie inside the grid)
         if constexpr (sizeof(T) == 4 && (MODE == M_STAGE2 || MODE == M_STAGE3)) {
-            if (use_tma && more && tid < 9 * TYS) {
+            if (ahead && more) {
                 const int c = tid / TYS, r = tid - c * TYS;
                 prefetch_l2(cx.bn + c * cells + plane + (long long)(r - ty) * nX - tx);
             }
         }
-        stencil_cell<T, ND, MODE, VAR>(I, cx, own, tv, kc, clk[ii], t_flux, sums, acc, sig, vac, ssm,
-                                       more ? cx.sig + plane : nullptr);
+        auto early = [&]() {   // FP32: the staged copies of plane k + 5, after the stress copies' wait
+            if (NS == 6 && !use_tma && more) stage(k + 5);
+        };
+        auto ring_read = [&]() {   // FP64
+            if (NS != 5) return true;
+            if (use_tma) {
+                if (!verdict()) return false;
+            } else if (more) {
+                __syncthreads();
+            }
+            if (more) request();
+            return true;
+        };
+        stencil_cell<T, ND, MODE, VAR>(I, cx, own, tv, kc, sums, acc, sig, vac, ssm,
+                                       more ? cx.sig + plane : nullptr, early, ring_read);
+        if (!ok) break;
         cx.sig += plane;
         if (cx.bn) cx.bn += plane;
         cx.out += plane;
         if (cx.spd) cx.spd += plane;
         if (ND == 3 && more) {
             if (use_tma) {
-                if (NS == 5) {
-                    __syncthreads();
-                    if (tid == 0) {
-                        fence_proxy_async();
-                        issue(k + 5);
-                    }
-                    issued = k + 5;
-                }
-                arrive(k + 5);
+                got = landed(k + 5);
             } else {
+                cp_async_wait_own();
                 __syncthreads();
-                load_box((k + 5) % NS, wrapz(z + 3), true);   // plane pr = k + 5 lives in slot pr % NS
             }
-            // arrive's block-wide vote already orders this cell's reads before the next copy into
-            // the ring; a barrier is left only for plain shared-memory stores (edge patches, thread
-            // staging) to become visible
-            if (!use_tma || edge) __syncthreads();
         }
     }
-    cp_async_wait_own();   // no stress copy in flight past here
+    cp_async_wait_own();   // no copy in flight past here
     if (!ok) {
         // a copy did not land in time: let every copy this block issued finish (bounded), then leave
-        for (int pr = max(0, issued - NS + 1); pr <= issued; ++pr)
-            mbar_wait(&bars[pr % NS], (uint32_t)((pr / NS) & 1));
+        for (int pr = max(0, issued - NS + 1); pr <= issued; ++pr) landed(pr);
         return;
     }
     if (MODE == M_STAGE1) {
