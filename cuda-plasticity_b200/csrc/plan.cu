@@ -179,12 +179,14 @@ int build_shapes(cdd_plan* p, size_t elt) {
     std::vector<int> pre_plane(1, 0), pre_rest[NUM_PASSES];
     for (int k = 0; k < NUM_PASSES; ++k) pre_rest[k].push_back(0);
     size_t smem_plane = 0;
-    int optin_dev = 0;
+    int optin_dev = 0, sms = 0;
     {
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&optin_dev, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     }
+    const int st_planes = stencil_default_planes(p->inst.data(), n, C.precision, 2 * (sms > 0 ? sms : 148));   // 2 blocks per SM
     for (int i = 0; i < n; ++i) {
         InstDev& I = p->inst[i];
         // rows kernels (R2C: 9 components, C2R: 6); ping-pong buffers of P padded rows
@@ -276,7 +278,7 @@ int build_shapes(cdd_plan* p, size_t elt) {
             for (int k = 0; k < NUM_PASSES; ++k) pre_rest[k].push_back(pre_rest[k].back() + (I.plane ? 0 : I.tile[k].blocks));
             if (I.plane && plane_smem_bytes(I) > smem_plane) smem_plane = plane_smem_bytes(I);
         }
-        stencil_geometry(I, C.precision, p->tune[i].stencil_planes);
+        stencil_geometry(I, C.precision, p->tune[i].stencil_planes > 0 ? p->tune[i].stencil_planes : st_planes);
         // effective launch shapes of this instance
         p->tune[i].rows_lines = I.tile[PASS_R2C].lines;
         p->tune[i].mid_cols = (I.nd == 3) ? I.tile[PASS_MID_F].lines : 0;

@@ -1549,28 +1549,50 @@ size_t stencil_smem_bytes(int precision, bool any3d) {
     return ((size_t)(any3d ? TileGeom<double>::NS : 1) * 9 * tile_pp<double>() + 6 * st_threads<double>()) * sizeof(double);
 }
 
-// Blocks of the stencil: (x, y) tiles times chunks of planes along axis 0. Built-in rule: about
-// 227K threads in all (1776 blocks of 128 threads, 888 of 256) but at least 8 planes per block (each
-// block first stages a 4-plane halo, so shorter chunks spend most of their time on it); planes > 0
-// sets the chunk length.
-void stencil_geometry(InstDev& I, int precision, int planes) {
-    const int nZ = (I.nd == 3) ? I.n0 : 1;
+static int stencil_tiles(const InstDev& I, int precision) {
     const int nY = (I.nd == 3) ? I.n1 : I.n0;
     const int nX = (I.nd == 3) ? I.n2 : I.n1;
     const int TYS = precision == CDD_F32 ? TileGeom<float>::TY : TileGeom<double>::TY;
-    const int tiles = ((nX + TXS - 1) / TXS) * ((nY + TYS - 1) / TYS);
+    return ((nX + TXS - 1) / TXS) * ((nY + TYS - 1) / TYS);
+}
+
+// Planes per block (one value for all 3-D instances of a plan). A block costs its planes and about c0 = 0.9
+// planes' time for staging the first five (flux form at 256^3, planes per block 1 / 2 / 4 / 8 / 16: FP64 3456 /
+// 2561 / 2110 / 1900 / 1815 us, FP32 1589 / 1176 / 983 / 894 / 863 us); `resident` blocks run at once. Many
+// short blocks pay c0 often, few long ones leave SMs idle (small grids) or a long tail: the sum of both
+// estimates is minimised. At least 8 planes per block whatever the grid, the rule before, gave one 32^3 FP64
+// flux 32 blocks and 50 us, against 25 us at one plane per block.
+int stencil_default_planes(const InstDev* insts, int n, int precision, int resident) {
+    const double c0 = 0.9;
+    int best = 1;
+    double best_cost = 1e300;
+    for (int z = 1; z <= 64; ++z) {
+        double sum = 0.0, longest = 0.0, blocks = 0.0;
+        for (int i = 0; i < n; ++i) {
+            const int nZ = (insts[i].nd == 3) ? insts[i].n0 : 1, len = z < nZ ? z : nZ;
+            const double b = (double)stencil_tiles(insts[i], precision) * ((nZ + len - 1) / len);
+            blocks += b;
+            sum += b * c0 + (double)stencil_tiles(insts[i], precision) * nZ;
+            if (len + c0 > longest) longest = len + c0;
+        }
+        const double cost = blocks <= resident ? longest : sum / resident + 0.5 * longest;
+        if (cost <= best_cost) { best_cost = cost; best = z; }
+    }
+    return best;
+}
+
+// Blocks of the stencil: (x, y) tiles times chunks of `planes` planes along axis 0.
+void stencil_geometry(InstDev& I, int precision, int planes) {
+    const int nZ = (I.nd == 3) ? I.n0 : 1;
     int chunks = 1;
     if (I.nd == 3) {
-        const int target = 1776 * 4 / TYS;
-        chunks = (target + tiles - 1) / tiles;
-        if (chunks > nZ / 8) chunks = nZ / 8;
-        if (planes > 0) chunks = (nZ + planes - 1) / planes;
+        chunks = (nZ + planes - 1) / planes;
         if (chunks > nZ) chunks = nZ;
         if (chunks < 1) chunks = 1;
     }
     I.st_zc = (nZ + chunks - 1) / chunks;
     chunks = (nZ + I.st_zc - 1) / I.st_zc;
-    I.stencil_blocks = tiles * chunks;
+    I.stencil_blocks = stencil_tiles(I, precision) * chunks;
 }
 
 }  // namespace cdd
