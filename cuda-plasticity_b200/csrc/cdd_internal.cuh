@@ -49,6 +49,9 @@ struct LinePlan {
     FDiv ns[MAX_STAGES];   // stage st: span of the finished sub-transforms (product of earlier radices)
     int twst[MAX_STAGES];  // stage st: offset (even, complex elements) of its twiddle rows
     int twspan;            // elements from twst[0] to the end of the last stage's rows
+    // two-pass form (see pass_stages): n = A B, pass A the first sa stages, pass B the others; pa, pb index
+    // CDD_PASS_A / CDD_PASS_B (0: no such form)
+    int pa, pb, sa, A, B;
 };
 
 // Radix rounded up to even: the length of one twiddle row (pairs load as one 16-byte vector).
@@ -178,7 +181,31 @@ __host__ __device__ inline bool rows_io_plan(const LinePlan& lp, int P) {
     if ((P * a) % 32 != 0 || (P * b) % 32 != 0) return false;
     return (a == 16 && (b == 16 || b == 8 || b == 4)) || (a == 8 && b == 4);
 }
-__host__ __device__ inline int rows_buffers(const LinePlan& lp, int P) { return rows_io_plan(lp, P) ? 1 : 2; }
+// Elements of a row pass's line buffer: one padded line of a register-resident plan; one line of B groups of
+// A + 1 of a two-pass plan (A is even: the odd pitch spreads a pass's accesses over the banks) and, for the
+// FP32 form, two FP64 partial row sums per group; else two padded lines (ping-pong stages).
+__host__ __device__ inline int rows_elems(const LinePlan& lp, int P, int velt) {
+    if (!rows_io_plan(lp, P) && lp.pa) return P * lp.B * (lp.A + 1 + (velt == 8 ? 2 : 0));
+    return (rows_io_plan(lp, P) ? 1 : 2) * P * (lp.n + (lp.n >> 4) + 1);
+}
+// Line pairs per block and threads of the row passes. 4096 (FP32) or 2048 (FP64) values per block; small
+// grids take fewer lines, down to two blocks per SM (24^3 FP32: 11 blocks and 28 us before, see rows_lines
+// in the plan), in the multiples that the register-resident form needs.
+inline int rows_lines(const LinePlan& lp, long long npairs, int velt) {
+    const int full = (velt == 8 ? 4096 : 2048) / lp.n;
+    int step = 1;
+    while (step < 8 && lp.nst == 2 && !rows_io_plan(lp, step)) step *= 2;
+    if (!rows_io_plan(lp, step)) step = 1;
+    long long P = lp.pa ? npairs / (2 * 148) / step * step : full;
+    if (P < step) P = step;
+    if (P > full) P = full;
+    if (P < 1) P = 1;
+    return (int)(P > npairs ? npairs : P);
+}
+inline int rows_threads(const LinePlan& lp, int P, int velt) {
+    const int big = lp.pa ? (lp.A > lp.B ? lp.A : lp.B) : lp.n / 4;
+    return (velt == 8 && P * big > 192) ? 256 : 128;
+}
 
 // Per-pass tiling of one instance (host-chosen, read by the kernels).
 struct PassTile {
@@ -670,18 +697,15 @@ __device__ __forceinline__ void fft_io_c(const LIn& in, const SColT<V, K>& x, co
     }
 }
 
-// The compile-time radix sequences of at least two stages (make_line_plan with the default largest
-// radix 16 for 32..512 and 48, 96, 192, 24).
+// The compile-time radix sequences of two stages (make_line_plan with the default largest radix 16 for 32..256,
+// 24 and 48).
 #define CDD_IO_SEQS(X)                                  \
     X(nst == 2 && r0 == 16 && r1 == 16, 16, 16)         \
     X(nst == 2 && r0 == 16 && r1 == 8, 16, 8)           \
     X(nst == 2 && r0 == 16 && r1 == 4, 16, 4)           \
     X(nst == 2 && r0 == 8 && r1 == 4, 8, 4)             \
-    X(nst == 3 && r0 == 16 && r1 == 8 && r2 == 4, 16, 8, 4) \
     X(nst == 2 && r0 == 16 && r1 == 3, 16, 3)           \
-    X(nst == 2 && r0 == 8 && r1 == 3, 8, 3)             \
-    X(nst == 3 && r0 == 8 && r1 == 4 && r2 == 3, 8, 4, 3)   \
-    X(nst == 3 && r0 == 16 && r1 == 4 && r2 == 3, 16, 4, 3)
+    X(nst == 2 && r0 == 8 && r1 == 3, 8, 3)
 
 // True when lp runs through fft_io (the host sizes shared memory with this).
 __host__ __device__ inline bool line_plan_io(const LinePlan& lp) {
@@ -714,8 +738,8 @@ __device__ __forceinline__ bool fft_io(const LIn& in, const SColT<V, K>& x, cons
 
 // Run all stages of `lp` on the lines of `lay`, starting in buffer a (b is scratch of the same
 // layout). Returns the buffer that holds the result. Every thread of the block must call this.
-// The radix sequences that make_line_plan gives the usual lengths (16 to 512, and 24, 48, 96, 192
-// with the default largest radix 16) run the compile-time stages; others the general engine.
+// 16, 512 and 1024 (largest radix 16) run compile-time stages, others the general engine; lengths with a two-pass
+// form do not come here.
 template <typename V, bool INV, typename Lay>
 __device__ __forceinline__ V* fft_lines_g(V* a, V* b, const Lay& lay, const LinePlan& lp,
                                           const V* __restrict__ twbase, int tid, int nt, int rebase);
@@ -726,16 +750,9 @@ __device__ __forceinline__ V* fft_lines(V* a, V* b, const Lay& lay, const LinePl
     const int nst = lp.nst, r0 = lp.radix[0], r1 = lp.radix[1], r2 = lp.radix[2];
 #define CDD_SEQ(COND, ...) \
     if (COND) return fft_lines_c<V, INV, Lay, 1, __VA_ARGS__>(a, b, lay, lp, twbase, tid, nt, rebase, 0);
-    CDD_SEQ(nst == 2 && r0 == 16 && r1 == 16, 16, 16)
-    CDD_SEQ(nst == 2 && r0 == 16 && r1 == 8, 16, 8)
-    CDD_SEQ(nst == 2 && r0 == 16 && r1 == 4, 16, 4)
-    CDD_SEQ(nst == 2 && r0 == 8 && r1 == 4, 8, 4)
     CDD_SEQ(nst == 3 && r0 == 16 && r1 == 8 && r2 == 4, 16, 8, 4)
+    CDD_SEQ(nst == 3 && r0 == 16 && r1 == 16 && r2 == 4, 16, 16, 4)
     CDD_SEQ(nst == 1 && r0 == 16, 16)
-    CDD_SEQ(nst == 2 && r0 == 16 && r1 == 3, 16, 3)
-    CDD_SEQ(nst == 2 && r0 == 8 && r1 == 3, 8, 3)
-    CDD_SEQ(nst == 3 && r0 == 8 && r1 == 4 && r2 == 3, 8, 4, 3)
-    CDD_SEQ(nst == 3 && r0 == 16 && r1 == 4 && r2 == 3, 16, 4, 3)
 #undef CDD_SEQ
     return fft_lines_g<V, INV>(a, b, lay, lp, twbase, tid, nt, rebase);
 }
@@ -762,6 +779,85 @@ __device__ __forceinline__ V* fft_lines_g(V* a, V* b, const Lay& lay, const Line
     }
     return src;
 }
+
+// ------------------------------------------------------------------------------------------
+// Two-pass transforms. A line of length n = A B runs in two passes over shared memory instead of one per
+// stage: a pass runs consecutive stages of the plan on the values a thread holds in registers.
+// Pass A (j < B): elements j + B q, q < A, stages 0 .. sa - 1, results m < A to j A + m of the Stockham
+// order; pass B (m < A): elements m + A q, q < B, the other stages, results X[m + A r]. Same codelets,
+// twiddle rows and operation order as one stage after the other, so the same bits.
+// ------------------------------------------------------------------------------------------
+// Stages st, st + 1, ... (radices R, Rest...) on v[0 .. R M), the digit of stage st on top; jm: the index of
+// the finished sub-transforms (span ns). The result with digits b_st, b_st+1, ... is left at slot
+// b_st M + ...; pass_out gives its output index b_st + R b_st+1 + ....
+template <int... Rs> struct PassOut;
+template <int R> struct PassOut<R> { static constexpr int of(int slot) { return slot; } };
+template <int R, int R1, int... Rest> struct PassOut<R, R1, Rest...> {
+    static constexpr int M = RadixProd<R1, Rest...>::v;
+    static constexpr int of(int slot) { return slot / M + R * PassOut<R1, Rest...>::of(slot % M); }
+};
+template <typename V, bool INV, bool FIRST, int R, int... Rest>
+__device__ __forceinline__ void pass_stages(V* v, const LinePlan& lp, const V* __restrict__ tws, int st, int jm, int ns) {
+    constexpr int M = RadixProd<Rest...>::v;
+    V w[R];
+    if constexpr (!FIRST) load_tw_row<R>(tws + (lp.twst[st] - lp.twst[0]) + jm * tw_row(R), w);
+#pragma unroll
+    for (int b = 0; b < M; ++b) {
+        V x[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const V a = v[r * M + b];
+            if constexpr (FIRST) x[r] = a;
+            else x[r] = (r == 0) ? a : (INV ? vmulc(a, w[r]) : vmul(a, w[r]));
+        }
+        dft<R, V, INV>(x);
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r * M + b] = x[r];
+    }
+    if constexpr (M > 1) {
+#pragma unroll
+        for (int b = 0; b < R; ++b)
+            pass_stages<V, INV, false, Rest...>(v + b * M, lp, tws, st + 1, jm + ns * b, ns * R);
+    }
+}
+
+// The passes: code, then radices. A: first stages of a plan, B: last ones. Every length 2^a 3^b or 2^a 5^c
+// that make_line_plan's default radices split into one of each (24 to 500 but for 288 and 512, whose (8, 4)
+// = 32 values spill; not the single-stage lengths 4, 8, 16). The BIG ones hold more than 16 values.
+#define CDD_PASS_A_SMALL(X) X(1, 2) X(2, 4) X(3, 8) X(4, 16) X(5, 2, 3) X(6, 4, 3) X(7, 2, 5)
+#define CDD_PASS_A_BIG(X) X(8, 8, 3) X(9, 2, 3, 3) X(10, 4, 5)
+#define CDD_PASS_B_SMALL(X) X(1, 3) X(2, 4) X(3, 8) X(4, 16) X(5, 5) X(6, 3, 3) X(7, 4, 3)
+#define CDD_PASS_B_BIG(X) X(8, 8, 3) X(9, 5, 5) X(10, 3, 3, 3) X(11, 4, 5)
+
+// Host: the split of lp with the smallest larger pass, if it has one.
+inline void set_two_pass(LinePlan& lp) {
+    lp.pa = lp.pb = lp.sa = lp.A = lp.B = 0;
+    auto same = [&lp](int s0, int s1, const std::vector<int>& r) {
+        if ((int)r.size() != s1 - s0) return false;
+        for (int i = s0; i < s1; ++i)
+            if (lp.radix[i] != r[i - s0]) return false;
+        return true;
+    };
+    int best = 1 << 30;
+    for (int s = 1; s < lp.nst; ++s) {
+        int a = 0, b = 0, A = 1, B = 1;
+        for (int i = 0; i < lp.nst; ++i) (i < s ? A : B) *= lp.radix[i];
+#define CDD_TRY_A(C, ...) if (same(0, s, {__VA_ARGS__})) a = C;
+#define CDD_TRY_B(C, ...) if (same(s, lp.nst, {__VA_ARGS__})) b = C;
+        CDD_PASS_A_SMALL(CDD_TRY_A) CDD_PASS_A_BIG(CDD_TRY_A)
+        CDD_PASS_B_SMALL(CDD_TRY_B) CDD_PASS_B_BIG(CDD_TRY_B)
+#undef CDD_TRY_A
+#undef CDD_TRY_B
+        const int big = A > B ? A : B;
+        if (a && b && big < best) {
+            best = big;
+            lp.pa = a; lp.pb = b; lp.sa = s; lp.A = A; lp.B = B;
+        }
+    }
+}
+
+inline bool pass_big(const LinePlan& lp) { return lp.pa && (lp.A > 16 || lp.B > 16); }
+inline int rows_tier(const LinePlan& lp, int P) { return rows_io_plan(lp, P) ? 0 : (pass_big(lp) ? 2 : 1); }
 
 // Find the instance that owns global block b, given prefix sums pre[0..n] of blocks.
 __device__ __forceinline__ int find_instance(const int* __restrict__ pre, int n, int b) {
@@ -790,6 +886,9 @@ struct PlanCore {
     bool any3d = false;
     bool any_glide = false;          // some instance uses the glide-only dynamics
     bool any_vac = false;            // some instance has vacancy coupling
+    int rows_tier = 1;               // row passes: 0 every instance register-resident (rows_io_plan), 2 some BIG passes, else 1
+    bool big_mid = false, big_green = false;   // some instance's middle / first axis takes BIG passes
+    bool green_lean = false;         // every instance's k-space pass can run its lean form (green_plan_lean)
     void* d_vac = nullptr;           // caller's vacancy concentrations (cdd_set_vacancy), field_elems / 9
     void* d_vtr = nullptr;           // trace of beta^P at the step start (vacancy instances), field_elems / 9
     long long field_elems = 0, stress_elems = 0, cells = 0, spec_elems = 0, rows_total = 0;
@@ -899,6 +998,32 @@ size_t stencil_smem_bytes(int precision, bool any3d);
 int stencil_default_planes(const InstDev* insts, int n, int precision, int resident);
 void stencil_geometry(InstDev& I, int precision, int planes);
 cudaError_t stress_set_attributes(int precision, size_t max_smem);
+// Axis-1 pass: 128-byte row segments (16 columns FP32, 8 FP64), one radix-16 butterfly per thread at 256.
+__host__ __device__ constexpr int mid_threads(size_t elt) { return elt == 4 ? 256 : 128; }
+__host__ __device__ constexpr int row_threads_max(size_t elt) { return elt == 4 ? 256 : 128; }   // row passes
+inline int mid_buffers(const LinePlan& lp) { return (line_plan_io(lp) || lp.pa) ? 1 : 2; }
+// Component counts of the k-space pass per mode (see contract_tile).
+__host__ __device__ constexpr int green_nin(int gmode) { return (gmode == 6 || gmode == 8) ? 9 : (gmode == 7 ? 1 : 6); }
+__host__ __device__ constexpr int green_nout(int gmode) {
+    return (gmode == 3 || gmode == 6) ? 9 : ((gmode == 4 || gmode == 5 || gmode == 8) ? 3 : (gmode == 7 ? 1 : 6));
+}
+
+// The passes of the stress pipeline on the plan's spectrum (r2c.cu, fft_mid.cu, green.cu, c2r.cu). rowsum: FP64
+// row sums (FP32 mean path) or null; mode: RowSource / RowDest.
+void launch_r2c(const PlanCore& P, const LaunchShape& L, const void* in, double* rowsum, int mode, int ncomp, cudaStream_t st);
+void launch_mid(const PlanCore& P, const LaunchShape& L, bool inv, int ncomp, int vac_only, cudaStream_t st);
+void launch_green(const PlanCore& P, const LaunchShape& L, int gmode, bool mean64, const void* ktab, void* phi, double* part,
+                  cudaStream_t st);
+void launch_c2r(const PlanCore& P, const LaunchShape& L, void* out, bool mean64, int mode, int ncomp, const void* beta, int epi,
+                cudaStream_t st);
+cudaError_t r2c_set_attributes(int precision, size_t smem);
+cudaError_t mid_set_attributes(int precision, size_t smem);
+cudaError_t green_set_attributes(int precision, size_t smem);
+cudaError_t c2r_set_attributes(int precision, size_t smem);
+int green_cols(const InstDev& I, size_t velt);
+int green_threads(const InstDev& I, size_t velt);
+size_t green_smem_bytes(const InstDev& I, int W, int slots, size_t velt);
+bool green_plan_lean(const LinePlan& lp);
 // Fused plane passes of the stress solve (stress.cu): whether instance I can take them and their
 // shared memory per block.
 bool plane_eligible(const InstDev& I, int precision, size_t smem_limit);

@@ -79,6 +79,7 @@ bool na_line_plan(int n, LinePlan& lp) {
         lp.ns[i] = fdiv_make(ns);
         ns *= r[i];
     }
+    set_two_pass(lp);
     return true;
 }
 
@@ -190,52 +191,52 @@ extern "C" int cdd_stress_noalloc(const cdd_instance* d, int precision, const vo
     P.n_inst = 1;
     P.precision = precision;
     P.any3d = (I.nd == 3);
+    P.big_mid = (I.nd == 3) && pass_big(I.lp_mid);
+    P.big_green = pass_big(I.lp_first);
     size_t smem_need = 48 * 1024;
     int blocks[NUM_PASSES] = {0, 0, 0, 0, 0};
     for (int k : {PASS_R2C, PASS_C2R}) {
         const int comps = 6;
         long long npairs = ((long long)comps * I.rows + 1) / 2;
-        const size_t line_bytes = (size_t)(I.nl + (I.nl >> 4) + 1) * velt;
-        int Pl = (velt == 8 ? 4096 : 2048) / I.nl;
-        if (Pl < 1) Pl = 1;
-        if (Pl > npairs) Pl = (int)npairs;
+        const int Pl = rows_lines(I.lp_last, npairs, (int)velt);
+        P.rows_tier = rows_tier(I.lp_last, Pl);
         PassTile& t = I.tile[k];
         t.lines = Pl;
-        t.threads = (velt == 8) ? 256 : 128;
+        t.threads = rows_threads(I.lp_last, Pl, (int)velt);
         t.blocks = (int)((npairs + Pl - 1) / Pl);
         t.tiles_a = 1;
         P.pass[k].threads = t.threads;
-        P.pass[k].smem = ((2 * (size_t)Pl * (line_bytes / velt) + 1) & ~(size_t)1) * velt +
+        P.pass[k].smem = (((size_t)rows_elems(I.lp_last, Pl, (int)velt) + 1) & ~(size_t)1) * velt +
                          (size_t)I.lp_last.twspan * velt + rows_table_bytes(Pl);
     }
     for (int k : {PASS_MID_F, PASS_MID_I}) {
         PassTile& t = I.tile[k];
-        P.pass[k].threads = 256;
+        P.pass[k].threads = mid_threads(elt);
         if (I.nd != 3) continue;
         const int comps = 6;
         int W = (int)(128 / velt);
         while (W > 1 && 2 * (size_t)W * I.n1 * velt > 96 * 1024) W >>= 1;
         t.lines = W;
         while ((1 << t.lgw) < W) ++t.lgw;
-        t.threads = 256;
+        t.threads = mid_threads(elt);
         t.tiles_a = (I.nh + W - 1) / W;
         t.blocks = comps * I.n0 * t.tiles_a;
-        P.pass[k].smem = ((line_plan_io(I.lp_mid) && I.lp_mid.nst == 2) ? 1 : 2) * (size_t)W * I.n1 * velt +
+        P.pass[k].smem = mid_buffers(I.lp_mid) * (size_t)W * I.n1 * velt +
                          (size_t)I.lp_mid.twspan * velt;
     }
     {
         PassTile& t = I.tile[PASS_GREEN];
-        int W = (int)(32 / velt);
-        while (W > 1 && (size_t)9 * (I.n0 * W + W) * velt > 100 * 1024) W >>= 1;
+        const int W = green_cols(I, velt);
         if ((size_t)9 * (I.n0 * W + W) * velt > 220 * 1024)
             return err(CDD_ERR_SHAPE, "cdd_stress_noalloc: axis-0 length too large for the k-space pass");
         t.lines = W;
         while ((1 << t.lgw) < W) ++t.lgw;
-        t.threads = 256;
+        t.threads = green_threads(I, velt);
         t.tiles_a = (I.nh + W - 1) / W;
         t.blocks = (I.nd == 3 ? I.n1 : 1) * t.tiles_a;
-        P.pass[PASS_GREEN].threads = 256;
-        P.pass[PASS_GREEN].smem = ((size_t)9 * (I.n0 * W + W) + 1) / 2 * 2 * velt + (size_t)I.lp_first.twspan * velt;
+        P.pass[PASS_GREEN].threads = t.threads;
+        P.pass[PASS_GREEN].smem = green_smem_bytes(I, W, 6, velt);
+        P.green_lean = green_plan_lean(I.lp_first);
     }
     for (int k = 0; k < NUM_PASSES; ++k) {
         blocks[k] = I.tile[k].blocks;

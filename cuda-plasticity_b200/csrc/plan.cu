@@ -1,4 +1,5 @@
 // Plan construction and the C ABI of libcdd (see include/cdd.h).
+#include <algorithm>
 #include <cerrno>
 #include <cmath>
 #include <cstdarg>
@@ -71,6 +72,7 @@ bool make_line_plan(int n, LinePlan& lp, int maxr = 16) {
         lp.ns[i] = fdiv_make(ns);
         ns *= r[i];
     }
+    set_two_pass(lp);
     return true;
 }
 
@@ -173,7 +175,9 @@ int build_shapes(cdd_plan* p, size_t elt) {
     int thr_max[NUM_PASSES] = {0, 0, 0, 0, 0};
     std::vector<int> pre9[NUM_PASSES];   // the observables' launch shapes (9 components)
     for (int k = 0; k < NUM_PASSES; ++k) pre9[k].push_back(0);
-    size_t smem_green12 = 0;
+    size_t smem_green12 = 0, smem_green9 = 0, smem_green_lim = 0;
+    bool lean = true;
+    int rtier = 0;
     // the fused plane passes of the stress solve (3-D FP32 shapes that allow them) and the separate
     // row / axis-1 passes of the other instances
     std::vector<int> pre_plane(1, 0), pre_rest[NUM_PASSES];
@@ -194,20 +198,17 @@ int build_shapes(cdd_plan* p, size_t elt) {
         for (int k : {PASS_R2C, PASS_C2R}) {
             const int comps = 6;
             long long npairs = ((long long)comps * I.rows + 1) / 2;
-            const size_t line_bytes = (size_t)(I.nl + (I.nl >> 4) + 1) * velt;
             const cdd_tuning& tu = p->tune[i];
-            int P = (velt == 8 ? 4096 : 2048) / I.nl;   // radix-16 stages: one butterfly per thread
+            int P = rows_lines(I.lp_last, npairs, (int)velt);
             if (tu.rows_lines > 0) P = tu.rows_lines;
-            if (P < 1) P = 1;
             if (P > npairs) P = (int)npairs;
             PassTile& t = I.tile[k];
+            rtier = std::max(rtier, rows_tier(I.lp_last, P));
             t.lines = P;
-            // one first-stage butterfly per thread for 16-point stages: 256 threads from 16 line pairs
-            // on (FP32), 128 below (and for FP64)
-            t.threads = (velt == 8 && P >= 16) ? 256 : 128;
+            t.threads = rows_threads(I.lp_last, P, (int)velt);
             t.blocks = (int)((npairs + P - 1) / P);
             t.tiles_a = 1;
-            size_t sm = (((size_t)rows_buffers(I.lp_last, P) * P * (line_bytes / velt) + 1) & ~(size_t)1) * velt +
+            size_t sm = (((size_t)rows_elems(I.lp_last, P, (int)velt) + 1) & ~(size_t)1) * velt +
                         (size_t)I.lp_last.twspan * velt + rows_table_bytes(P);   // buffers + twiddle rows + row table
             if (sm > smem_max[k]) smem_max[k] = sm;
             if (t.threads > thr_max[k]) thr_max[k] = t.threads;
@@ -220,23 +221,22 @@ int build_shapes(cdd_plan* p, size_t elt) {
             int W = (int)(128 / velt);
             while (W > 1 && 2 * (size_t)W * I.n1 * velt > 96 * 1024) W >>= 1;
             if (p->tune[i].mid_cols > 0) W = p->tune[i].mid_cols;
+            C.big_mid |= pass_big(I.lp_mid);
             t.lines = W;
             t.lgw = 0;
             while ((1 << t.lgw) < W) ++t.lgw;
-            t.threads = 256;
+            t.threads = mid_threads(elt);
             t.tiles_a = (I.nh + W - 1) / W;
             t.blocks = comps * I.n0 * t.tiles_a;
-            // one shared tile for two-stage plans run with the first and last stage in global memory
-            const int bufs = (line_plan_io(I.lp_mid) && I.lp_mid.nst == 2) ? 1 : 2;
-            size_t sm = bufs * (size_t)W * I.n1 * velt + (size_t)I.lp_mid.twspan * velt;
+            size_t sm = mid_buffers(I.lp_mid) * (size_t)W * I.n1 * velt + (size_t)I.lp_mid.twspan * velt;
             if (sm > smem_max[k]) smem_max[k] = sm;
             if (t.threads > thr_max[k]) thr_max[k] = t.threads;
         }
-        // fused Green pass along axis 0: 6 component slots + 3 scratch slots of W columns
+        // fused Green pass along axis 0: component slots of W columns, 32-byte row segments. The limits
+        // on W and on the axis-0 length are those of 9 slots (6 components and 3 of scratch).
         {
             PassTile& t = I.tile[PASS_GREEN];
-            int W = (int)(32 / velt);   // 32-byte row segments
-            while (W > 1 && (size_t)9 * (I.n0 * W + W) * velt > 100 * 1024) W >>= 1;
+            int W = green_cols(I, velt);
             if (p->tune[i].green_cols > 0) W = p->tune[i].green_cols;
             if ((size_t)9 * (I.n0 * W + W) * velt > 220 * 1024) {
                 if (p->tune[i].green_cols > 0)
@@ -246,17 +246,21 @@ int build_shapes(cdd_plan* p, size_t elt) {
             t.lines = W;
             t.lgw = 0;
             while ((1 << t.lgw) < W) ++t.lgw;
-            t.threads = 256;
+            t.threads = green_threads(I, velt);
+            if (t.threads > thr_max[PASS_GREEN]) thr_max[PASS_GREEN] = t.threads;
             t.tiles_a = (I.nh + W - 1) / W;
             t.blocks = (I.nd == 3 ? I.n1 : 1) * t.tiles_a;
-            size_t sm = ((size_t)9 * (I.n0 * W + W) + 1) / 2 * 2 * velt + (size_t)I.lp_first.twspan * velt;
+            const size_t sm = green_smem_bytes(I, W, 6, velt);
             if (sm > smem_max[PASS_GREEN]) smem_max[PASS_GREEN] = sm;
-            if (t.threads > thr_max[PASS_GREEN]) thr_max[PASS_GREEN] = t.threads;
+            const size_t lim = ((size_t)9 * (I.n0 * W + W) + 1) / 2 * 2 * velt + (size_t)I.lp_first.twspan * velt;
+            if (lim > smem_green_lim) smem_green_lim = lim;
+            lean &= green_plan_lean(I.lp_first);
+            C.big_green |= pass_big(I.lp_first);
         }
         for (int k = 0; k < NUM_PASSES; ++k) pre[k].push_back(pre[k].back() + I.tile[k].blocks);
         {
-            // the observables carry up to 9 components through the row and axis-1 passes and keep
-            // 9 + 3 component slots in the k-space pass
+            // the observables carry up to 9 components through the row and axis-1 passes and the k-space
+            // pass (offered where 9 + 3 slots fit the device)
             const long long np9 = (9LL * I.rows + 1) / 2;
             const int P = I.tile[PASS_R2C].lines;
             const int b_rows = (int)((np9 + P - 1) / P);
@@ -264,8 +268,10 @@ int build_shapes(cdd_plan* p, size_t elt) {
             const int b9[NUM_PASSES] = {b_rows, b_mid, I.tile[PASS_GREEN].blocks, b_mid, b_rows};
             for (int k = 0; k < NUM_PASSES; ++k) pre9[k].push_back(pre9[k].back() + b9[k]);
             const int W = I.tile[PASS_GREEN].lines;
-            const size_t sm = ((size_t)12 * (I.n0 * W + W) + 1) / 2 * 2 * velt + (size_t)I.lp_first.twspan * velt;
-            if (sm > smem_green12) smem_green12 = sm;
+            const size_t lim = ((size_t)12 * (I.n0 * W + W) + 1) / 2 * 2 * velt + (size_t)I.lp_first.twspan * velt;
+            if (lim > smem_green12) smem_green12 = lim;
+            const size_t sm = green_smem_bytes(I, W, 9, velt);
+            if (sm > smem_green9) smem_green9 = sm;
         }
         {
             const bool ok = plane_eligible(I, C.precision, (size_t)optin_dev);
@@ -305,15 +311,15 @@ int build_shapes(cdd_plan* p, size_t elt) {
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         for (int k = 0; k < NUM_PASSES; ++k)
-            if (optin > 0 && smem_max[k] + 1024 > (size_t)optin)
+            if (const size_t need = (k == PASS_GREEN) ? smem_green_lim : smem_max[k]; optin > 0 && need + 1024 > (size_t)optin)
                 return fail(CDD_ERR_ARG, "launch shapes need %zu bytes of shared memory in FFT pass %d (limit %d)",
-                            smem_max[k], k, optin);
+                            need, k, optin);
     }
     size_t smem_all = 0;
     for (int k = 0; k < NUM_PASSES; ++k) {
         LaunchShape& L = C.pass[k];
         L.blocks = pre[k].back();
-        L.threads = (k == PASS_R2C || k == PASS_C2R) ? thr_max[k] : 256;
+        L.threads = (k == PASS_MID_F || k == PASS_MID_I) ? mid_threads(elt) : thr_max[k];
         L.smem = smem_max[k];
         if (L.smem > smem_all) smem_all = L.smem;
         CDD_CUDA(dalloc(p, (void**)&L.d_pre, sizeof(int) * (n + 1)));
@@ -321,7 +327,7 @@ int build_shapes(cdd_plan* p, size_t elt) {
         LaunchShape& L9 = C.pass9[k];
         L9.blocks = pre9[k].back();
         L9.threads = L.threads;
-        L9.smem = (k == PASS_GREEN) ? smem_green12 : L.smem;
+        L9.smem = (k == PASS_GREEN) ? smem_green9 : L.smem;
         if (L9.smem > smem_all) smem_all = L9.smem;
         CDD_CUDA(dalloc(p, (void**)&L9.d_pre, sizeof(int) * (n + 1)));
         CDD_CUDA(cudaMemcpy(L9.d_pre, pre9[k].data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
@@ -345,7 +351,8 @@ int build_shapes(cdd_plan* p, size_t elt) {
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         C.obs_ok = !(optin > 0 && smem_green12 + 1024 > (size_t)optin);
         if (!C.obs_ok) C.pass9[PASS_GREEN].smem = C.pass[PASS_GREEN].smem;   // never launched
-        if (C.pass9[PASS_GREEN].smem > smem_all) smem_all = C.pass9[PASS_GREEN].smem;
+        C.green_lean = lean;
+        C.rows_tier = rtier;
     }
     C.stencil.blocks = pre_st.back();
     C.stencil.threads = 256;
