@@ -21,14 +21,19 @@ k_c2r_rows(const InstDev* __restrict__ insts, int n_inst,
     const int lb = blockIdx.x - pre[ii];
     const int N = I.nl, P = I.tile[PASS_C2R].lines, ld = rows_ld(N), nh = I.nh;
     const long long nrows = (long long)ncomp * I.rows;
-    if (2LL * lb * P >= nrows) return;   // launch sized for more components than this pass carries
-    if (mode == RD_VAC && (!I.vacancy || !clk[ii].active)) return;
+    // a launch sized for more components than this pass carries, or other instances' diffusion
+    if (2LL * lb * P >= nrows || (mode == RD_VAC && !I.vacancy)) {
+        pdl_wait();
+        return;
+    }
     const long long npairs = (nrows + 1) / 2;
     const int tid = threadIdx.x, nt = blockDim.x;
     const V* src = spec + I.spoff;
     const bool io = rows_io_plan(I.lp_last, P);
     V* tws = s + ((rows_elems(I.lp_last, P, sizeof(V)) + 1) & ~1);
     stage_tw_to_smem(I.lp_last, tw, tws, tid, nt);
+    pdl_wait();
+    if (mode == RD_VAC && !clk[ii].active) return;
     // row table: the destination rows of each of the block's 2P rows and their FP64 mean stress
     RowPtr* rt = rows_table(tws, I.lp_last.twspan);
     RowPtr* re = rt + 2 * P;                                        // epilogue source rows
@@ -187,7 +192,7 @@ k_c2r_rows(const InstDev* __restrict__ insts, int n_inst,
 template <typename T, bool MEAN64>
 static void c2r_t(const PlanCore& P, const LaunchShape& L, void* out, int mode, int ncomp, const void* beta, int epi, cudaStream_t st) {
     typedef typename VecOf<T>::type V;
-#define CDD_LAUNCH_R(TIER) k_c2r_rows<T, MEAN64, TIER><<<L.blocks, L.threads, L.smem, st>>>(P.d_inst, P.n_inst, L.d_pre, (const V*)P.d_spec, (T*)out, \
+#define CDD_LAUNCH_R(TIER) launch_pdl(P, k_c2r_rows<T, MEAN64, TIER>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, (const V*)P.d_spec, (T*)out, \
         (const V*)P.d_tw, P.d_sbar, mode, ncomp, (const T*)beta, epi, P.d_clock)
     if (P.rows_tier == 0) CDD_LAUNCH_R(0);
     else if (P.rows_tier == 1) CDD_LAUNCH_R(1);

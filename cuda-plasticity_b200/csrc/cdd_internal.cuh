@@ -859,6 +859,16 @@ inline void set_two_pass(LinePlan& lp) {
 inline bool pass_big(const LinePlan& lp) { return lp.pa && (lp.A > 16 || lp.B > 16); }
 inline int rows_tier(const LinePlan& lp, int P) { return rows_io_plan(lp, P) ? 0 : (pass_big(lp) ? 2 : 1); }
 
+// Programmatic dependent launch (launch_pdl): a kernel starts while the one before it in the stream runs its last
+// blocks, prepares what no kernel writes (instance table, twiddle rows, barriers), and then waits for that
+// one to have finished and its writes to be visible. Only then does it let its own successor start: let go
+// earlier, the successors pile up on the SMs that drain first (96^3 FP32 step 573 us instead of 557).
+// Every block of every kernel waits, also those with nothing to do: a kernel that finished without waiting
+// would let its successor past its predecessor.
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.wait;\n griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Find the instance that owns global block b, given prefix sums pre[0..n] of blocks.
 __device__ __forceinline__ int find_instance(const int* __restrict__ pre, int n, int b) {
     int lo = 0, hi = n - 1;
@@ -925,6 +935,29 @@ struct PlanCore {
     void* d_f0b = nullptr;           // reverse RK3: cotangents of F0 and F1
     void* d_f1b = nullptr;
 };
+
+// Launch on a plan's stream. Programmatic (see pdl_wait) where launches cost most: calls outside a stream capture
+// (24^3 FP32 step 152 -> 115 us, 32^3 FP64 stress 33 -> 19, 128^3 FP32 step 1028 -> 992) and the graphs of small
+// plans (2-D 128^2 FP64 step 85 -> 78 us). In larger plans' graphs, whose nodes follow one another in about a
+// microsecond anyway, it costs more than it gives (64^3 FP64 step 340 -> 354 us, 512^2 FP32 226 -> 255: blocks
+// that start under a kernel with a large shared-memory carve-out run with little L1).
+template <typename... K, typename... A>
+inline cudaError_t launch_pdl(const PlanCore& P, void (*kernel)(K...), dim3 grid, unsigned threads, size_t smem,
+                              cudaStream_t st, A&&... args) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool known = cudaStreamIsCapturing(st, &cap) == cudaSuccess;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = at;
+    c.numAttrs = (known && (cap == cudaStreamCaptureStatusNone || P.cells <= 65536)) ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<K>(args)...);
+}
 
 // Tensor maps of one stage-input buffer for the TMA-staged instances (see stencil.cu).
 struct StencilMapSet {
@@ -1001,7 +1034,7 @@ cudaError_t stress_set_attributes(int precision, size_t max_smem);
 // Axis-1 pass: 128-byte row segments (16 columns FP32, 8 FP64), one radix-16 butterfly per thread at 256.
 __host__ __device__ constexpr int mid_threads(size_t elt) { return elt == 4 ? 256 : 128; }
 __host__ __device__ constexpr int row_threads_max(size_t elt) { return elt == 4 ? 256 : 128; }   // row passes
-inline int mid_buffers(const LinePlan& lp) { return (line_plan_io(lp) || lp.pa) ? 1 : 2; }
+__host__ __device__ inline int mid_buffers(const LinePlan& lp) { return (line_plan_io(lp) || lp.pa) ? 1 : 2; }
 // Component counts of the k-space pass per mode (see contract_tile).
 __host__ __device__ constexpr int green_nin(int gmode) { return (gmode == 6 || gmode == 8) ? 9 : (gmode == 7 ? 1 : 6); }
 __host__ __device__ constexpr int green_nout(int gmode) {

@@ -13,15 +13,13 @@ namespace cdd {
 template <typename T, bool INV, bool BIG>
 __device__ __forceinline__ void fft_mid_tile(const InstDev& I, typename VecOf<T>::type* s,
                                              typename VecOf<T>::type* base,
-                                             const typename VecOf<T>::type* __restrict__ tw, int lgw, int wv,
+                                             const typename VecOf<T>::type* __restrict__ tws, int lgw, int wv,
                                              int tid, int nt) {
     typedef typename VecOf<T>::type V;
     const int W = 1 << lgw;
     const int N = I.n1, nhp = I.nhp;
     if (line_plan_io(I.lp_mid)) {
         // both stages' other ends in global memory, one shared tile
-        V* tws = s + N * W;
-        stage_tw_to_smem(I.lp_mid, tw, tws, tid, nt);
         const GColT<V, 1> g{base, nhp, 0, lgw, wv};
         const SColT<V, 1> x{s, lgw, 0}, y{s + N * W, lgw, 0};
         fft_io<V, INV, 1>(g, x, y, g, lgw, I.lp_mid, tws, tid, nt, I.lp_mid.twst[0]);
@@ -30,8 +28,6 @@ __device__ __forceinline__ void fft_mid_tile(const InstDev& I, typename VecOf<T>
     if (I.lp_mid.pa) {
         // two passes through one shared tile
         const LinePlan& lp = I.lp_mid;
-        V* tws = s + N * W;
-        stage_tw_to_smem(lp, tw, tws, tid, nt);
         __syncthreads();
         const Cols<V> g{base, 0, wv}, t{s, 0, W};
         col_pass_a<V, INV, BIG ? 2 : 1>(g, nhp, (long long)lp.B * nhp, t, (long long)lp.A << lgw, W, W, lgw, lp, tws, tid, nt);
@@ -49,8 +45,6 @@ __device__ __forceinline__ void fft_mid_tile(const InstDev& I, typename VecOf<T>
             s[i] = z;
         }
     }
-    V* tws = s + 2 * N * W;
-    stage_tw_to_smem(I.lp_mid, tw, tws, tid, nt);
     cp_async_wait_all();
     __syncthreads();
     ColLayout<1> lay{lgw, 0};
@@ -84,16 +78,19 @@ k_fft_mid(const InstDev* __restrict__ insts, int n_inst,
     const int ta = lb % ta_n; lb /= ta_n;
     const int i0 = lb % I.n0;
     const int c = lb / I.n0;
-    if (c >= ncomp) return;   // launch sized for more components than this pass carries
-    if (vac_only && !I.vacancy) return;
     const int N = I.n1, nhp = I.nhp, nh = I.nh;
     const int col0 = ta * W;
     const int wv = min(W, nh - col0);
     const int tid = threadIdx.x, nt = blockDim.x;
+    V* tws = s + mid_buffers(I.lp_mid) * N * W;   // twiddle rows after the tile buffers
+    stage_tw_to_smem(I.lp_mid, tw, tws, tid, nt);
+    pdl_wait();
+    if (c >= ncomp) return;   // launch sized for more components than this pass carries
+    if (vac_only && !I.vacancy) return;
     V* base = spec + I.spoff + ((long long)c * I.n0 + i0) * (long long)N * nhp + col0;
-    if (lgw == 4) fft_mid_tile<T, INV, BIG>(I, s, base, tw, 4, wv, tid, nt);
-    else if (lgw == 3) fft_mid_tile<T, INV, BIG>(I, s, base, tw, 3, wv, tid, nt);
-    else fft_mid_tile<T, INV, BIG>(I, s, base, tw, lgw, wv, tid, nt);
+    if (lgw == 4) fft_mid_tile<T, INV, BIG>(I, s, base, tws, 4, wv, tid, nt);
+    else if (lgw == 3) fft_mid_tile<T, INV, BIG>(I, s, base, tws, 3, wv, tid, nt);
+    else fft_mid_tile<T, INV, BIG>(I, s, base, tws, lgw, wv, tid, nt);
 }
 
 template <typename T, bool INV>
@@ -101,10 +98,10 @@ static void mid_t(const PlanCore& P, const LaunchShape& L, int ncomp, int vac_on
     typedef typename VecOf<T>::type V;
     const int pass = INV ? PASS_MID_I : PASS_MID_F;
     if (P.big_mid)
-        k_fft_mid<T, INV, true><<<L.blocks, L.threads, L.smem, st>>>(P.d_inst, P.n_inst, L.d_pre, (V*)P.d_spec, (const V*)P.d_tw,
+        launch_pdl(P, k_fft_mid<T, INV, true>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, (V*)P.d_spec, (const V*)P.d_tw,
                                                                      pass, ncomp, vac_only);
     else
-        k_fft_mid<T, INV, false><<<L.blocks, L.threads, L.smem, st>>>(P.d_inst, P.n_inst, L.d_pre, (V*)P.d_spec, (const V*)P.d_tw,
+        launch_pdl(P, k_fft_mid<T, INV, false>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, (V*)P.d_spec, (const V*)P.d_tw,
                                                                       pass, ncomp, vac_only);
 }
 

@@ -417,7 +417,10 @@ k_green(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ p
     V* s = reinterpret_cast<V*>(smem_raw);
     const int ii = find_instance(pre, n_inst, blockIdx.x);
     const InstDev& I = insts[ii];
-    if (gmode == 7 && !I.vacancy) return;
+    if (gmode == 7 && !I.vacancy) {
+        pdl_wait();
+        return;
+    }
     const int lb = blockIdx.x - pre[ii];
     const PassTile& tl = I.tile[PASS_GREEN];
     const int lgw = tl.lgw, ta_n = tl.tiles_a;
@@ -438,6 +441,7 @@ k_green(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ p
     V* scratch = s + slots * cs;
     V* tws = s + (((two ? slots : slots + 3) * cs + 1) & ~1);   // twiddle rows after the slots
     stage_tw_to_smem(lp, tw, tws, tid, nt);
+    pdl_wait();
     const Cols<V> glob{base, cstride, wv}, slot{s, cs, W};
     if (two) {
         __syncthreads();
@@ -519,7 +523,7 @@ static void green_t(const PlanCore& P, const LaunchShape& L, int gmode, bool mea
     typedef typename VecOf<T>::type V;
     const int tier = (P.green_lean && gmode <= 1) ? 0 : (P.big_green ? 2 : 1);
 #define CDD_LAUNCH_G(TIER)                                                                                              \
-    k_green<T, TIER><<<L.blocks, L.threads, L.smem, st>>>(P.d_inst, P.n_inst, L.d_pre, gmode, mean64, (V*)P.d_spec,      \
+    launch_pdl(P, k_green<T, TIER>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, gmode, mean64, (V*)P.d_spec,      \
                                                           (const V*)P.d_tw, (const T*)ktab, (V*)phi, part, P.d_clock)
     if (tier == 0) CDD_LAUNCH_G(0);
     else if (tier == 1) CDD_LAUNCH_G(1);

@@ -23,8 +23,11 @@ k_r2c_rows(const InstDev* __restrict__ insts, int n_inst,
     const int lb = blockIdx.x - pre[ii];
     const int N = I.nl, P = I.tile[PASS_R2C].lines, ld = rows_ld(N);
     const long long nrows = (long long)ncomp * I.rows;
-    if (2LL * lb * P >= nrows) return;   // launch sized for more components than this pass carries
-    if (mode == RS_VAC && !I.vacancy) return;
+    // a launch sized for more components than this pass carries, or other instances' diffusion
+    if (2LL * lb * P >= nrows || (mode == RS_VAC && !I.vacancy)) {
+        pdl_wait();
+        return;
+    }
     const long long npairs = (nrows + 1) / 2;
     const int tid = threadIdx.x, nt = blockDim.x;
     const T half = (T)0.5;
@@ -46,6 +49,7 @@ k_r2c_rows(const InstDev* __restrict__ insts, int n_inst,
         rt[r] = e;
     }
     stage_tw_to_smem(I.lp_last, tw, tws, tid, nt);
+    pdl_wait();
     __syncthreads();
     {
         const LinePlan& lq = I.lp_last;
@@ -146,7 +150,7 @@ k_r2c_rows(const InstDev* __restrict__ insts, int n_inst,
 template <typename T, bool MEAN64>
 static void r2c_t(const PlanCore& P, const LaunchShape& L, const void* in, double* rowsum, int mode, int ncomp, cudaStream_t st) {
     typedef typename VecOf<T>::type V;
-#define CDD_LAUNCH_R(TIER) k_r2c_rows<T, MEAN64, TIER><<<L.blocks, L.threads, L.smem, st>>>(P.d_inst, P.n_inst, L.d_pre, (const T*)in, (V*)P.d_spec, \
+#define CDD_LAUNCH_R(TIER) launch_pdl(P, k_r2c_rows<T, MEAN64, TIER>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, (const T*)in, (V*)P.d_spec, \
         (const V*)P.d_tw, rowsum, mode, ncomp)
     if (P.rows_tier == 0) CDD_LAUNCH_R(0);
     else if (P.rows_tier == 1) CDD_LAUNCH_R(1);

@@ -996,6 +996,12 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
 
     __shared__ StageConst kc;   // read per cell from shared memory (keeps registers free)
     __shared__ BoxGeomT<T> bg;
+    if (use_tma && tid == 0) {
+#pragma unroll 1
+        for (int s = 0; s < NS; ++s) mbar_init(&bars[s], 1);
+        fence_mbar_init();
+    }
+    pdl_wait();
     if (tid == 0) {
         kc = stage_const<MODE>(I, clk[ii], t_flux);
         bg = {src, cells, x0, y0, nX, nY, nZ, ND == 3 ? z0 - 2 : 0, box_chunk<T>(src, nX)};
@@ -1018,12 +1024,8 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
     int issued = -1;   // highest plane index handed to TMA
     int ok = 1;        // block-uniform: every plane waited for has arrived
     if (use_tma) {
-        if (tid == 0) {
-#pragma unroll 1
-            for (int s = 0; s < NS; ++s) mbar_init(&bars[s], 1);
-            fence_mbar_init();
+        if (tid == 0)
             for (int pr = 0; pr < NPL; ++pr) issue(pr);
-        }
         issued = NPL - 1;
     } else {
 #pragma unroll 1
@@ -1056,7 +1058,7 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
 #pragma unroll
     for (int c = 0; c < 6; ++c) cp_async_elem(ssm + c * ST_THREADS, cx.sig + c * cells);
     cp_async_commit();
-    // the first planes: the barrier makes the barriers' initialisation, kc and the staged copies visible
+    // the first planes: the barrier makes the staged copies visible
     if (!use_tma) cp_async_wait_own();
     __syncthreads();
     bool got = true;   // this thread saw every plane of the coming cell arrive
@@ -1194,6 +1196,7 @@ __global__ void __launch_bounds__(1024) k_dt(const InstDev* __restrict__ insts,
     const int ii = blockIdx.x;
     const InstDev& I = insts[ii];
     const int b0 = pre[ii], b1 = pre[ii + 1];
+    pdl_wait();
     double m = 0.0, es = 0.0, zs = 0.0;
     // one pass over the block partials, unrolled so that several loads are in flight; observable
     // sums: fixed-order strided partial sums, then a fixed tree (deterministic)
@@ -1236,6 +1239,7 @@ __global__ void __launch_bounds__(256) k_axpy_f0(const InstDev* __restrict__ ins
                                                  T* __restrict__ f0, const InstClock* __restrict__ clk) {
     const int ii = find_instance(pre, n_inst, blockIdx.x);
     const InstDev& I = insts[ii];
+    pdl_wait();
     if (!clk[ii].active || I.plane) return;
     const T dt = (T)clk[ii].dt;
     const long long n = 9 * I.cells;
@@ -1283,6 +1287,7 @@ __global__ void __launch_bounds__(256) k_vac_trace(const InstDev* __restrict__ i
                                                    T* __restrict__ tr) {
     const int ii = find_instance(pre, n_inst, blockIdx.x);
     const InstDev& I = insts[ii];
+    pdl_wait();
     if (!I.vacancy) return;
     const long long cell = (long long)(blockIdx.x - pre[ii]) * blockDim.x + threadIdx.x;
     if (cell >= I.cells) return;
@@ -1297,6 +1302,7 @@ __global__ void __launch_bounds__(256) k_vac_update(const InstDev* __restrict__ 
                                                     const InstClock* __restrict__ clk) {
     const int ii = find_instance(pre, n_inst, blockIdx.x);
     const InstDev& I = insts[ii];
+    pdl_wait();
     if (!I.vacancy || !clk[ii].active) return;
     const long long cell = (long long)(blockIdx.x - pre[ii]) * blockDim.x + threadIdx.x;
     if (cell >= I.cells) return;
@@ -1317,6 +1323,7 @@ __global__ void __launch_bounds__(256) k_observe(const InstDev* __restrict__ ins
     const int ii = find_instance(pre, n_inst, blockIdx.x);
     const InstDev& I = insts[ii];
     const long long cell = (long long)(blockIdx.x - pre[ii]) * blockDim.x + threadIdx.x;
+    pdl_wait();
     double e = 0.0, z = 0.0;
     if (cell < I.cells) {
         const T* sp = sig + I.soff + cell;
@@ -1339,6 +1346,7 @@ __global__ void __launch_bounds__(256) k_obs_reduce(const InstDev* __restrict__ 
                                                     double* __restrict__ obs) {
     __shared__ double red[8];
     const int ii = blockIdx.x;
+    pdl_wait();
     double es = 0.0, zs = 0.0;
     for (int b = pre[ii] + threadIdx.x; b < pre[ii + 1]; b += blockDim.x) {
         es += bsum[2 * b];
@@ -1365,7 +1373,7 @@ static void stencil_dispatch(const PlanCore& P, int mode, const void* bs, const 
     // the plan has such instances
     const int var = (P.any_glide ? 1 : 0) | (P.any_vac ? 2 : 0);
 #define CDD_LAUNCH_V(M, V, SP)                                                                           \
-    k_stencil<T, M, V><<<L.blocks, st_threads<T>(), L.smem, st>>>(P.d_inst, P.n_inst, L.d_pre, b, n, o, s, SP,     \
+    launch_pdl(P, k_stencil<T, M, V>, L.blocks, st_threads<T>(), L.smem, st, P.d_inst, P.n_inst, L.d_pre, b, n, o, s, SP,     \
                                                              P.d_clock, t, P.d_bmax, P.d_bsum, P.d_status,    \
                                                              (const T*)P.d_vac, maps)
 #define CDD_LAUNCH_ST(M, SP)                                  \
@@ -1388,7 +1396,7 @@ static void stencil_dispatch(const PlanCore& P, int mode, const void* bs, const 
 template <typename T>
 static cudaError_t vac_pre_t(const PlanCore& P, const void* beta, cudaStream_t st) {
     const LaunchShape& L = P.obs;
-    k_vac_trace<T><<<L.blocks, L.threads, 0, st>>>(P.d_inst, P.n_inst, L.d_pre, (const T*)beta, (T*)P.d_vtr);
+    launch_pdl(P, k_vac_trace<T>, L.blocks, L.threads, 0, st, P.d_inst, P.n_inst, L.d_pre, (const T*)beta, (T*)P.d_vtr);
     return cudaGetLastError();
 }
 
@@ -1399,7 +1407,7 @@ cudaError_t launch_vacancy_pre(const PlanCore& P, const void* beta, cudaStream_t
 template <typename T>
 static cudaError_t vac_post_t(const PlanCore& P, const void* beta, cudaStream_t st) {
     const LaunchShape& L = P.obs;
-    k_vac_update<T><<<L.blocks, L.threads, 0, st>>>(P.d_inst, P.n_inst, L.d_pre, (const T*)beta,
+    launch_pdl(P, k_vac_update<T>, L.blocks, L.threads, 0, st, P.d_inst, P.n_inst, L.d_pre, (const T*)beta,
                                                     (const T*)P.d_vtr, (T*)P.d_vac, P.d_clock);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -1481,6 +1489,7 @@ bool encode_stencil_maps(const PlanCore& P, const InstDev* insts, const void* ba
 // Start every instance's clock at t with no end time (fixed-dt steps at a caller-given time).
 __global__ void k_set_clock(InstClock* __restrict__ clk, int n_inst, double t) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
     if (i < n_inst) {
         clk[i].t = t;
         clk[i].t_end = 1.0e300;
@@ -1488,12 +1497,12 @@ __global__ void k_set_clock(InstClock* __restrict__ clk, int n_inst, double t) {
 }
 
 cudaError_t launch_set_clock(const PlanCore& P, double t, cudaStream_t st) {
-    k_set_clock<<<(P.n_inst + 127) / 128, 128, 0, st>>>(P.d_clock, P.n_inst, t);
+    launch_pdl(P, k_set_clock, (P.n_inst + 127) / 128, 128, 0, st, P.d_clock, P.n_inst, t);
     return cudaGetLastError();
 }
 
 cudaError_t launch_dt(const PlanCore& P, int fixed, double dt_fixed, cudaStream_t st) {
-    k_dt<<<P.n_inst, 1024, 0, st>>>(P.d_inst, P.stencil.d_pre, P.d_bmax, P.d_bsum, P.d_clock, P.d_obs,
+    launch_pdl(P, k_dt, P.n_inst, 1024, 0, st, P.d_inst, P.stencil.d_pre, P.d_bmax, P.d_bsum, P.d_clock, P.d_obs,
                                    P.d_status, fixed, dt_fixed);
     return cudaGetLastError();
 }
@@ -1501,10 +1510,10 @@ cudaError_t launch_dt(const PlanCore& P, int fixed, double dt_fixed, cudaStream_
 cudaError_t launch_axpy_f0(const PlanCore& P, const void* u, void* rhs_f0, cudaStream_t st) {
     const LaunchShape& L = P.cellwise;
     if (P.precision == CDD_F32)
-        k_axpy_f0<float><<<L.blocks, 256, 0, st>>>(P.d_inst, P.n_inst, L.d_pre, (const float*)u,
+        launch_pdl(P, k_axpy_f0<float>, L.blocks, 256, 0, st, P.d_inst, P.n_inst, L.d_pre, (const float*)u,
                                                    (float*)rhs_f0, P.d_clock);
     else
-        k_axpy_f0<double><<<L.blocks, 256, 0, st>>>(P.d_inst, P.n_inst, L.d_pre, (const double*)u,
+        launch_pdl(P, k_axpy_f0<double>, L.blocks, 256, 0, st, P.d_inst, P.n_inst, L.d_pre, (const double*)u,
                                                     (double*)rhs_f0, P.d_clock);
     return cudaGetLastError();
 }
@@ -1512,12 +1521,12 @@ cudaError_t launch_axpy_f0(const PlanCore& P, const void* u, void* rhs_f0, cudaS
 cudaError_t launch_observe(const PlanCore& P, const void* beta, cudaStream_t st) {
     const LaunchShape& L = P.obs;
     if (P.precision == CDD_F32)
-        k_observe<float><<<L.blocks, 256, 0, st>>>(P.d_inst, P.n_inst, L.d_pre, (const float*)beta,
+        launch_pdl(P, k_observe<float>, L.blocks, 256, 0, st, P.d_inst, P.n_inst, L.d_pre, (const float*)beta,
                                                          (const float*)P.d_sigma, P.d_bsum);
     else
-        k_observe<double><<<L.blocks, 256, 0, st>>>(P.d_inst, P.n_inst, L.d_pre, (const double*)beta,
+        launch_pdl(P, k_observe<double>, L.blocks, 256, 0, st, P.d_inst, P.n_inst, L.d_pre, (const double*)beta,
                                                           (const double*)P.d_sigma, P.d_bsum);
-    k_obs_reduce<<<P.n_inst, 256, 0, st>>>(P.d_inst, P.obs.d_pre, P.d_bsum, P.d_obs);
+    launch_pdl(P, k_obs_reduce, P.n_inst, 256, 0, st, P.d_inst, P.obs.d_pre, P.d_bsum, P.d_obs);
     return cudaGetLastError();
 }
 

@@ -209,6 +209,7 @@ k_plane_fwd(const InstDev* __restrict__ insts, int n_inst, const int* __restrict
     typedef typename VecOf<T>::type V;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cg::cluster_group cl = cg::this_cluster();
+    pdl_wait();
     cl.sync();   // every block of the cluster runs before any stores into another
     const int ii = find_instance(pre, n_inst, blockIdx.x);
     const InstDev& I = insts[ii];
@@ -285,6 +286,7 @@ k_plane_inv(const InstDev* __restrict__ insts, int n_inst, const int* __restrict
     typedef typename VecOf<T>::type V;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cg::cluster_group cl = cg::this_cluster();
+    pdl_wait();
     cl.sync();   // every block of the cluster runs before any stores into another
     const int ii = find_instance(pre, n_inst, blockIdx.x);
     const InstDev& I = insts[ii];
@@ -352,6 +354,7 @@ k_mean_beta(const InstDev* __restrict__ insts, const double* __restrict__ rowsum
     const InstDev& I = insts[blockIdx.x];
     const int c = blockIdx.y;
     cg::cluster_group cl = cg::this_cluster();
+    pdl_wait();
     const int part = (int)cl.block_rank();
     __shared__ double red[32];
     __shared__ double share;
@@ -410,19 +413,19 @@ static cudaError_t run_stress(const PlanCore& P, const void* beta, void* sigma, 
         if (e != cudaSuccess) return e;
     }
     if (plane && u)
-        k_plane_fwd<float, true><<<P.plane.blocks, P.plane.threads, P.plane.smem, st>>>(
+        launch_pdl(P, k_plane_fwd<float, true>, P.plane.blocks, P.plane.threads, P.plane.smem, st, 
             P.d_inst, P.n_inst, P.plane.d_pre, (const float*)beta, spec, tw, P.d_rowsum, (float*)beta, (const float*)u,
             P.d_clock);
     else if (plane)
-        k_plane_fwd<float, false><<<P.plane.blocks, P.plane.threads, P.plane.smem, st>>>(
+        launch_pdl(P, k_plane_fwd<float, false>, P.plane.blocks, P.plane.threads, P.plane.smem, st, 
             P.d_inst, P.n_inst, P.plane.d_pre, (const float*)beta, spec, tw, P.d_rowsum, nullptr, nullptr, nullptr);
     if (LR[PASS_R2C].blocks > 0) launch_r2c(P, LR[PASS_R2C], beta, f32 ? P.d_rowsum : nullptr, RS_SYM, 6, st);
-    if (f32) k_mean_beta<<<dim3(P.n_inst, 6, MEAN_SPLIT), 1024, 0, st>>>(P.d_inst, P.d_rowsum, P.d_sbar);
+    if (f32) launch_pdl(P, k_mean_beta, dim3(P.n_inst, 6, MEAN_SPLIT), 1024, 0, st, P.d_inst, P.d_rowsum, P.d_sbar);
     launch_mid(P, LR[PASS_MID_F], false, 6, 0, st);
     launch_green(P, P.pass[PASS_GREEN], 0, f32, P.d_k, phi, nullptr, st);
     launch_mid(P, LR[PASS_MID_I], true, 6, 0, st);
     if (plane)
-        k_plane_inv<float><<<P.plane.blocks, P.plane.threads, P.plane.smem, st>>>(
+        launch_pdl(P, k_plane_inv<float>, P.plane.blocks, P.plane.threads, P.plane.smem, st, 
             P.d_inst, P.n_inst, P.plane.d_pre, spec, (float*)sigma, tw, P.d_sbar);
     if (LR[PASS_C2R].blocks > 0) launch_c2r(P, LR[PASS_C2R], sigma, f32, RD_STRESS, 6, nullptr, EPI_NONE, st);
     return cudaGetLastError();
