@@ -739,11 +739,11 @@ cudaError_t launch_flux_branches(const PlanCore& P, const void* beta, double t, 
     cudaError_t e;
     if ((e = launch_stress(P, beta, P.d_sigma, st))) return e;
     if (P.precision == CDD_F32)
-        launch_pdl(P, k_vjp_cells<float>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const float*)beta,
+        launch_pdl(k_vjp_cells<float>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const float*)beta,
                                                             (const float*)P.d_sigma, nullptr, t, nullptr, flags,
                                                             nullptr, P.d_bload);
     else
-        launch_pdl(P, k_vjp_cells<double>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const double*)beta,
+        launch_pdl(k_vjp_cells<double>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const double*)beta,
                                                              (const double*)P.d_sigma, nullptr, t, nullptr, flags,
                                                              nullptr, P.d_bload);
     return cudaGetLastError();
@@ -757,11 +757,11 @@ cudaError_t launch_vjp_stage(const PlanCore& P, const void* v, const void* sig_v
     cudaError_t e;
     const bool f32 = (P.precision == CDD_F32);
     if (f32)
-        launch_pdl(P, k_vjp_cells<float>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const float*)v,
+        launch_pdl(k_vjp_cells<float>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const float*)v,
                                                             (const float*)sig_v, (const float*)gbar, t,
                                                             (float*)P.d_ubar, P.d_flags, (float*)P.d_sb6, P.d_bload);
     else
-        launch_pdl(P, k_vjp_cells<double>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const double*)v,
+        launch_pdl(k_vjp_cells<double>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const double*)v,
                                                              (const double*)sig_v, (const double*)gbar, t,
                                                              (double*)P.d_ubar, P.d_flags, (double*)P.d_sb6,
                                                              P.d_bload);
@@ -769,18 +769,18 @@ cudaError_t launch_vjp_stage(const PlanCore& P, const void* v, const void* sig_v
     if ((e = launch_stress_adjoint(P, P.d_sb6, P.d_adj9, st, pbar ? phi_v : nullptr, pbar ? P.d_gpart : nullptr)))
         return e;
     if (pbar) {
-        launch_pdl(P, k_param_reduce, P.n_inst, 256, 0, st, P.d_inst, V.d_pre, P.d_bload, P.pass[PASS_GREEN].d_pre,
+        launch_pdl(k_param_reduce, P.n_inst, 256, 0, st, P.d_inst, V.d_pre, P.d_bload, P.pass[PASS_GREEN].d_pre,
                                                  phi_v ? P.d_gpart : nullptr, c, t, pbar);
         if ((e = cudaGetLastError())) return e;
     }
     if (f32) {
         Axpy<float> ax{(float)c, {(const float*)x[0], (const float*)x[1], (const float*)x[2]},
                        {(float)a[0], (float)a[1], (float)a[2]}};
-        launch_pdl(P, k_vjp_gather<float>, G.blocks, 256, 0, st, P.d_inst, P.n_inst, G.d_pre, (const float*)P.d_ubar, P.d_flags,
+        launch_pdl(k_vjp_gather<float>, G.blocks, 256, 0, st, P.d_inst, P.n_inst, G.d_pre, (const float*)P.d_ubar, P.d_flags,
                                                      (const float*)P.d_adj9, ax, (float*)out);
     } else {
         Axpy<double> ax{c, {(const double*)x[0], (const double*)x[1], (const double*)x[2]}, {a[0], a[1], a[2]}};
-        launch_pdl(P, k_vjp_gather<double>, G.blocks, 256, 0, st, P.d_inst, P.n_inst, G.d_pre, (const double*)P.d_ubar,
+        launch_pdl(k_vjp_gather<double>, G.blocks, 256, 0, st, P.d_inst, P.n_inst, G.d_pre, (const double*)P.d_ubar,
                                                       P.d_flags, (const double*)P.d_adj9, ax, (double*)out);
     }
     return cudaGetLastError();
@@ -793,25 +793,25 @@ cudaError_t launch_flux_vjp(const PlanCore& P, const void* beta, double t, const
     cudaError_t e;
     if ((e = launch_stress(P, beta, P.d_sigma, st))) return e;
     if (P.precision == CDD_F32) {
-        launch_pdl(P, k_vjp_cells<float>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const float*)beta,
+        launch_pdl(k_vjp_cells<float>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const float*)beta,
                                                             (const float*)P.d_sigma, (const float*)gbar, t,
                                                             (float*)P.d_ubar, P.d_flags, (float*)sigbar, P.d_bload);
     } else {
-        launch_pdl(P, k_vjp_cells<double>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const double*)beta,
+        launch_pdl(k_vjp_cells<double>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const double*)beta,
                                                              (const double*)P.d_sigma, (const double*)gbar, t,
                                                              (double*)P.d_ubar, P.d_flags, (double*)sigbar,
                                                              P.d_bload);
     }
     if ((e = cudaGetLastError())) return e;
-    if (load_bar) launch_pdl(P, k_vjp_load_reduce, P.n_inst, 256, 0, st, V.d_pre, P.d_bload, load_bar);
+    if (load_bar) launch_pdl(k_vjp_load_reduce, P.n_inst, 256, 0, st, V.d_pre, P.d_bload, load_bar);
     if ((e = launch_stress_adjoint(P, sigbar, P.d_adj9, st))) return e;
     if (P.precision == CDD_F32) {
         const Axpy<float> ax{1.f, {nullptr, nullptr, nullptr}, {0.f, 0.f, 0.f}};
-        launch_pdl(P, k_vjp_gather<float>, G.blocks, 256, 0, st, P.d_inst, P.n_inst, G.d_pre, (const float*)P.d_ubar, P.d_flags,
+        launch_pdl(k_vjp_gather<float>, G.blocks, 256, 0, st, P.d_inst, P.n_inst, G.d_pre, (const float*)P.d_ubar, P.d_flags,
                                                      (const float*)P.d_adj9, ax, (float*)betabar);
     } else {
         const Axpy<double> ax{1.0, {nullptr, nullptr, nullptr}, {0.0, 0.0, 0.0}};
-        launch_pdl(P, k_vjp_gather<double>, G.blocks, 256, 0, st, P.d_inst, P.n_inst, G.d_pre, (const double*)P.d_ubar,
+        launch_pdl(k_vjp_gather<double>, G.blocks, 256, 0, st, P.d_inst, P.n_inst, G.d_pre, (const double*)P.d_ubar,
                                                       P.d_flags, (const double*)P.d_adj9, ax, (double*)betabar);
     }
     return cudaGetLastError();

@@ -192,7 +192,7 @@ k_c2r_rows(const InstDev* __restrict__ insts, int n_inst,
 template <typename T, bool MEAN64>
 static void c2r_t(const PlanCore& P, const LaunchShape& L, void* out, int mode, int ncomp, const void* beta, int epi, cudaStream_t st) {
     typedef typename VecOf<T>::type V;
-#define CDD_LAUNCH_R(TIER) launch_pdl(P, k_c2r_rows<T, MEAN64, TIER>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, (const V*)P.d_spec, (T*)out, \
+#define CDD_LAUNCH_R(TIER) launch_pdl(k_c2r_rows<T, MEAN64, TIER>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, (const V*)P.d_spec, (T*)out, \
         (const V*)P.d_tw, P.d_sbar, mode, ncomp, (const T*)beta, epi, P.d_clock)
     if (P.rows_tier == 0) CDD_LAUNCH_R(0);
     else if (P.rows_tier == 1) CDD_LAUNCH_R(1);

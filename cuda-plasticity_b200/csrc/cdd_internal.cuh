@@ -859,15 +859,14 @@ inline void set_two_pass(LinePlan& lp) {
 inline bool pass_big(const LinePlan& lp) { return lp.pa && (lp.A > 16 || lp.B > 16); }
 inline int rows_tier(const LinePlan& lp, int P) { return rows_io_plan(lp, P) ? 0 : (pass_big(lp) ? 2 : 1); }
 
-// Programmatic dependent launch (launch_pdl): a kernel starts while the one before it in the stream runs its last
-// blocks, prepares what no kernel writes (instance table, twiddle rows, barriers), and then waits for that
-// one to have finished and its writes to be visible. Only then does it let its own successor start: let go
-// earlier, the successors pile up on the SMs that drain first (96^3 FP32 step 573 us instead of 557).
-// Every block of every kernel waits, also those with nothing to do: a kernel that finished without waiting
-// would let its successor past its predecessor.
-__device__ __forceinline__ void pdl_wait() {
-    asm volatile("griddepcontrol.wait;\n griddepcontrol.launch_dependents;" ::: "memory");
-}
+// Programmatic dependent launch (launch_pdl): a kernel's blocks start as the blocks of the one before it in the
+// stream end, prepare what no kernel writes (instance table, twiddle rows, barriers), and then wait for that
+// kernel to have finished and its writes to be visible. Every block of every kernel waits, also those
+// with nothing to do: a kernel that finished without waiting would let its successor past its predecessor.
+// No kernel lets its successor start before its own blocks end (griddepcontrol.launch_dependents): those blocks
+// would pile up on the SMs that drain first and hold them at the carve-out of the kernel before (measured:
+// 256^3 FP64 step 13.28 -> 13.72 ms, 512^2 FP32 226 -> 256 us).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Find the instance that owns global block b, given prefix sums pre[0..n] of blocks.
 __device__ __forceinline__ int find_instance(const int* __restrict__ pre, int n, int b) {
@@ -936,16 +935,11 @@ struct PlanCore {
     void* d_f1b = nullptr;
 };
 
-// Launch on a plan's stream. Programmatic (see pdl_wait) where launches cost most: calls outside a stream capture
-// (24^3 FP32 step 152 -> 115 us, 32^3 FP64 stress 33 -> 19, 128^3 FP32 step 1028 -> 992) and the graphs of small
-// plans (2-D 128^2 FP64 step 85 -> 78 us). In larger plans' graphs, whose nodes follow one another in about a
-// microsecond anyway, it costs more than it gives (64^3 FP64 step 340 -> 354 us, 512^2 FP32 226 -> 255: blocks
-// that start under a kernel with a large shared-memory carve-out run with little L1).
+// Programmatic launch (see pdl_wait) on a plan's stream, captured or not. Plain -> programmatic: eager 24^3 FP32
+// step 151 -> 111 us, 32^3 FP64 stress 33 -> 20, 96^3 FP32 step 614 -> 562, 256^3 FP32 step 6555 -> 6502; in
+// graphs, whose nodes follow one another within about a microsecond anyway, 0 to 4%.
 template <typename... K, typename... A>
-inline cudaError_t launch_pdl(const PlanCore& P, void (*kernel)(K...), dim3 grid, unsigned threads, size_t smem,
-                              cudaStream_t st, A&&... args) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    const bool known = cudaStreamIsCapturing(st, &cap) == cudaSuccess;
+inline cudaError_t launch_pdl(void (*kernel)(K...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A&&... args) {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -955,7 +949,7 @@ inline cudaError_t launch_pdl(const PlanCore& P, void (*kernel)(K...), dim3 grid
     c.dynamicSmemBytes = smem;
     c.stream = st;
     c.attrs = at;
-    c.numAttrs = (known && (cap == cudaStreamCaptureStatusNone || P.cells <= 65536)) ? 1 : 0;
+    c.numAttrs = 1;
     return cudaLaunchKernelEx(&c, kernel, static_cast<K>(args)...);
 }
 

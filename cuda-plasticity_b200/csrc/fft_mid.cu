@@ -98,10 +98,10 @@ static void mid_t(const PlanCore& P, const LaunchShape& L, int ncomp, int vac_on
     typedef typename VecOf<T>::type V;
     const int pass = INV ? PASS_MID_I : PASS_MID_F;
     if (P.big_mid)
-        launch_pdl(P, k_fft_mid<T, INV, true>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, (V*)P.d_spec, (const V*)P.d_tw,
+        launch_pdl(k_fft_mid<T, INV, true>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, (V*)P.d_spec, (const V*)P.d_tw,
                                                                      pass, ncomp, vac_only);
     else
-        launch_pdl(P, k_fft_mid<T, INV, false>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, (V*)P.d_spec, (const V*)P.d_tw,
+        launch_pdl(k_fft_mid<T, INV, false>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, (V*)P.d_spec, (const V*)P.d_tw,
                                                                       pass, ncomp, vac_only);
 }
 

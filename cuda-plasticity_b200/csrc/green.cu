@@ -523,7 +523,7 @@ static void green_t(const PlanCore& P, const LaunchShape& L, int gmode, bool mea
     typedef typename VecOf<T>::type V;
     const int tier = (P.green_lean && gmode <= 1) ? 0 : (P.big_green ? 2 : 1);
 #define CDD_LAUNCH_G(TIER)                                                                                              \
-    launch_pdl(P, k_green<T, TIER>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, gmode, mean64, (V*)P.d_spec,      \
+    launch_pdl(k_green<T, TIER>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, gmode, mean64, (V*)P.d_spec,      \
                                                           (const V*)P.d_tw, (const T*)ktab, (V*)phi, part, P.d_clock)
     if (tier == 0) CDD_LAUNCH_G(0);
     else if (tier == 1) CDD_LAUNCH_G(1);

@@ -191,7 +191,6 @@ extern "C" int cdd_stress_noalloc(const cdd_instance* d, int precision, const vo
     P.n_inst = 1;
     P.precision = precision;
     P.any3d = (I.nd == 3);
-    P.cells = I.cells;
     P.big_mid = (I.nd == 3) && pass_big(I.lp_mid);
     P.big_green = pass_big(I.lp_first);
     size_t smem_need = 48 * 1024;

@@ -150,7 +150,7 @@ k_r2c_rows(const InstDev* __restrict__ insts, int n_inst,
 template <typename T, bool MEAN64>
 static void r2c_t(const PlanCore& P, const LaunchShape& L, const void* in, double* rowsum, int mode, int ncomp, cudaStream_t st) {
     typedef typename VecOf<T>::type V;
-#define CDD_LAUNCH_R(TIER) launch_pdl(P, k_r2c_rows<T, MEAN64, TIER>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, (const T*)in, (V*)P.d_spec, \
+#define CDD_LAUNCH_R(TIER) launch_pdl(k_r2c_rows<T, MEAN64, TIER>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, (const T*)in, (V*)P.d_spec, \
         (const V*)P.d_tw, rowsum, mode, ncomp)
     if (P.rows_tier == 0) CDD_LAUNCH_R(0);
     else if (P.rows_tier == 1) CDD_LAUNCH_R(1);

@@ -1373,7 +1373,7 @@ static void stencil_dispatch(const PlanCore& P, int mode, const void* bs, const 
     // the plan has such instances
     const int var = (P.any_glide ? 1 : 0) | (P.any_vac ? 2 : 0);
 #define CDD_LAUNCH_V(M, V, SP)                                                                           \
-    launch_pdl(P, k_stencil<T, M, V>, L.blocks, st_threads<T>(), L.smem, st, P.d_inst, P.n_inst, L.d_pre, b, n, o, s, SP,     \
+    launch_pdl(k_stencil<T, M, V>, L.blocks, st_threads<T>(), L.smem, st, P.d_inst, P.n_inst, L.d_pre, b, n, o, s, SP,     \
                                                              P.d_clock, t, P.d_bmax, P.d_bsum, P.d_status,    \
                                                              (const T*)P.d_vac, maps)
 #define CDD_LAUNCH_ST(M, SP)                                  \
@@ -1396,7 +1396,7 @@ static void stencil_dispatch(const PlanCore& P, int mode, const void* bs, const 
 template <typename T>
 static cudaError_t vac_pre_t(const PlanCore& P, const void* beta, cudaStream_t st) {
     const LaunchShape& L = P.obs;
-    launch_pdl(P, k_vac_trace<T>, L.blocks, L.threads, 0, st, P.d_inst, P.n_inst, L.d_pre, (const T*)beta, (T*)P.d_vtr);
+    launch_pdl(k_vac_trace<T>, L.blocks, L.threads, 0, st, P.d_inst, P.n_inst, L.d_pre, (const T*)beta, (T*)P.d_vtr);
     return cudaGetLastError();
 }
 
@@ -1407,7 +1407,7 @@ cudaError_t launch_vacancy_pre(const PlanCore& P, const void* beta, cudaStream_t
 template <typename T>
 static cudaError_t vac_post_t(const PlanCore& P, const void* beta, cudaStream_t st) {
     const LaunchShape& L = P.obs;
-    launch_pdl(P, k_vac_update<T>, L.blocks, L.threads, 0, st, P.d_inst, P.n_inst, L.d_pre, (const T*)beta,
+    launch_pdl(k_vac_update<T>, L.blocks, L.threads, 0, st, P.d_inst, P.n_inst, L.d_pre, (const T*)beta,
                                                     (const T*)P.d_vtr, (T*)P.d_vac, P.d_clock);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -1497,12 +1497,12 @@ __global__ void k_set_clock(InstClock* __restrict__ clk, int n_inst, double t) {
 }
 
 cudaError_t launch_set_clock(const PlanCore& P, double t, cudaStream_t st) {
-    launch_pdl(P, k_set_clock, (P.n_inst + 127) / 128, 128, 0, st, P.d_clock, P.n_inst, t);
+    launch_pdl(k_set_clock, (P.n_inst + 127) / 128, 128, 0, st, P.d_clock, P.n_inst, t);
     return cudaGetLastError();
 }
 
 cudaError_t launch_dt(const PlanCore& P, int fixed, double dt_fixed, cudaStream_t st) {
-    launch_pdl(P, k_dt, P.n_inst, 1024, 0, st, P.d_inst, P.stencil.d_pre, P.d_bmax, P.d_bsum, P.d_clock, P.d_obs,
+    launch_pdl(k_dt, P.n_inst, 1024, 0, st, P.d_inst, P.stencil.d_pre, P.d_bmax, P.d_bsum, P.d_clock, P.d_obs,
                                    P.d_status, fixed, dt_fixed);
     return cudaGetLastError();
 }
@@ -1510,10 +1510,10 @@ cudaError_t launch_dt(const PlanCore& P, int fixed, double dt_fixed, cudaStream_
 cudaError_t launch_axpy_f0(const PlanCore& P, const void* u, void* rhs_f0, cudaStream_t st) {
     const LaunchShape& L = P.cellwise;
     if (P.precision == CDD_F32)
-        launch_pdl(P, k_axpy_f0<float>, L.blocks, 256, 0, st, P.d_inst, P.n_inst, L.d_pre, (const float*)u,
+        launch_pdl(k_axpy_f0<float>, L.blocks, 256, 0, st, P.d_inst, P.n_inst, L.d_pre, (const float*)u,
                                                    (float*)rhs_f0, P.d_clock);
     else
-        launch_pdl(P, k_axpy_f0<double>, L.blocks, 256, 0, st, P.d_inst, P.n_inst, L.d_pre, (const double*)u,
+        launch_pdl(k_axpy_f0<double>, L.blocks, 256, 0, st, P.d_inst, P.n_inst, L.d_pre, (const double*)u,
                                                     (double*)rhs_f0, P.d_clock);
     return cudaGetLastError();
 }
@@ -1521,12 +1521,12 @@ cudaError_t launch_axpy_f0(const PlanCore& P, const void* u, void* rhs_f0, cudaS
 cudaError_t launch_observe(const PlanCore& P, const void* beta, cudaStream_t st) {
     const LaunchShape& L = P.obs;
     if (P.precision == CDD_F32)
-        launch_pdl(P, k_observe<float>, L.blocks, 256, 0, st, P.d_inst, P.n_inst, L.d_pre, (const float*)beta,
+        launch_pdl(k_observe<float>, L.blocks, 256, 0, st, P.d_inst, P.n_inst, L.d_pre, (const float*)beta,
                                                          (const float*)P.d_sigma, P.d_bsum);
     else
-        launch_pdl(P, k_observe<double>, L.blocks, 256, 0, st, P.d_inst, P.n_inst, L.d_pre, (const double*)beta,
+        launch_pdl(k_observe<double>, L.blocks, 256, 0, st, P.d_inst, P.n_inst, L.d_pre, (const double*)beta,
                                                           (const double*)P.d_sigma, P.d_bsum);
-    launch_pdl(P, k_obs_reduce, P.n_inst, 256, 0, st, P.d_inst, P.obs.d_pre, P.d_bsum, P.d_obs);
+    launch_pdl(k_obs_reduce, P.n_inst, 256, 0, st, P.d_inst, P.obs.d_pre, P.d_bsum, P.d_obs);
     return cudaGetLastError();
 }
 

@@ -413,19 +413,19 @@ static cudaError_t run_stress(const PlanCore& P, const void* beta, void* sigma, 
         if (e != cudaSuccess) return e;
     }
     if (plane && u)
-        launch_pdl(P, k_plane_fwd<float, true>, P.plane.blocks, P.plane.threads, P.plane.smem, st, 
+        launch_pdl(k_plane_fwd<float, true>, P.plane.blocks, P.plane.threads, P.plane.smem, st, 
             P.d_inst, P.n_inst, P.plane.d_pre, (const float*)beta, spec, tw, P.d_rowsum, (float*)beta, (const float*)u,
             P.d_clock);
     else if (plane)
-        launch_pdl(P, k_plane_fwd<float, false>, P.plane.blocks, P.plane.threads, P.plane.smem, st, 
+        launch_pdl(k_plane_fwd<float, false>, P.plane.blocks, P.plane.threads, P.plane.smem, st, 
             P.d_inst, P.n_inst, P.plane.d_pre, (const float*)beta, spec, tw, P.d_rowsum, nullptr, nullptr, nullptr);
     if (LR[PASS_R2C].blocks > 0) launch_r2c(P, LR[PASS_R2C], beta, f32 ? P.d_rowsum : nullptr, RS_SYM, 6, st);
-    if (f32) launch_pdl(P, k_mean_beta, dim3(P.n_inst, 6, MEAN_SPLIT), 1024, 0, st, P.d_inst, P.d_rowsum, P.d_sbar);
+    if (f32) launch_pdl(k_mean_beta, dim3(P.n_inst, 6, MEAN_SPLIT), 1024, 0, st, P.d_inst, P.d_rowsum, P.d_sbar);
     launch_mid(P, LR[PASS_MID_F], false, 6, 0, st);
     launch_green(P, P.pass[PASS_GREEN], 0, f32, P.d_k, phi, nullptr, st);
     launch_mid(P, LR[PASS_MID_I], true, 6, 0, st);
     if (plane)
-        launch_pdl(P, k_plane_inv<float>, P.plane.blocks, P.plane.threads, P.plane.smem, st, 
+        launch_pdl(k_plane_inv<float>, P.plane.blocks, P.plane.threads, P.plane.smem, st, 
             P.d_inst, P.n_inst, P.plane.d_pre, spec, (float*)sigma, tw, P.d_sbar);
     if (LR[PASS_C2R].blocks > 0) launch_c2r(P, LR[PASS_C2R], sigma, f32, RD_STRESS, 6, nullptr, EPI_NONE, st);
     return cudaGetLastError();
