@@ -18,20 +18,21 @@ namespace cdd {
 
 namespace {
 
+// Offsets of the neighbours at distance 1 and 2 along one axis (a component has fewer than 2^31 cells).
 struct Nbr {
-    long long p1, p2, m1, m2;
+    int p1, p2, m1, m2;
 };
 
-__device__ __forceinline__ Nbr make_nbr(int i, int n, long long stride) {
+__device__ __forceinline__ Nbr make_nbr(int i, int n, int stride) {
     int ip1 = (i + 1 == n) ? 0 : i + 1;
     int ip2 = (ip1 + 1 == n) ? 0 : ip1 + 1;
     int im1 = (i == 0) ? n - 1 : i - 1;
     int im2 = (im1 == 0) ? n - 1 : im1 - 1;
     Nbr r;
-    r.p1 = (long long)(ip1 - i) * stride;
-    r.p2 = (long long)(ip2 - i) * stride;
-    r.m1 = (long long)(im1 - i) * stride;
-    r.m2 = (long long)(im2 - i) * stride;
+    r.p1 = (ip1 - i) * stride;
+    r.p2 = (ip2 - i) * stride;
+    r.m1 = (im1 - i) * stride;
+    r.m2 = (im2 - i) * stride;
     return r;
 }
 
@@ -93,20 +94,24 @@ __device__ __forceinline__ double bsum(double v, double* red) {
 }
 
 constexpr int VJP_THREADS = 128;
+template <typename T> constexpr size_t vjp_smem() { return (size_t)54 * VJP_THREADS * sizeof(T); }   // derivatives
 constexpr int VJP_PARTS = 5;     // per-block partials: <sigbar, sigma>, tr tr, diag sigbar (3)
+
+// Keeps the compiler from carrying values of the shared slots across (it would hold all 54 in registers again).
+__device__ __forceinline__ void vjp_phase() { asm volatile("" ::: "memory"); }
 
 template <typename T, int ND>
 __device__ __forceinline__ void vjp_cell(const InstDev& I, long long cl, bool valid, const T* __restrict__ beta,
                                          const T* __restrict__ sig, const T* __restrict__ gbar, double tload,
                                          T* __restrict__ ubar, uint32_t* __restrict__ flags,
-                                         T* __restrict__ sigbar, double* lsum) {
+                                         T* __restrict__ sigbar, double* lsum, T* us) {
     const long long cells = I.cells;
     Nbr nb[ND];
     {
         int i0, i1, i2;
         cell_coords(cl, ND, I.n1, I.n2, i0, i1, i2);
         if (ND == 3) {
-            nb[0] = make_nbr(i0, I.n0, (long long)I.n1 * I.n2);
+            nb[0] = make_nbr(i0, I.n0, I.n1 * I.n2);
             nb[1] = make_nbr(i1, I.n1, I.n2);
             nb[ND - 1] = make_nbr(i2, I.n2, 1);
         } else {
@@ -118,17 +123,23 @@ __device__ __forceinline__ void vjp_cell(const InstDev& I, long long cl, bool va
     const T* u = beta + I.foff + cl;
 
     // ---------------- forward recomputation ----------------
-    T U[ND][2][9];
+    // the 54 derivatives live in this thread's shared-memory slots (U): in registers, beside their cotangents,
+    // they left 8 warps per SM (FP32) or spilled 2 KB per thread (FP64)
+    auto U = [us](int d, int s, int c) -> T { return us[((2 * d + s) * 9 + c) * VJP_THREADS]; };
     uint32_t fw[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
     for (int c = 0; c < 9; ++c)
 #pragma unroll
         for (int d = 0; d < ND; ++d) {
             int sp, sm;
-            derivs_sel(u + (long long)c * cells, nb[d], ih, U[d][0][c], U[d][1][c], sp, sm);
+            T up, um;
+            derivs_sel(u + (long long)c * cells, nb[d], ih, up, um, sp, sm);
+            us[(2 * d * 9 + c) * VJP_THREADS] = up;
+            us[((2 * d + 1) * 9 + c) * VJP_THREADS] = um;
             const int slot = c * 3 + d;
             fw[slot >> 3] |= (uint32_t)(sp | (sm << 2)) << (4 * (slot & 7));
         }
+    vjp_phase();
     double add[3] = {0.0, 0.0, 0.0};
     if (I.has_load) {
         double eps[3];
@@ -166,13 +177,13 @@ __device__ __forceinline__ void vjp_cell(const InstDev& I, long long cl, bool va
                 T a = 0;
 #pragma unroll
                 for (int n = 0; n < 3; ++n) {
-                    const T v = U[d][s][3 * l + n];
+                    const T v = U(d, s, 3 * l + n);
                     a += v * S[d][n];
                     sd += v * S[l][n];
                     if (l != d) pq += v * v;
                 }
                 A[d][s][l] = a;
-                tu += U[d][s][4 * l];
+                tu += U(d, s, 4 * l);
             }
             A[d][s][d] -= sd;
             trU[d][s] = tu;
@@ -180,7 +191,7 @@ __device__ __forceinline__ void vjp_cell(const InstDev& I, long long cl, bool va
             if (lam_on) {
                 A[d][s][d] += str * tu;
 #pragma unroll
-                for (int l = 0; l < 3; ++l) A[d][s][l] -= str * U[d][s][3 * l + d];
+                for (int l = 0; l < 3; ++l) A[d][s][l] -= str * U(d, s, 3 * l + d);
             }
         }
 #pragma unroll
@@ -191,11 +202,11 @@ __device__ __forceinline__ void vjp_cell(const InstDev& I, long long cl, bool va
             for (int b = 0; b < 2; ++b) {
                 T acc = 0;
 #pragma unroll
-                for (int j = 0; j < 3; ++j) acc += U[pd[p]][a][3 * pe[p] + j] * U[pe[p] % ND][b][3 * pd[p] + j];
+                for (int j = 0; j < 3; ++j) acc += U(pd[p], a, 3 * pe[p] + j) * U(pe[p] % ND, b, 3 * pd[p] + j);
                 Cp[p][a][b] = acc;
             }
     constexpr int NC = 1 << ND;
-    T V[NC][3], As[NC][3], rr[NC];
+    T V[NC][3], rr[NC];
     int sg[NC][3];
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
@@ -213,7 +224,6 @@ __device__ __forceinline__ void vjp_cell(const InstDev& I, long long cl, bool va
             T a = 0;
 #pragma unroll
             for (int d = 0; d < ND; ++d) a += A[d][sg[c][d]][l];
-            As[c][l] = a;
             V[c][l] = a * rr[c];
         }
     }
@@ -264,112 +274,74 @@ __device__ __forceinline__ void vjp_cell(const InstDev& I, long long cl, bool va
     T coef[ND];
 #pragma unroll
     for (int d = 0; d < ND; ++d) coef[d] = pm[d] * pp[d] / tot[d];
-    T hs[9];
-    T Jp = 0;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            T h = 0;
-#pragma unroll
-            for (int d = 0; d < ND; ++d) h += Q[d][0][d] * U[d][0][3 * i + j] + Q[d][1][d] * U[d][1][3 * i + j];
-            if (i < ND) {
-#pragma unroll
-                for (int s = 0; s < 2; ++s)
-#pragma unroll
-                    for (int l = 0; l < 3; ++l) h -= Q[i % ND][s][l] * U[i % ND][s][3 * l + j];
-            }
-            hs[3 * i + j] = h;
-        }
-    if (lam_on) {
-#pragma unroll
-        for (int d = 0; d < ND; ++d)
-#pragma unroll
-            for (int s = 0; s < 2; ++s) Jp += Q[d][s][d] * trU[d][s];
-#pragma unroll
-        for (int j = 0; j < ND; ++j)
-#pragma unroll
-            for (int s = 0; s < 2; ++s)
-#pragma unroll
-                for (int l = 0; l < 3; ++l) Jp -= Q[j][s][l] * U[j][s][3 * l + j];
-    }
-    const T J = -Lam / (T)3 * Jp;
-
+    vjp_phase();
     // ---------------- reverse ----------------
+    // rhs_ij = -hs_ij inv_abc + sum_d (U+ - U-)_ij coef_d  [- J inv_abc on the diagonal]. First the cotangents
+    // of Q, coef and inv_abc, then those of the corners, A, P and C; the 54 derivatives' cotangents are formed last,
+    // each from these in one go, and stored at once.
     T gb[9];
     const T* gp = gbar + I.foff + cl;
 #pragma unroll
     for (int c = 0; c < 9; ++c) gb[c] = (valid && gbar) ? gp[c * cells] : (T)0;
-    T Ub[ND][2][9];
-#pragma unroll
-    for (int d = 0; d < ND; ++d)
-#pragma unroll
-        for (int s = 0; s < 2; ++s)
-#pragma unroll
-            for (int c = 0; c < 9; ++c) Ub[d][s][c] = 0;
-    T Qb[ND][2][3], trUb[ND][2], coefb[ND];
+    T Qb[ND][2][3], coefb[ND];
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
         coefb[d] = 0;
 #pragma unroll
-        for (int s = 0; s < 2; ++s) {
-            trUb[d][s] = 0;
+        for (int s = 0; s < 2; ++s)
 #pragma unroll
             for (int l = 0; l < 3; ++l) Qb[d][s][l] = 0;
-        }
     }
-    // rhs_ij = -hs_ij inv_abc + sum_d (U+ - U-)_ij coef_d  [- J inv_abc on the diagonal]
     T inv_abc_b = 0;
-    T gdiag = gb[0] + gb[4] + gb[8];
-#pragma unroll
-    for (int c = 0; c < 9; ++c) inv_abc_b -= gb[c] * hs[c];
-    if (lam_on) inv_abc_b -= J * gdiag;
-    const T Jpb = lam_on ? (-inv_abc * gdiag) * (-Lam / (T)3) : (T)0;
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             const int c = 3 * i + j;
             const T vb = gb[c];
-            const T hb = -gb[c] * inv_abc;
+            const T hb = -vb * inv_abc;
+            T h = 0;   // hs_ij
 #pragma unroll
             for (int d = 0; d < ND; ++d) {
-                Ub[d][0][c] += vb * coef[d];
-                Ub[d][1][c] -= vb * coef[d];
-                coefb[d] += vb * (U[d][0][c] - U[d][1][c]);
-                Qb[d][0][d] += hb * U[d][0][c];
-                Ub[d][0][c] += hb * Q[d][0][d];
-                Qb[d][1][d] += hb * U[d][1][c];
-                Ub[d][1][c] += hb * Q[d][1][d];
+                const T u0 = U(d, 0, c), u1 = U(d, 1, c);
+                h += Q[d][0][d] * u0 + Q[d][1][d] * u1;
+                coefb[d] += vb * (u0 - u1);
+                Qb[d][0][d] += hb * u0;
+                Qb[d][1][d] += hb * u1;
             }
             if (i < ND) {
 #pragma unroll
                 for (int s = 0; s < 2; ++s)
 #pragma unroll
                     for (int l = 0; l < 3; ++l) {
-                        Qb[i % ND][s][l] -= hb * U[i % ND][s][3 * l + j];
-                        Ub[i % ND][s][3 * l + j] -= hb * Q[i % ND][s][l];
+                        const T v = U(i % ND, s, 3 * l + j);
+                        h -= Q[i % ND][s][l] * v;
+                        Qb[i % ND][s][l] -= hb * v;
                     }
             }
+            inv_abc_b -= vb * h;
         }
+    const T gdiag = gb[0] + gb[4] + gb[8];
+    const T Jpb = lam_on ? (-inv_abc * gdiag) * (-Lam / (T)3) : (T)0;
     if (lam_on) {
+        T Jp = 0;   // J = -Lambda / 3 Jp
 #pragma unroll
         for (int d = 0; d < ND; ++d)
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
-                Qb[d][s][d] += Jpb * trU[d][s];
-                trUb[d][s] += Jpb * Q[d][s][d];
-            }
-#pragma unroll
-        for (int j = 0; j < ND; ++j)
-#pragma unroll
-            for (int s = 0; s < 2; ++s)
+                const T tu = U(d, s, 0) + U(d, s, 4) + U(d, s, 8);
+                Jp += Q[d][s][d] * tu;
+                Qb[d][s][d] += Jpb * tu;
 #pragma unroll
                 for (int l = 0; l < 3; ++l) {
-                    Qb[j][s][l] -= Jpb * U[j][s][3 * l + j];
-                    Ub[j][s][3 * l + j] -= Jpb * Q[j][s][l];
+                    const T v = U(d, s, 3 * l + d);
+                    Jp -= Q[d][s][l] * v;
+                    Qb[d][s][l] -= Jpb * v;
                 }
+            }
+        inv_abc_b -= -Lam / (T)3 * Jp * gdiag;
     }
+    vjp_phase();
     T ppb[ND], pmb[ND], totb[ND];
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
@@ -377,37 +349,34 @@ __device__ __forceinline__ void vjp_cell(const InstDev& I, long long cl, bool va
         ppb[d] = coefb[d] * pm[d] / tot[d];
         totb[d] = -coefb[d] * coef[d] / tot[d] - inv_abc_b * inv_abc / tot[d];
     }
-    T Vb[NC][3];
+    auto weight = [&](int c, int skip) {   // product of a corner's weights but axis `skip`
+        T ww = 1;
+#pragma unroll
+        for (int d = 0; d < ND; ++d)
+            if (d != skip) ww *= (sg[c][d] == 0) ? pm[d] : pp[d];
+        return ww;
+    };
+    auto qsum = [&](int c, int l) {   // cotangent of w_c V_cl
+        T q = 0;
+#pragma unroll
+        for (int d = 0; d < ND; ++d) q += Qb[d][sg[c][d]][l];
+        return q;
+    };
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
         T wb = 0;
 #pragma unroll
-        for (int l = 0; l < 3; ++l) {
-            T q = 0;
-#pragma unroll
-            for (int d = 0; d < ND; ++d) q += Qb[d][sg[c][d]][l];
-            wb += q * V[c][l];
-            Vb[c][l] = q * w[c];
-        }
+        for (int l = 0; l < 3; ++l) wb += qsum(c, l) * V[c][l];
 #pragma unroll
         for (int d = 0; d < ND; ++d) {
-            T others = 1;
-#pragma unroll
-            for (int e = 0; e < ND; ++e)
-                if (e != d) others *= (sg[c][e] == 0) ? pm[e] : pp[e];
-            if (sg[c][d] == 0) pmb[d] += wb * others;
-            else ppb[d] += wb * others;
+            if (sg[c][d] == 0) pmb[d] += wb * weight(c, d);
+            else ppb[d] += wb * weight(c, d);
         }
     }
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
         ppb[d] += totb[d];
         pmb[d] += totb[d];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            if (c == cmx[d]) Vb[c][d] += ppb[d];
-            if (c == cmn[d]) Vb[c][d] -= pmb[d];
-        }
     }
     T Ab[ND][2][3], Pb[ND][2], Cpb[NP][2][2];
 #pragma unroll
@@ -426,75 +395,70 @@ __device__ __forceinline__ void vjp_cell(const InstDev& I, long long cl, bool va
             for (int b = 0; b < 2; ++b) Cpb[p][a][b] = 0;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-        T rb = 0;
+        const T wc = weight(c, -1);
+        T rb = 0;   // V_c . its cotangent
 #pragma unroll
         for (int l = 0; l < 3; ++l) {
-            rb += Vb[c][l] * As[c][l];
-            const T asb = Vb[c][l] * rr[c];
+            T vb = qsum(c, l) * wc;
+            if (l < ND) {
+                if (c == cmx[l % ND]) vb += ppb[l % ND];
+                if (c == cmn[l % ND]) vb -= pmb[l % ND];
+            }
+            rb += vb * V[c][l];
+            const T asb = vb * rr[c];
 #pragma unroll
             for (int d = 0; d < ND; ++d) Ab[d][sg[c][d]][l] += asb;
         }
-        const T rho2b = rb * (T)-0.5 * rr[c] * rr[c] * rr[c];
+        const T rho2b = (T)-0.5 * rb * (rr[c] * rr[c]);
 #pragma unroll
         for (int d = 0; d < ND; ++d) Pb[d][sg[c][d]] += rho2b;
 #pragma unroll
         for (int p = 0; p < NP; ++p) Cpb[p][sg[c][pd[p]]][sg[c][pe[p] % ND]] -= (T)2 * rho2b;
     }
-    // P, C -> U
-#pragma unroll
-    for (int d = 0; d < ND; ++d)
-#pragma unroll
-        for (int s = 0; s < 2; ++s)
-#pragma unroll
-            for (int l = 0; l < 3; ++l)
-                if (l != d) {
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) Ub[d][s][3 * l + j] += (T)2 * U[d][s][3 * l + j] * Pb[d][s];
-                }
-#pragma unroll
-    for (int p = 0; p < NP; ++p)
-#pragma unroll
-        for (int a = 0; a < 2; ++a)
-#pragma unroll
-            for (int b = 0; b < 2; ++b)
-#pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    const T cb = Cpb[p][a][b];
-                    Ub[pd[p]][a][3 * pe[p] + j] += cb * U[pe[p] % ND][b][3 * pd[p] + j];
-                    Ub[pe[p] % ND][b][3 * pd[p] + j] += cb * U[pd[p]][a][3 * pe[p] + j];
-                }
-    // A -> U, S
+    vjp_phase();
     T Sb[3][3];
 #pragma unroll
     for (int m = 0; m < 3; ++m)
 #pragma unroll
         for (int n = 0; n < 3; ++n) Sb[m][n] = 0;
     T strb = 0;
+    T* ub = ubar ? ubar + 54 * I.coff + cl : nullptr;
 #pragma unroll
     for (int d = 0; d < ND; ++d)
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
             const T sdb = -Ab[d][s][d];
+            const T ghd = (s == 0 ? coef[d] : -coef[d]) - inv_abc * Q[d][s][d];
+            T trub = 0;
+            if (lam_on) {
+                trub = Jpb * Q[d][s][d] + Ab[d][s][d] * str;
+                strb += Ab[d][s][d] * (U(d, s, 0) + U(d, s, 4) + U(d, s, 8));
+            }
 #pragma unroll
             for (int l = 0; l < 3; ++l)
 #pragma unroll
                 for (int n = 0; n < 3; ++n) {
-                    const T v = U[d][s][3 * l + n];
-                    Ub[d][s][3 * l + n] += Ab[d][s][l] * S[d][n] + sdb * S[l][n];
+                    const T v = U(d, s, 3 * l + n);
+                    T a = gb[3 * l + n] * ghd + gb[3 * d + n] * (inv_abc * Q[d][s][l]);
+                    if (l != d) a += (T)2 * v * Pb[d][s];
+                    if (l != d && l < ND) {   // C: the pair of axes d and l
+                        const int p = (ND == 3) ? ((l == (d + 1) % 3) ? d : l) : 0;
+#pragma unroll
+                        for (int b = 0; b < 2; ++b)
+                            a += (pd[p] == d ? Cpb[p][s][b] : Cpb[p][b][s]) * U(l % ND, b, 3 * d + n);
+                    }
+                    a += Ab[d][s][l] * S[d][n] + sdb * S[l][n];
                     Sb[d][n] += Ab[d][s][l] * v;
                     Sb[l][n] += sdb * v;
+                    if (lam_on) {
+                        if (n == d) {
+                            a -= Jpb * Q[d][s][l] + Ab[d][s][l] * str;
+                            strb -= Ab[d][s][l] * v;
+                        }
+                        if (l == n) a += trub;
+                    }
+                    if (ub && valid) ub[(long long)((2 * d + s) * 9 + 3 * l + n) * cells] = a;
                 }
-            if (lam_on) {
-                strb += Ab[d][s][d] * trU[d][s];
-                trUb[d][s] += Ab[d][s][d] * str;
-#pragma unroll
-                for (int l = 0; l < 3; ++l) {
-                    strb -= Ab[d][s][l] * U[d][s][3 * l + d];
-                    Ub[d][s][3 * l + d] -= Ab[d][s][l] * str;
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 3; ++j) Ub[d][s][4 * j] += trUb[d][s];
         }
     if (lam_on) {
 #pragma unroll
@@ -522,15 +486,6 @@ __device__ __forceinline__ void vjp_cell(const InstDev& I, long long cl, bool va
         lsum[3] += sb6[3];
         lsum[4] += sb6[5];
     }
-    if (ubar) {
-        T* ub = ubar + 54 * I.coff + cl;
-#pragma unroll
-        for (int d = 0; d < ND; ++d)
-#pragma unroll
-            for (int s = 0; s < 2; ++s)
-#pragma unroll
-                for (int c = 0; c < 9; ++c) ub[(long long)((2 * d + s) * 9 + c) * cells] = Ub[d][s][c];
-    }
     // Word 3 holds the selections of slots 24..26 in bits 0..11; bits 12..31 record the corners
     // that attain the directional max / min speeds (index + 1, 0 = the zero entry), base 9.
     {
@@ -549,14 +504,20 @@ __device__ __forceinline__ void vjp_cell(const InstDev& I, long long cl, bool va
     for (int q = 0; q < 4; ++q) fl[(long long)q * cells] = fw[q];
 }
 
+// Bound by instruction issue (FP32: 5600 warp instructions per 32 cells, 55% of the slots, with instruction-cache
+// misses of its 90 KB of code as the largest stall). Four FP32 blocks per SM (128 registers) instead of two,
+// two FP64 ones with 0.4 KB of spills instead of 2 KB; the reverse of one step at 64^3 FP32 583 -> 525 us (with
+// k_param_reduce), 32^3 FP64 223 -> 181. Three FP32 blocks without spills: 250 us per VJP against 213.
 template <typename T>
-__global__ void __launch_bounds__(VJP_THREADS) k_vjp_cells(const InstDev* __restrict__ insts, int n_inst,
+__global__ void __launch_bounds__(VJP_THREADS, sizeof(T) == 4 ? 4 : 2) k_vjp_cells(const InstDev* __restrict__ insts, int n_inst,
                                                            const int* __restrict__ pre,
                                                            const T* __restrict__ beta, const T* __restrict__ sig,
                                                            const T* __restrict__ gbar, double t,
                                                            T* __restrict__ ubar, uint32_t* __restrict__ flags,
                                                            T* __restrict__ sigbar, double* __restrict__ bload) {
     __shared__ double red[VJP_THREADS / 32];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T* us = reinterpret_cast<T*>(smem_raw) + threadIdx.x;
     const int ii = find_instance(pre, n_inst, blockIdx.x);
     const InstDev& I = insts[ii];
     const long long cell = (long long)(blockIdx.x - pre[ii]) * VJP_THREADS + threadIdx.x;
@@ -564,36 +525,14 @@ __global__ void __launch_bounds__(VJP_THREADS) k_vjp_cells(const InstDev* __rest
     pdl_wait();
     double lsum[VJP_PARTS] = {0.0, 0.0, 0.0, 0.0, 0.0};
     if (I.nd == 3)
-        vjp_cell<T, 3>(I, valid ? cell : 0, valid, beta, sig, gbar, t, ubar, flags, sigbar, lsum);
+        vjp_cell<T, 3>(I, valid ? cell : 0, valid, beta, sig, gbar, t, ubar, flags, sigbar, lsum, us);
     else
-        vjp_cell<T, 2>(I, valid ? cell : 0, valid, beta, sig, gbar, t, ubar, flags, sigbar, lsum);
+        vjp_cell<T, 2>(I, valid ? cell : 0, valid, beta, sig, gbar, t, ubar, flags, sigbar, lsum, us);
     if (!sigbar) return;
 #pragma unroll
     for (int i = 0; i < VJP_PARTS; ++i) {
         double s = bsum<T>(lsum[i], red);
         if (threadIdx.x == 0) bload[VJP_PARTS * blockIdx.x + i] = s;
-    }
-}
-
-// Coefficient of u_q (q = -2..2) in u+ * h (selection sp) and in u- * h (selection sm).
-__device__ __forceinline__ float coef_p(int q, int s) {
-    const float a = (s == 1) ? 1.f : 0.f, b = (s == 2) ? 1.f : 0.f;
-    switch (q) {
-        case -1: return -0.5f * b;
-        case 0: return -1.f - 0.5f * a + b;
-        case 1: return 1.f + a - 0.5f * b;
-        case 2: return -0.5f * a;
-        default: return 0.f;
-    }
-}
-__device__ __forceinline__ float coef_m(int q, int s) {
-    const float a = (s == 1) ? 1.f : 0.f, b = (s == 2) ? 1.f : 0.f;
-    switch (q) {
-        case -2: return 0.5f * b;
-        case -1: return -1.f + 0.5f * a - b;
-        case 0: return 1.f - a + 0.5f * b;
-        case 1: return 0.5f * a;
-        default: return 0.f;
     }
 }
 
@@ -615,7 +554,7 @@ __device__ __forceinline__ void gather_cell(const InstDev& I, long long y, const
         int i0, i1, i2;
         cell_coords(y, ND, I.n1, I.n2, i0, i1, i2);
         if (ND == 3) {
-            nb[0] = make_nbr(i0, I.n0, (long long)I.n1 * I.n2);
+            nb[0] = make_nbr(i0, I.n0, I.n1 * I.n2);
             nb[1] = make_nbr(i1, I.n1, I.n2);
             nb[ND - 1] = make_nbr(i2, I.n2, 1);
         } else {
@@ -626,32 +565,39 @@ __device__ __forceinline__ void gather_cell(const InstDev& I, long long y, const
     const T ih = (T)I.inv_h;
     const T* ub = ubar + 54 * I.coff + y;
     const uint32_t* fl = flags + 4 * I.coff + y;
-    // neighbour-major: the four selection words of each of the 5 ND neighbours are read once; a
-    // one-sided derivative at distance q = -2 (forward) or q = +2 (backward) does not involve y
-    // (coef_p(-2, .) = coef_m(2, .) = 0), so those values are not read
+    // Along one axis u+_x = (d_x - (e_x+1 or e_x or 0) / 2) / h and u-_x = (d_x-1 + (e_x or e_x-1 or 0) / 2) / h with the
+    // differences d_x = u_x+1 - u_x, e_x = u_x+1 - 2 u_x + u_x-1 and the recorded selections, so with the cotangents
+    // P of u+ and M of u-
+    //   D_x = P_x + M_x+1,  E_x = (M_x [1] + M_x+1 [2] - P_x-1 [1] - P_x [2]) / 2   ([k]: selection k at that cell)
+    // and the value's cotangent is D_y-1 - D_y + E_y-1 - 2 E_y + E_y+1: 8 loads and about 45 instructions per component
+    // and axis. (The five cells' coefficients formed one by one took twice the instructions.)
     T acc[9];
 #pragma unroll
     for (int c = 0; c < 9; ++c) acc[c] = 0;
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
-        // cell x = y - q holds y at offset q
-        const long long off[5] = {nb[d].p2, nb[d].p1, 0, nb[d].m1, nb[d].m2};   // q = -2 .. 2
+        const int off[5] = {nb[d].m2, nb[d].m1, 0, nb[d].p1, nb[d].p2};   // cells y-2 .. y+2
+        uint32_t fw[5][4];
 #pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            const int q = k - 2;
-            const long long x = off[k];
-            uint32_t fw[4];
+        for (int k = 0; k < 5; ++k)
 #pragma unroll
-            for (int w = 0; w < 4; ++w) fw[w] = fl[x + (long long)w * cells];
-            const T* up = ub + x + (long long)(2 * d * 9) * cells;
+            for (int w = 0; w < 4; ++w) fw[k][w] = (fl + (long long)w * cells)[off[k]];
+#pragma unroll
+        for (int c = 0; c < 9; ++c) {
+            const T* up = ub + (long long)(2 * d * 9 + c) * cells;
             const T* um = up + 9 * cells;
+            const int slot = c * 3 + d, w = slot >> 3, bit = 4 * (slot & 7);
+            T P[5], M[5];   // P at y-2 .. y+1, M at y-1 .. y+2
 #pragma unroll
-            for (int c = 0; c < 9; ++c) {
-                const int slot = c * 3 + d;
-                const uint32_t f = (fw[slot >> 3] >> (4 * (slot & 7))) & 15u;
-                if (q > -2) acc[c] += up[(long long)c * cells] * (T)coef_p(q, (int)(f & 3u));
-                if (q < 2) acc[c] += um[(long long)c * cells] * (T)coef_m(q, (int)(f >> 2));
-            }
+            for (int k = 0; k < 4; ++k) P[k] = up[off[k]];
+#pragma unroll
+            for (int k = 1; k < 5; ++k) M[k] = um[off[k]];
+            auto p = [&](int k, int sel) { return (fw[k][w] >> (bit + sel - 1)) & 1u ? P[k] : (T)0; };
+            auto m = [&](int k, int sel) { return (fw[k][w] >> (bit + sel + 1)) & 1u ? M[k] : (T)0; };
+            const T em = (m(1, 1) + m(2, 2)) - (p(0, 1) + p(1, 2));   // 2 E_y-1, 2 E_y, 2 E_y+1
+            const T e0 = (m(2, 1) + m(3, 2)) - (p(1, 1) + p(2, 2));
+            const T ep = (m(3, 1) + m(4, 2)) - (p(2, 1) + p(3, 2));
+            acc[c] += ((P[1] + M[2]) - (P[2] + M[3])) + ((T)0.5 * (em + ep) - e0);
         }
     }
 #pragma unroll
@@ -700,50 +646,52 @@ __global__ void __launch_bounds__(256) k_vjp_load_reduce(const int* __restrict__
 // doubles per instance): [0] <sigbar, sigma_int>, [1] tr sigbar . tr sigma_int, [2] the k-space
 // sum of the nu derivative per unit dA (from the green-block partials), [3..5] the diagonal of
 // sigbar (load), [6..8] the same times (t - load_t0).
+// One block per instance and sum (blockIdx.y; one block for all six took 14 us at 64^3).
 __global__ void __launch_bounds__(256) k_param_reduce(const InstDev* __restrict__ insts,
                                                       const int* __restrict__ pre_v, const double* __restrict__ bpart,
                                                       const int* __restrict__ pre_g, const double* __restrict__ gpart,
                                                       double c, double t, double* __restrict__ pbar) {
     __shared__ double red[8];
-    const int ii = blockIdx.x;
+    const int ii = blockIdx.x, i = blockIdx.y;
+    const bool k = i == VJP_PARTS;   // the k-space sum
+    const int* pre = k ? pre_g : pre_v;
+    const int b0 = pre[ii], b1 = pre[ii + 1];
     pdl_wait();
-    double v[VJP_PARTS + 1];
-    for (int i = 0; i < VJP_PARTS; ++i) {
-        double acc = 0.0;
-        for (int b = pre_v[ii] + threadIdx.x; b < pre_v[ii + 1]; b += blockDim.x) acc += bpart[VJP_PARTS * b + i];
-        v[i] = bsum<double>(acc, red);
+    const double* src = k ? gpart : bpart + i;
+    const int stride = k ? 1 : VJP_PARTS;
+    double acc = 0.0;
+    if (src) {
+#pragma unroll 4
+        for (int b = b0 + threadIdx.x; b < b1; b += 256) acc += src[(long long)stride * b];
     }
-    {
-        double acc = 0.0;
-        if (gpart)
-            for (int b = pre_g[ii] + threadIdx.x; b < pre_g[ii + 1]; b += blockDim.x) acc += gpart[b];
-        v[VJP_PARTS] = bsum<double>(acc, red);
-    }
+    const double v = bsum<double>(acc, red);
     if (threadIdx.x == 0) {
         double* o = pbar + CDD_PBAR * ii;
-        const double tl = t - insts[ii].load_t0;
-        o[0] += c * v[0];
-        o[1] += c * v[1];
-        o[2] += c * v[5];
-        for (int i = 0; i < 3; ++i) {
-            o[3 + i] += c * v[2 + i];
-            o[6 + i] += c * tl * v[2 + i];
+        if (k) o[2] += c * v;
+        else if (i < 2) o[i] += c * v;
+        else {
+            o[1 + i] += c * v;
+            o[4 + i] += c * (t - insts[ii].load_t0) * v;
         }
     }
 }
 
 }  // namespace
 
+cudaError_t adjoint_set_attributes(int precision) {
+    return precision == CDD_F32 ? set_dyn_smem_limit(k_vjp_cells<float>, SIZE_MAX) : set_dyn_smem_limit(k_vjp_cells<double>, SIZE_MAX);
+}
+
 cudaError_t launch_flux_branches(const PlanCore& P, const void* beta, double t, uint32_t* flags, cudaStream_t st) {
     const LaunchShape& V = P.vjp;
     cudaError_t e;
     if ((e = launch_stress(P, beta, P.d_sigma, st))) return e;
     if (P.precision == CDD_F32)
-        launch_pdl(k_vjp_cells<float>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const float*)beta,
+        launch_pdl(k_vjp_cells<float>, V.blocks, VJP_THREADS, vjp_smem<float>(), st, P.d_inst, P.n_inst, V.d_pre, (const float*)beta,
                                                             (const float*)P.d_sigma, nullptr, t, nullptr, flags,
                                                             nullptr, P.d_bload);
     else
-        launch_pdl(k_vjp_cells<double>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const double*)beta,
+        launch_pdl(k_vjp_cells<double>, V.blocks, VJP_THREADS, vjp_smem<double>(), st, P.d_inst, P.n_inst, V.d_pre, (const double*)beta,
                                                              (const double*)P.d_sigma, nullptr, t, nullptr, flags,
                                                              nullptr, P.d_bload);
     return cudaGetLastError();
@@ -757,11 +705,11 @@ cudaError_t launch_vjp_stage(const PlanCore& P, const void* v, const void* sig_v
     cudaError_t e;
     const bool f32 = (P.precision == CDD_F32);
     if (f32)
-        launch_pdl(k_vjp_cells<float>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const float*)v,
+        launch_pdl(k_vjp_cells<float>, V.blocks, VJP_THREADS, vjp_smem<float>(), st, P.d_inst, P.n_inst, V.d_pre, (const float*)v,
                                                             (const float*)sig_v, (const float*)gbar, t,
                                                             (float*)P.d_ubar, P.d_flags, (float*)P.d_sb6, P.d_bload);
     else
-        launch_pdl(k_vjp_cells<double>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const double*)v,
+        launch_pdl(k_vjp_cells<double>, V.blocks, VJP_THREADS, vjp_smem<double>(), st, P.d_inst, P.n_inst, V.d_pre, (const double*)v,
                                                              (const double*)sig_v, (const double*)gbar, t,
                                                              (double*)P.d_ubar, P.d_flags, (double*)P.d_sb6,
                                                              P.d_bload);
@@ -769,7 +717,7 @@ cudaError_t launch_vjp_stage(const PlanCore& P, const void* v, const void* sig_v
     if ((e = launch_stress_adjoint(P, P.d_sb6, P.d_adj9, st, pbar ? phi_v : nullptr, pbar ? P.d_gpart : nullptr)))
         return e;
     if (pbar) {
-        launch_pdl(k_param_reduce, P.n_inst, 256, 0, st, P.d_inst, V.d_pre, P.d_bload, P.pass[PASS_GREEN].d_pre,
+        launch_pdl(k_param_reduce, dim3(P.n_inst, VJP_PARTS + 1), 256, 0, st, P.d_inst, V.d_pre, P.d_bload, P.pass[PASS_GREEN].d_pre,
                                                  phi_v ? P.d_gpart : nullptr, c, t, pbar);
         if ((e = cudaGetLastError())) return e;
     }
@@ -793,11 +741,11 @@ cudaError_t launch_flux_vjp(const PlanCore& P, const void* beta, double t, const
     cudaError_t e;
     if ((e = launch_stress(P, beta, P.d_sigma, st))) return e;
     if (P.precision == CDD_F32) {
-        launch_pdl(k_vjp_cells<float>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const float*)beta,
+        launch_pdl(k_vjp_cells<float>, V.blocks, VJP_THREADS, vjp_smem<float>(), st, P.d_inst, P.n_inst, V.d_pre, (const float*)beta,
                                                             (const float*)P.d_sigma, (const float*)gbar, t,
                                                             (float*)P.d_ubar, P.d_flags, (float*)sigbar, P.d_bload);
     } else {
-        launch_pdl(k_vjp_cells<double>, V.blocks, VJP_THREADS, 0, st, P.d_inst, P.n_inst, V.d_pre, (const double*)beta,
+        launch_pdl(k_vjp_cells<double>, V.blocks, VJP_THREADS, vjp_smem<double>(), st, P.d_inst, P.n_inst, V.d_pre, (const double*)beta,
                                                              (const double*)P.d_sigma, (const double*)gbar, t,
                                                              (double*)P.d_ubar, P.d_flags, (double*)sigbar,
                                                              P.d_bload);

@@ -971,6 +971,7 @@ cudaError_t launch_stress_adjoint(const PlanCore& P, const void* sigbar6, void* 
                                   const void* phi = nullptr, double* part = nullptr);
 cudaError_t launch_stress_dnu(const PlanCore& P, const void* beta, void* out6, cudaStream_t st);
 // adjoint.cu
+cudaError_t adjoint_set_attributes(int precision);
 cudaError_t launch_flux_branches(const PlanCore& P, const void* beta, double t, uint32_t* flags, cudaStream_t st);
 // One stage of the reverse sweep: out = c L_v^T g + sum a_k x_k (x_k may be null), with v's stress
 // sig_v and k-space phi_v precomputed; parameter cotangents (scaled by c) added to pbar if non-null.

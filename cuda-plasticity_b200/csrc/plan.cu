@@ -1034,6 +1034,7 @@ int ensure_adjoint_scratch(cdd_plan* p) {
         (e = dalloc(p, &C.d_f0b, elt * (size_t)C.field_elems)) ||
         (e = dalloc(p, &C.d_f1b, elt * (size_t)C.field_elems)))
         return fail(CDD_ERR_ALLOC, "adjoint scratch: %s", cudaGetErrorString(e));
+    CDD_CUDA(adjoint_set_attributes(C.precision));
     return CDD_OK;
 }
 
