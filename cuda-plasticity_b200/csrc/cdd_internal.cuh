@@ -1023,7 +1023,7 @@ inline cudaError_t set_dyn_smem_limit(F* fn, size_t smem) {
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v);
 }
 size_t stencil_smem_bytes(int precision, bool any3d);
-int stencil_default_planes(const InstDev* insts, int n, int precision, int resident);
+int stencil_default_planes(const InstDev* insts, int n, int precision, int sms);
 void stencil_geometry(InstDev& I, int precision, int planes);
 cudaError_t stress_set_attributes(int precision, size_t max_smem);
 // Axis-1 pass: 128-byte row segments (16 columns FP32, 8 FP64), one radix-16 butterfly per thread at 256.

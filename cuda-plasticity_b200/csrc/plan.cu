@@ -190,7 +190,7 @@ int build_shapes(cdd_plan* p, size_t elt) {
         cudaDeviceGetAttribute(&optin_dev, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     }
-    const int st_planes = stencil_default_planes(p->inst.data(), n, C.precision, 2 * (sms > 0 ? sms : 148));   // 2 blocks per SM
+    const int st_planes = stencil_default_planes(p->inst.data(), n, C.precision, sms > 0 ? sms : 148);
     for (int i = 0; i < n; ++i) {
         InstDev& I = p->inst[i];
         // rows kernels (R2C: 9 components, C2R: 6); ping-pong buffers of P padded rows

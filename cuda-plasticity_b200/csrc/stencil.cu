@@ -50,22 +50,33 @@ template <> struct TileGeom<float> { static constexpr int RX = 40, OX = 4, NS = 
 template <> struct TileGeom<double> { static constexpr int RX = 36, OX = 2, NS = 5, TY = 4; };
 template <typename T> __host__ __device__ constexpr int tile_ry() { return TileGeom<T>::TY + 4; }
 template <typename T> __host__ __device__ constexpr int st_threads() { return TXS * TileGeom<T>::TY; }
+constexpr int ST_BLOCKS = 2;   // per SM
 template <typename T> __host__ __device__ constexpr int tile_pp() { return tile_ry<T>() * TileGeom<T>::RX; }   // per component
 
+// What a block keeps of beta_s. FP32 3-D: a ring of plane boxes. FP64 3-D: the box of the current plane only, and
+// for each thread the five values z-2 .. z+2 of its own column (`column`), which it copies and reads back itself:
+// a block starts after one box instead of five (FP64 flux at one plane per block, 128^3: 532 -> 361 us, 64^3 60 ->
+// 54 us). Its 73 KB would let three blocks run, but at the 168 registers that leaves each thread the spills
+// cost more than the warps give (256^3 2.65 ms against 1.65; 160-thread blocks at 200 registers 2.50).
+template <typename T, int ND> __host__ __device__ constexpr bool own_columns() { return sizeof(T) == 8 && ND == 3; }
 template <typename T, int ND>
 struct TileView {
     static constexpr int RX = TileGeom<T>::RX, PP = tile_pp<T>();
+    static constexpr bool OWN = own_columns<T, ND>();
     const T* sm;       // shared memory base
-    int so[5];         // element offsets of the ring planes z-2 .. z+2 (3-D); so[2] = current plane
+    const T* column;   // this thread's column slots (own_columns)
+    int so[5];         // element offsets of the planes z-2 .. z+2 (3-D), in sm or column; so[2] = current plane
     int idx;           // in-plane offset of this thread's cell (halo included)
-    __device__ __forceinline__ T center(int c) const { return sm[so[2] + c * PP + idx]; }
+    __device__ __forceinline__ T center(int c) const {
+        return OWN ? column[so[2] + c * st_threads<T>()] : sm[so[2] + c * PP + idx];
+    }
     __device__ __forceinline__ void load5(int c, int d, T* v) const {
         if (ND == 3 && d == 0) {
 #pragma unroll
-            for (int q = 0; q < 5; ++q) v[q] = sm[so[q] + c * PP + idx];
+            for (int q = 0; q < 5; ++q) v[q] = OWN ? column[so[q] + c * st_threads<T>()] : sm[so[q] + c * PP + idx];
         } else {
             const int st = (d == ND - 1) ? 1 : RX;
-            const T* p = sm + so[2] + c * PP + idx;
+            const T* p = sm + (OWN ? 0 : so[2]) + c * PP + idx;
             v[0] = p[-2 * st]; v[1] = p[-st]; v[2] = p[0]; v[3] = p[st]; v[4] = p[2 * st];
         }
     }
@@ -456,7 +467,7 @@ __device__ __forceinline__ void flux_f32(const TileView<float, ND>& tv, float ih
 // by 8 resident warps per SM to hide its latency. All 54 derivatives stay in registers (246, no spills), formed
 // once: forming them again for the rhs, with the five-compare minmod, 8 square roots and 8 + 4 divisions
 // of the form before it, took 4272 us per 256^3 flux, this 2704 us; with the plane copies under the cell's own
-// work (march) and 20 planes per block, 1796 us.
+// work (march) and 20 planes per block, 1796 us; with own columns and Newton's rsqrt and reciprocal, 1649 us.
 // d + h minmod(e, m) for h = -1/2 or 1/2: the factor is 0 unless the signs of e and m agree (an integer test),
 // and times the smaller magnitude otherwise, so the FP64 pipe sees one compare and one multiply-add. A NaN in
 // e (two cells away) leaves m, as minmod's 0 leaves d: only the cells whose d or m is NaN become NaN.
@@ -471,6 +482,23 @@ __device__ __forceinline__ void derivs5_f64(const double* v, double& up, double&
     const double e0 = d1 - d0, em1 = d0 - dm1, em2 = dm1 - dm2;
     up = limited_f64(d0, e0, em1, -0.5);
     um = limited_f64(dm1, em2, em1, 0.5);
+}
+
+// 1 / sqrt(x) and 1 / x of normal positive x: the hardware's approximations (about 2^-22) and Newton's iteration,
+// y <- y + y (1 - x y^2) / 2 and y <- y + y (1 - x y), twice: no branches, unlike the library's, whose special
+// cases cannot occur here (x >= ME Dx^2, x >= ME; 0 or NaN results for infinite or NaN x as NaN).
+__device__ __forceinline__ double rsqrt_f64(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double h = 0.5 * y, e = fma(-x * y, y, 1.0);
+    y = fma(h, e, y);
+    return fma(0.5 * y, fma(-x * y, y, 1.0), y);
+}
+__device__ __forceinline__ double rcp_f64(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    y = fma(y, fma(-x, y, 1.0), y);
+    return fma(y, fma(-x, y, 1.0), y);
 }
 
 // meh: ME Dx^2. ring_read(): called once the thread has read all it needs of the ring but its cell's own
@@ -541,7 +569,7 @@ __device__ __forceinline__ bool flux_f64(const TileView<double, ND>& tv, double 
         const int sz = (ND == 3) ? (c & 1) : 0;
         double r2 = fma(-2.0, Cp[0][sx][sy], meh + Pq[0][sx] + Pq[1][sy]);
         if (ND == 3) r2 = fma(-2.0, Cp[1 % NP][sy][sz] + Cp[2 % NP][sz][sx], r2 + Pq[2 % ND][sz]);
-        const double inv = rsqrt(r2);
+        const double inv = rsqrt_f64(r2);
         double av[3];
 #pragma unroll
         for (int l = 0; l < 3; ++l) {
@@ -577,18 +605,19 @@ __device__ __forceinline__ bool flux_f64(const TileView<double, ND>& tv, double 
     spd = 0.0;
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
-        double mx = 0.0, mn = 0.0;
+        double mx = 0.0, mn = 0.0, sum = 0.0;
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
             mx = V[c][d] > mx ? V[c][d] : mx;
             mn = V[c][d] < mn ? V[c][d] : mn;
-            vsum += V[c][d];
+            sum += V[c][d];
         }
+        vsum += sum;
         pp[d] = mx;
         pm[d] = -mn;
         const double tot = pp[d] + pm[d] + ME;
         spd += tot;
-        const double it = 1.0 / tot;
+        const double it = rcp_f64(tot);
         wm[d] = pm[d] * it;
         wp[d] = pp[d] * it;
     }
@@ -954,8 +983,8 @@ __device__ __forceinline__ void box_async(T* dst, const BoxGeomT<T>& g, int zp) 
 // narrower) copies with wrapped addresses (box_async). (A TMA copy of an edge tile would need its
 // out-of-grid cells patched once it has landed, by loads whose latency nothing hides: 30% of the FP64 flux
 // at 128^3, where half of the tiles are at an edge.)
-// FP32 (6 slots) requests plane z+3 as cell z starts. FP64 (5 slots, two blocks of 110 KB) requests it into the
-// slot of plane z-2 once the whole block has formed its derivatives, so the copy runs under the
+// FP32 (6 box slots) requests plane z+3 as cell z starts. FP64 (one box, own columns) requests the box of plane
+// z+1 and the columns' plane z+3 once the whole block has formed its derivatives, so the copies run under the
 // corner and rhs work of the same cell; that barrier also collects the verdict of the bounded waits.
 template <typename T, int ND, int MODE, int VAR>
 __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, double* red, uint64_t* bars,
@@ -967,7 +996,10 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
                                       int* __restrict__ status, const T* __restrict__ vac) {
     constexpr int RX = TileGeom<T>::RX, OX = TileGeom<T>::OX, PP = tile_pp<T>();
     constexpr int TYS = TileGeom<T>::TY, RY = tile_ry<T>(), ST_THREADS = st_threads<T>();
-    constexpr int NS = (ND == 3) ? TileGeom<T>::NS : 1;
+    constexpr bool OWN = own_columns<T, ND>();
+    constexpr int NB = (ND == 3 && !OWN) ? TileGeom<T>::NS : 1;      // plane boxes
+    constexpr int NS = OWN ? TileGeom<T>::NS : NB;                   // slots of the five planes z-2 .. z+2
+    constexpr int SP = OWN ? 9 * ST_THREADS : 9 * PP;                // elements per slot
     constexpr uint32_t PLANE_BYTES = 9u * PP * sizeof(T);
     const int nZ = (ND == 3) ? I.n0 : 1;
     const int nY = (ND == 3) ? I.n1 : I.n0;
@@ -998,7 +1030,7 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
     __shared__ BoxGeomT<T> bg;
     if (use_tma && tid == 0) {
 #pragma unroll 1
-        for (int s = 0; s < NS; ++s) mbar_init(&bars[s], 1);
+        for (int s = 0; s < NB; ++s) mbar_init(&bars[s], 1);
         fence_mbar_init();
     }
     pdl_wait();
@@ -1007,33 +1039,60 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
         bg = {src, cells, x0, y0, nX, nY, nZ, ND == 3 ? z0 - 2 : 0, box_chunk<T>(src, nX)};
     }
     __syncthreads();
-    // plane with relative index pr (= z - (z0 - 2)) lives in slot pr % NS
-    auto issue = [&](int pr) {   // TMA, one thread
-        const int slot = pr % NS;
+    // Box n: the plane with relative index n (= z - (z0 - 2)), or with own columns the n-th cell's (relative
+    // index n + 2); it lives in box slot n % NB.
+    constexpr int REL = OWN ? 2 : 0;
+    auto issue = [&](int n) {   // TMA, one thread
+        const int slot = n % NB;
         mbar_expect_tx(&bars[slot], PLANE_BYTES);
         tma_load_5d(sm + slot * 9 * PP, &maps.m[I.tma_slot], &bars[slot], bg.x0 - OX, bg.y0 - 2,
-                    bg.plane_of(pr), 0, I.tma_sub);
+                    bg.plane_of(n + REL), 0, I.tma_sub);
     };
-    auto stage = [&](int pr) {   // asynchronous copies, all threads
-        box_async<T>(sm + (pr % NS) * 9 * PP, bg, bg.plane_of(pr));
+    auto stage = [&](int n) {   // asynchronous copies, all threads
+        box_async<T>(sm + (n % NB) * 9 * PP, bg, bg.plane_of(n + REL));
         cp_async_commit();
     };
-    auto landed = [&](int pr) { return mbar_wait(&bars[pr % NS], (uint32_t)((pr / NS) & 1)); };
+    auto landed = [&](int n) { return mbar_wait(&bars[n % NB], (uint32_t)((n / NB) & 1)); };
+    // own columns: the thread's nine values of the next plane (relative index 0, 1, ...), to the next slot
+    T* column = sm + NB * 9 * PP + tid;
+    const T* col_src = nullptr;
+    int col_z = 0, col_slot = 0;
+    if constexpr (OWN) {
+        col_z = bg.plane_of(0);
+        col_src = bg.src + (long long)col_z * plane + (vxy ? y * nX + x : 0);
+    }
+    auto column_async = [&]() {
+        T* d = column + col_slot;
+#pragma unroll
+        for (int c = 0; c < 9; ++c) cp_async_elem(d + c * ST_THREADS, col_src + c * cells);
+        cp_async_commit();
+        col_slot = (col_slot + SP == NS * SP) ? 0 : col_slot + SP;
+        col_src += plane;
+        if (++col_z == nZ) {
+            col_z = 0;
+            col_src -= cells;
+        }
+    };
 
-    constexpr int NPL = (ND == 3) ? 5 : 1;   // planes z0-2 .. z0+2 (3-D), the plane (2-D)
-    int issued = -1;   // highest plane index handed to TMA
+    constexpr int NPL = (ND == 3 && !OWN) ? 5 : 1;   // first boxes: planes z0-2 .. z0+2, or the current plane
+    int issued = -1;   // last box handed to TMA
     int ok = 1;        // block-uniform: every plane waited for has arrived
     if (use_tma) {
         if (tid == 0)
-            for (int pr = 0; pr < NPL; ++pr) issue(pr);
+            for (int n = 0; n < NPL; ++n) issue(n);
         issued = NPL - 1;
     } else {
 #pragma unroll 1
-        for (int pr = 0; pr < NPL; ++pr) stage(pr);
+        for (int n = 0; n < NPL; ++n) stage(n);
+    }
+    if constexpr (OWN) {
+#pragma unroll 1
+        for (int q = 0; q < 5; ++q) column_async();
     }
     Stage1Acc<T> sums;
     // FP32: this thread's FP64 sum slots after the stress slots
-    double* acc = reinterpret_cast<double*>(sm + NS * 9 * PP + 6 * ST_THREADS) + tid;
+    T* ssm = sm + NB * 9 * PP + (OWN ? NS * SP : 0) + tid;
+    double* acc = reinterpret_cast<double*>(ssm - tid + 6 * ST_THREADS) + tid;
     if (MODE == M_STAGE1) sums.start(acc, ST_THREADS);
     // this thread's cell in plane z0 (cell (z0, 0, 0) for threads outside the grid: in-bounds
     // loads, no stores)
@@ -1052,9 +1111,9 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
     }
     TileView<T, ND> tv;
     tv.sm = sm;
+    tv.column = column;
     tv.idx = (ty + 2) * RX + tx + OX;
-    // the stress of the thread's cell, one plane ahead, in shared memory after the ring
-    T* ssm = sm + NS * 9 * PP + tid;
+    // the stress of the thread's cell, one plane ahead, in its shared-memory slots after the planes
 #pragma unroll
     for (int c = 0; c < 6; ++c) cp_async_elem(ssm + c * ST_THREADS, cx.sig + c * cells);
     cp_async_commit();
@@ -1064,7 +1123,7 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
     bool got = true;   // this thread saw every plane of the coming cell arrive
     if (use_tma) {
 #pragma unroll 1
-        for (int pr = 0; pr < NPL; ++pr) got &= landed(pr);
+        for (int n = 0; n < NPL; ++n) got &= landed(n);
     }
     // FP32 stage updates read beta_n of their cell after the flux (no registers to hold it across): its rows
     // of the next plane are requested into L2 a plane ahead, one 128-byte row of 32 cells per thread for
@@ -1081,28 +1140,29 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
             }
             return ok != 0;
         };
-        auto request = [&]() {   // plane k + 5
+        const int next = OWN ? k + 1 : k + 5;   // box to request
+        auto request = [&]() {
             if (use_tma) {
                 if (tid == 0) {
                     fence_proxy_async();
-                    issue(k + 5);
+                    issue(next);
                 }
-                issued = k + 5;
+                issued = next;
             } else {
-                stage(k + 5);
+                stage(next);
             }
         };
-        if (NS != 5 && use_tma && !verdict()) break;
-        if (NS == 6 && use_tma && more) request();
+        if (!OWN && use_tma && !verdict()) break;
+        if (ND == 3 && !OWN && use_tma && more) request();
         if (ND == 3) {
             // ring planes z-2 .. z+2 live in slots (k + q) mod NS, rotated by one plane per step
             if (k == 0) {
 #pragma unroll
-                for (int q = 0; q < 5; ++q) tv.so[q] = q * 9 * PP;
+                for (int q = 0; q < 5; ++q) tv.so[q] = q * SP;
             } else {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) tv.so[q] = tv.so[q + 1];
-                tv.so[4] = (tv.so[3] + 9 * PP == NS * 9 * PP) ? 0 : tv.so[3] + 9 * PP;
+                tv.so[4] = (tv.so[3] + SP == NS * SP) ? 0 : tv.so[3] + SP;
             }
         } else {
             tv.so[2] = 0;
@@ -1114,10 +1174,11 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
             }
         }
         auto early = [&]() {   // FP32: the staged copies of plane k + 5, after the stress copies' wait
-            if (NS == 6 && !use_tma && more) stage(k + 5);
+            if (ND == 3 && !OWN && !use_tma && more) stage(next);
         };
         auto ring_read = [&]() {   // FP64
-            if (NS != 5) return true;
+            if (!OWN) return true;
+            if (more) column_async();   // plane z + 3, into the slot of z - 2 that this thread has read
             if (use_tma) {
                 if (!verdict()) return false;
             } else if (more) {
@@ -1135,7 +1196,7 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
         if (cx.spd) cx.spd += plane;
         if (ND == 3 && more) {
             if (use_tma) {
-                got = landed(k + 5);
+                got = landed(next);
             } else {
                 cp_async_wait_own();
                 __syncthreads();
@@ -1145,7 +1206,7 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
     cp_async_wait_own();   // no copy in flight past here
     if (!ok) {
         // a copy did not land in time: let every copy this block issued finish (bounded), then leave
-        for (int pr = max(0, issued - NS + 1); pr <= issued; ++pr) landed(pr);
+        for (int n = max(0, issued - NB + 1); n <= issued; ++n) landed(n);
         return;
     }
     if (MODE == M_STAGE1) {
@@ -1161,7 +1222,7 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
 }
 
 template <typename T, int MODE, int VAR>
-__global__ void __launch_bounds__(st_threads<T>(), 2)
+__global__ void __launch_bounds__(st_threads<T>(), ST_BLOCKS)
 k_stencil(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ pre,
           const T* __restrict__ bs, const T* bn, T* out, const T* __restrict__ sig,
           T* __restrict__ speed_out, const InstClock* __restrict__ clk, double t_flux,
@@ -1550,12 +1611,12 @@ cudaError_t stencil_set_attributes(int precision, size_t smem) {
     return precision == CDD_F32 ? st_attr<float>(smem) : st_attr<double>(smem);
 }
 
-// The plane ring plus the 6 stress slots of every thread (FP32: and its two FP64 sum slots).
+// The plane boxes and columns plus the 6 stress slots of every thread (FP32: and its two FP64 sum slots).
 size_t stencil_smem_bytes(int precision, bool any3d) {
     if (precision == CDD_F32)
         return ((size_t)(any3d ? TileGeom<float>::NS : 1) * 9 * tile_pp<float>() + 6 * st_threads<float>()) * sizeof(float) +
                2 * st_threads<float>() * sizeof(double);
-    return ((size_t)(any3d ? TileGeom<double>::NS : 1) * 9 * tile_pp<double>() + 6 * st_threads<double>()) * sizeof(double);
+    return ((size_t)9 * tile_pp<double>() + ((any3d ? TileGeom<double>::NS * 9 : 0) + 6) * st_threads<double>()) * sizeof(double);
 }
 
 static int stencil_tiles(const InstDev& I, int precision) {
@@ -1565,26 +1626,27 @@ static int stencil_tiles(const InstDev& I, int precision) {
     return ((nX + TXS - 1) / TXS) * ((nY + TYS - 1) / TYS);
 }
 
-// Planes per block (one value for all 3-D instances of a plan). A block costs its planes and about c0 = 0.9
-// planes' time for staging the first five (flux form at 256^3, planes per block 1 / 2 / 4 / 8 / 16: FP64 3456 /
-// 2561 / 2110 / 1900 / 1815 us, FP32 1589 / 1176 / 983 / 894 / 863 us); `resident` blocks run at once. Many
-// short blocks pay c0 often, few long ones leave SMs idle (small grids) or a long tail: the sum of both
-// estimates is minimised. At least 8 planes per block whatever the grid, the rule before, gave one 32^3 FP64
-// flux 32 blocks and 50 us, against 25 us at one plane per block.
-int stencil_default_planes(const InstDev* insts, int n, int precision, int resident) {
-    const double c0 = 0.9;
+// Planes per block (one value for all 3-D instances of a plan). A block costs its planes and about c0 planes'
+// time for its start (flux form at 256^3, planes per block 1 / 2 / 4 / 8 / 24: FP64 2565 / 2107 / 1837 / 1712 /
+// 1649 us, FP32 1589 / 1180 / 982 / 894 / 851 us); two blocks per SM run at once, and a block alone on its SM takes
+// about 0.7 of the time. Many short blocks pay c0 often, few long ones leave SMs idle (small grids) or a tail
+// (a share of a block): the estimate is minimised. At least 8 planes per block whatever the grid, the rule
+// before, gave one 32^3 FP64 flux 32 blocks and 50 us, against 25 us at one plane per block.
+int stencil_default_planes(const InstDev* insts, int n, int precision, int sms) {
+    const double c0 = precision == CDD_F32 ? 0.9 : 0.55, tail = precision == CDD_F32 ? 0.2 : 0.4;
+    const int resident = ST_BLOCKS * sms;
     int best = 1;
     double best_cost = 1e300;
     for (int z = 1; z <= 64; ++z) {
         double sum = 0.0, longest = 0.0, blocks = 0.0;
         for (int i = 0; i < n; ++i) {
-            const int nZ = (insts[i].nd == 3) ? insts[i].n0 : 1, len = z < nZ ? z : nZ;
+            const int nZ = (insts[i].nd == 3) ? insts[i].n0 : 1, len = (nZ + (nZ + z - 1) / z - 1) / ((nZ + z - 1) / z);
             const double b = (double)stencil_tiles(insts[i], precision) * ((nZ + len - 1) / len);
             blocks += b;
             sum += b * c0 + (double)stencil_tiles(insts[i], precision) * nZ;
             if (len + c0 > longest) longest = len + c0;
         }
-        const double cost = blocks <= resident ? longest : sum / resident + 0.5 * longest;
+        const double cost = blocks <= sms ? 0.7 * longest : (blocks <= resident ? longest : sum / resident + tail * longest);
         if (cost <= best_cost) { best_cost = cost; best = z; }
     }
     return best;
