@@ -913,7 +913,8 @@ struct PlanCore {
     double* d_rowsum = nullptr;      // FP32 path: FP64 per-row sums
     double* d_sbar = nullptr;        // FP32 path: FP64 mean of each beta component (9 per instance)
     double* d_bmax = nullptr;        // per-block wave-speed maxima
-    double* d_bsum = nullptr;        // per-block energy and mean-zz partial sums (2 per block)
+    unsigned* d_done = nullptr;      // per-instance count of finished stage-1 blocks
+    double* d_bsum = nullptr;        // observables: per-block energy and mean-zz partial sums (2 per block)
     double* d_obs = nullptr;         // per-instance energy, mean zz (2 per instance)
     int* d_status = nullptr;
     LaunchShape pass[NUM_PASSES];
@@ -983,12 +984,12 @@ cudaError_t launch_flux_vjp(const PlanCore& P, const void* beta, double t, const
 // stencil.cu
 enum StencilMode { M_FLUX = 0, M_STAGE1 = 1, M_STAGE2 = 2, M_STAGE3 = 3 };
 cudaError_t launch_stencil(const PlanCore& P, int mode, const void* bs, const void* bn, void* out,
-                           void* speed, double t_flux, const StencilMapSet& maps, cudaStream_t st);
+                           void* speed, double t_flux, const StencilMapSet& maps, cudaStream_t st, int fixed = 0,
+                           double dt_fixed = 0.0);   // stage 1 also sets the instances' time steps
 // Encode the tensor maps of buffer `base` for every run of instances with tma_slot >= 0; returns false
 // (and leaves maps disabled) if the driver entry point is missing or an address is misaligned.
 bool encode_stencil_maps(const PlanCore& P, const InstDev* insts, const void* base, StencilMapSet& maps);
 bool stencil_tma_eligible(const InstDev& I, int precision);
-cudaError_t launch_dt(const PlanCore& P, int fixed, double dt_fixed, cudaStream_t st);
 cudaError_t launch_set_clock(const PlanCore& P, double t, cudaStream_t st);
 // Vacancy coupling around a step: save tr(beta^P) before it; after it, c += vac_beta d tr and the
 // diffusion c^ *= exp(-vac_gamma dt k^2) (FFT passes over one component).

@@ -397,6 +397,38 @@ __device__ __forceinline__ void fft_slots(V* s, int n, V* scratch, int lgw, int 
     }
 }
 
+// FP32 stress solves: FP64 mean of each of the six components from the row sums, for the C2R pass's mean stress.
+// The launch's first 6 n_inst blocks, one per instance and component, form them beside the k-space work (a
+// kernel of its own took 5 to 18 us per solve). Fixed order: deterministic.
+struct MeanArgs {
+    int blocks;              // 6 n_inst, or 0
+    const double* rowsum;
+    double* mean9;           // 9 per instance
+};
+__device__ __noinline__ void mean_block(const InstDev& I, int ii, int c, const MeanArgs& a) {
+    __shared__ double red[8];
+    const int tid = threadIdx.x, nt = blockDim.x;
+    pdl_wait();
+    const double* rs = a.rowsum + I.rsoff + (long long)c * I.rows;
+    // eight independent accumulators per thread keep several loads in flight
+    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    int r = tid;
+    for (; r + 7 * nt < I.rows; r += 8 * nt)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[q] += rs[r + q * nt];
+    for (; r < I.rows; r += nt) acc[0] += rs[r];
+    double v = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((tid & 31) == 0) red[tid >> 5] = v;
+    __syncthreads();
+    if (tid == 0) {
+        double sum = 0.0;
+        for (int w = 0; w < (nt >> 5); ++w) sum += red[w];
+        a.mean9[9 * ii + c] = sum * I.inv_cells;
+    }
+}
+
 // Fused k-space pass along axis 0: forward FFT of the input components, contraction (scaled by 1 / cells),
 // inverse FFT of the outputs, in place on the spectrum. A block owns W = 2^lgw spectrum columns (32 bytes) of row
 // i1 (3-D) of one instance and all their components.
@@ -408,20 +440,25 @@ __device__ __forceinline__ void fft_slots(V* s, int n, V* scratch, int lgw, int 
 // on 192 threads). Bound by the latency of its phases and, at FP64, the FP64 pipe.
 template <typename T, int TIER>
 __global__ void __launch_bounds__(sizeof(T) == 4 ? 256 : 192, (TIER == 2 && sizeof(T) == 8) ? 2 : 3)
-k_green(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ pre, int gmode, int mean64,
+k_green(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ pre, int gmode, int mean64, MeanArgs mean,
         typename VecOf<T>::type* __restrict__ spec, const typename VecOf<T>::type* __restrict__ tw,
         const T* __restrict__ ktab, typename VecOf<T>::type* __restrict__ phi, double* __restrict__ part,
         const InstClock* __restrict__ clk) {
     typedef typename VecOf<T>::type V;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V* s = reinterpret_cast<V*>(smem_raw);
-    const int ii = find_instance(pre, n_inst, blockIdx.x);
+    if ((int)blockIdx.x < mean.blocks) {
+        mean_block(insts[blockIdx.x / 6], blockIdx.x / 6, blockIdx.x % 6, mean);
+        return;
+    }
+    const int blk = blockIdx.x - mean.blocks;
+    const int ii = find_instance(pre, n_inst, blk);
     const InstDev& I = insts[ii];
     if (gmode == 7 && !I.vacancy) {
         pdl_wait();
         return;
     }
-    const int lb = blockIdx.x - pre[ii];
+    const int lb = blk - pre[ii];
     const PassTile& tl = I.tile[PASS_GREEN];
     const int lgw = tl.lgw, ta_n = tl.tiles_a;
     const int i1 = lb / ta_n;          // 0 in 2-D
@@ -495,7 +532,7 @@ k_green(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ p
         if (tid == 0) {
             double sum = 0.0;
             for (int w = 0; w < nt / 32; ++w) sum += red[w];
-            part[blockIdx.x] = sum * I.inv_cells;
+            part[blk] = sum * I.inv_cells;
         }
     }
     __syncthreads();
@@ -522,9 +559,10 @@ static void green_t(const PlanCore& P, const LaunchShape& L, int gmode, bool mea
                     cudaStream_t st) {
     typedef typename VecOf<T>::type V;
     const int tier = (P.green_lean && gmode <= 1) ? 0 : (P.big_green ? 2 : 1);
-#define CDD_LAUNCH_G(TIER)                                                                                              \
-    launch_pdl(k_green<T, TIER>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, gmode, mean64, (V*)P.d_spec,      \
-                                                          (const V*)P.d_tw, (const T*)ktab, (V*)phi, part, P.d_clock)
+    const MeanArgs mean{mean64 ? 6 * P.n_inst : 0, P.d_rowsum, P.d_sbar};
+#define CDD_LAUNCH_G(TIER)                                                                                               \
+    launch_pdl(k_green<T, TIER>, L.blocks + mean.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, gmode, mean64, \
+               mean, (V*)P.d_spec, (const V*)P.d_tw, (const T*)ktab, (V*)phi, part, P.d_clock)
     if (tier == 0) CDD_LAUNCH_G(0);
     else if (tier == 1) CDD_LAUNCH_G(1);
     else CDD_LAUNCH_G(2);

@@ -400,8 +400,7 @@ int record_step(cdd_plan* p, void* beta, cudaStream_t st, int fixed, double dt_f
     const StencilMapSet& mu = user_maps(p, beta);
     if (C.any_vac) CDD_CUDA(launch_vacancy_pre(C, beta, st));
     CDD_CUDA(launch_stress(C, beta, C.d_sigma, st));
-    CDD_CUDA(launch_stencil(C, M_STAGE1, beta, beta, C.d_f0, nullptr, 0.0, mu, st));
-    CDD_CUDA(launch_dt(C, fixed, dt_fixed, st));
+    CDD_CUDA(launch_stencil(C, M_STAGE1, beta, beta, C.d_f0, nullptr, 0.0, mu, st, fixed, dt_fixed));
     CDD_CUDA(launch_stress_f0(C, beta, C.d_f0, C.d_sigma, st));
     CDD_CUDA(launch_stencil(C, M_STAGE2, C.d_f0, beta, C.d_f1, nullptr, 0.0, p->maps_f0, st));
     CDD_CUDA(launch_stress(C, C.d_f1, C.d_sigma, st));
@@ -663,7 +662,9 @@ int cdd_plan_create_tuned(const cdd_instance* inst, int n_inst, int precision, c
     if (precision == CDD_F32) ALLOC_OR_FAIL(C.d_rowsum, sizeof(double) * (size_t)C.rows_total);
     ALLOC_OR_FAIL(C.d_sbar, sizeof(double) * 9 * n_inst);
     ALLOC_OR_FAIL(C.d_bmax, sizeof(double) * (size_t)C.stencil.blocks);
-    ALLOC_OR_FAIL(C.d_bsum, sizeof(double) * 2 * (size_t)(C.stencil.blocks > C.obs.blocks ? C.stencil.blocks : C.obs.blocks));
+    ALLOC_OR_FAIL(C.d_bsum, sizeof(double) * 2 * (size_t)C.obs.blocks);
+    ALLOC_OR_FAIL(C.d_done, sizeof(unsigned) * n_inst);
+    cudaMemset(C.d_done, 0, sizeof(unsigned) * n_inst);
     ALLOC_OR_FAIL(C.d_obs, sizeof(double) * 2 * n_inst);
     ALLOC_OR_FAIL(C.d_status, sizeof(int));
     cudaMemset(C.d_status, 0, sizeof(int));
@@ -1130,8 +1131,7 @@ int cdd_step_record(cdd_plan* p, void* beta, double t, double dt, void* rec, voi
     CDD_CUDA(cudaMemcpyAsync(u, beta, elt * (size_t)C.field_elems, cudaMemcpyDeviceToDevice, st));
     CDD_CUDA(launch_stress(C, beta, s_u, st, r + L.pu * elt));
     K.d_sigma = s_u;
-    CDD_CUDA(launch_stencil(K, M_STAGE1, beta, beta, f0, nullptr, 0.0, user_maps(p, beta), st));
-    CDD_CUDA(launch_dt(C, 1, dt, st));
+    CDD_CUDA(launch_stencil(K, M_STAGE1, beta, beta, f0, nullptr, 0.0, user_maps(p, beta), st, 1, dt));
     CDD_CUDA(launch_stress_f0(C, beta, f0, s_f0, st, r + L.pf0 * elt));
     K.d_sigma = s_f0;
     StencilMapSet m0, m1;

@@ -145,15 +145,28 @@ __device__ __forceinline__ void r2c_rows_io(const InstDev& I, int lb, int P, int
         const RowPtr ea = rt[2 * l], eb = rt[2 * l + 1];
         V v[R0];
         double sa = 0.0, sb = 0.0;
+        // rows that are their own partners (diagonal components, stress rows) are read once: 0.5 (x + x) = x
+        if (!F0 && ea.q == ea.p && eb.q == eb.p) {
 #pragma unroll
-        for (int r = 0; r < R0; ++r) {
-            const int i = j + R1 * r;
-            T a = 0, b = 0;
-            if (ea.p >= 0) a = row_value<T, F0>(beta, f0w, u, dt, ea, i);
-            if (eb.p >= 0) b = row_value<T, F0>(beta, f0w, u, dt, eb, i);
-            if (MEAN64) { sa += (double)a; sb += (double)b; }
-            v[r].x = a;
-            v[r].y = b;
+            for (int r = 0; r < R0; ++r) {
+                const int i = j + R1 * r;
+                v[r].x = ea.p >= 0 ? beta[ea.p + i] : (T)0;
+                v[r].y = eb.p >= 0 ? beta[eb.p + i] : (T)0;
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < R0; ++r) {
+                const int i = j + R1 * r;
+                T a = 0, b = 0;
+                if (ea.p >= 0) a = row_value<T, F0>(beta, f0w, u, dt, ea, i);
+                if (eb.p >= 0) b = row_value<T, F0>(beta, f0w, u, dt, eb, i);
+                v[r].x = a;
+                v[r].y = b;
+            }
+        }
+        if (MEAN64) {
+#pragma unroll
+            for (int r = 0; r < R0; ++r) { sa += (double)v[r].x; sb += (double)v[r].y; }
         }
         if (MEAN64) {
 #pragma unroll
@@ -226,15 +239,27 @@ __device__ __forceinline__ void r2c_pass_a(const LinePlan& lp, int P, const RowP
         const RowPtr ea = rt[2 * l], eb = rt[2 * l + 1];
         V v[A];
         double sa = 0.0, sb = 0.0;
+        if (ea.q == ea.p && eb.q == eb.p) {
 #pragma unroll
-        for (int q = 0; q < A; ++q) {
-            const int i = j + B * q;
-            T a = 0, b = 0;
-            if (ea.p >= 0) a = (T)0.5 * (beta[ea.p + i] + beta[ea.q + i]);
-            if (eb.p >= 0) b = (T)0.5 * (beta[eb.p + i] + beta[eb.q + i]);
-            if (MEAN64) { sa += (double)a; sb += (double)b; }
-            v[q].x = a;
-            v[q].y = b;
+            for (int q = 0; q < A; ++q) {
+                const int i = j + B * q;
+                v[q].x = ea.p >= 0 ? beta[ea.p + i] : (T)0;
+                v[q].y = eb.p >= 0 ? beta[eb.p + i] : (T)0;
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < A; ++q) {
+                const int i = j + B * q;
+                T a = 0, b = 0;
+                if (ea.p >= 0) a = (T)0.5 * (beta[ea.p + i] + beta[ea.q + i]);
+                if (eb.p >= 0) b = (T)0.5 * (beta[eb.p + i] + beta[eb.q + i]);
+                v[q].x = a;
+                v[q].y = b;
+            }
+        }
+        if (MEAN64) {
+#pragma unroll
+            for (int q = 0; q < A; ++q) { sa += (double)v[q].x; sb += (double)v[q].y; }
         }
         if (MEAN64) {
             part[2 * g] = sa;

@@ -737,8 +737,6 @@ __device__ __forceinline__ void applied_load(const InstDev& I, double t, double*
 struct StageConst {
     double ld[3];
     double dt;
-    double cnu;   // nu / (1 + nu) of the elastic energy density (|sigma|^2 - cnu tr^2) / (4 mu)
-    float cnu_f;  // the same rounded to FP32 (the FP32 form's per-cell density)
     double meh;   // ME Dx^2 (FP64)
     bool active;
 };
@@ -751,8 +749,6 @@ __device__ __forceinline__ StageConst stage_const(const InstDev& I, const InstCl
     const double tload = (MODE == M_FLUX) ? t_flux : ((MODE == M_STAGE1) ? ck.t : ck.t_stage);
     applied_load(I, tload, k.ld);
     k.dt = ck.dt;
-    k.cnu = I.nu / (1.0 + I.nu);
-    k.cnu_f = (float)k.cnu;
     k.meh = ME * I.h * I.h;
     k.active = ck.active != 0;
     return k;
@@ -772,48 +768,25 @@ template <typename T> struct CellCtx {
     bool has_load, lam_on, glide;
 };
 
-// Stage-1 observables of a thread's cells: the CFL speed maximum (NaN and Inf map to +Inf) and
-// the FP64 sums of the elastic energy density and of b_zz. FP64 keeps all three in registers.
-// FP32 (its 256-thread tiles run at most 128 registers per thread) keeps the maximum as a float (a
-// maximum of floats is exact) and the two FP64 sums in this thread's two shared-memory slots
-// (`acc`, `acc + ST_THREADS`), so that nothing of them stays in registers across the march.
-template <typename T> struct Stage1Acc {
-    double vmax = 0.0, esum = 0.0, zsum = 0.0;
-    __device__ __forceinline__ void start(double*, int) {}
-    __device__ __forceinline__ void speed(T s) {
-        double v = (double)s;
-        if (!(v <= 1.0e300)) v = __longlong_as_double(0x7ff0000000000000LL);   // NaN/Inf -> +Inf
-        vmax = fmax(vmax, v);
-    }
-    __device__ __forceinline__ void energy(double e, double*, int) { esum += e; }
-    __device__ __forceinline__ void bzz(double z, double*, int) { zsum += z; }
-    __device__ __forceinline__ double max_speed() const { return vmax; }
-    __device__ __forceinline__ double energy_sum(const double*) const { return esum; }
-    __device__ __forceinline__ double bzz_sum(const double*, int) const { return zsum; }
-};
-template <> struct Stage1Acc<float> {
-    float vmax = 0.0f;
-    __device__ __forceinline__ void start(double* acc, int nt) { acc[0] = 0.0; acc[nt] = 0.0; }
-    __device__ __forceinline__ void speed(float s) {
-        if (!(s <= 3.402823466e38f)) s = __int_as_float(0x7f800000);   // NaN/Inf -> +Inf
-        vmax = fmaxf(vmax, s);
-    }
-    __device__ __forceinline__ void energy(double e, double* acc, int) { acc[0] += e; }
-    __device__ __forceinline__ void bzz(double z, double* acc, int nt) { acc[nt] += z; }
-    __device__ __forceinline__ double max_speed() const { return (double)vmax; }
-    __device__ __forceinline__ double energy_sum(const double* acc) const { return acc[0]; }
-    __device__ __forceinline__ double bzz_sum(const double* acc, int nt) const { return acc[nt]; }
-};
+// CFL speed maximum of a thread's stage-1 cells; NaN and Inf map to +Inf. (A maximum of floats is exact.)
+__device__ __forceinline__ void speed_max(float& m, float s) {
+    if (!(s <= 3.402823466e38f)) s = __int_as_float(0x7f800000);
+    m = fmaxf(m, s);
+}
+__device__ __forceinline__ void speed_max(double& m, double s) {
+    if (!(s <= 1.0e300)) s = __longlong_as_double(0x7ff0000000000000LL);
+    m = fmax(m, s);
+}
 
 // ssm: this thread's 6 shared-memory stress slots (component c at ssm[c * ST_THREADS]), filled by
 // asynchronous copies issued one cell earlier; sig_next: the stress of the thread's cell in the
-// next plane (its copies are issued as soon as this cell's values are read), or null; acc: this
-// thread's FP64 sum slots (FP32 stage 1); kc: the block's constants, in shared memory; early() is
-// called once the stress slots are free (FP32), ring_read() as in flux_f64 (FP64).
+// next plane (its copies are issued as soon as this cell's values are read), or null; vmax: the thread's
+// speed maximum (stage 1); kc: the block's constants, in shared memory; early() is called once the
+// stress slots are free (FP32), ring_read() as in flux_f64 (FP64).
 template <typename T, int ND, int MODE, int VAR, class FE, class FR>
 __device__ __forceinline__ void stencil_cell(const InstDev& I, const CellCtx<T>& cx, bool valid,
                                              const TileView<T, ND>& tv, const StageConst& kc,
-                                             Stage1Acc<T>& sums, double* acc,
+                                             T& vmax,
                                              const T* __restrict__ sig0, const T* __restrict__ vac,
                                              T* ssm, const T* sig_next, const FE& early, const FR& ring_read) {
     // compile-time variant: bit 0 carries the glide-only projection, bit 1 the vacancy term
@@ -838,24 +811,6 @@ __device__ __forceinline__ void stencil_cell(const InstDev& I, const CellCtx<T>&
             cp_async_commit();
         }
         early();
-        if (MODE == M_STAGE1 && valid) {
-            // observables of the step-start state: elastic energy of the internal stress (k_dt
-            // applies 1 / (4 mu) to the instance sum). FP32 forms the cell's density in FP32 (its
-            // stress is FP32; sq >= tr^2 / 3 > cnu tr^2, so nothing cancels) and adds it to the FP64
-            // sum; FP64 in FP64.
-            if constexpr (sizeof(T) == 4) {
-                const float d = fmaf(s6[0], s6[0], fmaf(s6[3], s6[3], s6[5] * s6[5]));
-                const float o = fmaf(s6[1], s6[1], fmaf(s6[2], s6[2], s6[4] * s6[4]));
-                const float tr = s6[0] + s6[3] + s6[5];
-                sums.energy((double)fmaf(-kc.cnu_f, tr * tr, fmaf(2.0f, o, d)), acc, st_threads<T>());
-            } else {
-                const double s0 = (double)s6[0], s1 = (double)s6[1], s2 = (double)s6[2];
-                const double s3 = (double)s6[3], s4 = (double)s6[4], s5 = (double)s6[5];
-                const double sq = s0 * s0 + s3 * s3 + s5 * s5 + 2.0 * (s1 * s1 + s2 * s2 + s4 * s4);
-                const double tr = s0 + s3 + s5;
-                sums.energy(sq - kc.cnu * tr * tr, acc, st_threads<T>());
-            }
-        }
         S[0][0] = (T)((double)s6[0] + ld[0]);
         S[1][1] = (T)((double)s6[3] + ld[1]);
         S[2][2] = (T)((double)s6[5] + ld[2]);
@@ -894,8 +849,7 @@ __device__ __forceinline__ void stencil_cell(const InstDev& I, const CellCtx<T>&
             T* o = cx.out;
 #pragma unroll
             for (int c = 0; c < 9; ++c) o[c * cells] = rhs[c];
-            sums.speed(spd);
-            sums.bzz((double)tv.center(8), acc, st_threads<T>());   // mean b_zz of the step-start state
+            speed_max(vmax, spd);
         }
     } else if constexpr (UPD) {
         if (valid && kc.active) {
@@ -916,6 +870,53 @@ __device__ __forceinline__ void stencil_cell(const InstDev& I, const CellCtx<T>&
             }
         }
     }
+}
+
+// Per-instance time step: dt = cfl / (max(shape) * max speed), clamped to t_end (FieldMover.py L94-111), by the
+// block of the instance that finishes stage 1 last: every block writes its maximum and counts itself in
+// done[ii]. (A kernel of its own took 8 us of a step.) A non-finite maximum (also of a block whose planes did not
+// arrive) raises ST_NONFINITE and skips the step. The maximum is exact in any order.
+struct DtArgs {
+    const int* pre;      // prefix sums of the stencil blocks
+    double* bmax;        // per-block speed maxima
+    unsigned* done;      // per-instance count of finished blocks (0 between launches)
+    int fixed;           // step of dt_fixed
+    double dt_fixed;
+};
+__device__ __noinline__ void step_dt(const InstDev& I, int ii, double m, const DtArgs& a, InstClock* clk, int* status,
+                                     double* red) {
+    __shared__ int last;
+    const int b0 = a.pre[ii], b1 = a.pre[ii + 1];
+    if (threadIdx.x == 0) {
+        a.bmax[blockIdx.x] = m;
+        __threadfence();
+        last = atomicAdd(a.done + ii, 1u) == (unsigned)(b1 - b0 - 1);
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    m = 0.0;
+#pragma unroll 4
+    for (int b = b0 + threadIdx.x; b < b1; b += blockDim.x) m = fmax(m, __ldcg(a.bmax + b));
+    m = block_reduce_max(m, red);
+    if (threadIdx.x != 0) return;
+    InstClock c = clk[ii];
+    c.vmax = m;
+    c.t_stage = c.t;
+    const bool finite = (m <= 1.0e300);
+    if (!a.fixed && !finite) atomicOr(status, (int)ST_NONFINITE);
+    const bool act = (c.t < c.t_end) && (a.fixed || finite);
+    double dt;
+    if (a.fixed) dt = a.dt_fixed;
+    else dt = act ? I.cfl / (I.nmax * m) : 0.0;
+    if (!a.fixed && I.dt_max > 0.0 && dt > I.dt_max) dt = I.dt_max;   // dtBound (FieldMover.py L359-360)
+    if (act && c.t + dt > c.t_end) dt = c.t_end - c.t;
+    if (!act) dt = 0.0;
+    c.dt = dt;
+    c.active = act ? 1 : 0;
+    if (act) { c.t = c.t + dt; c.steps += 1; }
+    clk[ii] = c;
+    a.done[ii] = 0;
 }
 
 // The plane box of a stencil tile: RX x RY cells from (x0 - OX, y0 - 2) of the instance's field
@@ -991,8 +992,7 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
                                       const StencilMapSet& maps,
                                       const T* __restrict__ bs, const T* bn, T* out,
                                       const T* __restrict__ sig, T* __restrict__ speed_out,
-                                      const InstClock* __restrict__ clk, double t_flux,
-                                      double* __restrict__ bmax, double* __restrict__ bsum,
+                                      InstClock* clk, double t_flux, const DtArgs& dta,
                                       int* __restrict__ status, const T* __restrict__ vac) {
     constexpr int RX = TileGeom<T>::RX, OX = TileGeom<T>::OX, PP = tile_pp<T>();
     constexpr int TYS = TileGeom<T>::TY, RY = tile_ry<T>(), ST_THREADS = st_threads<T>();
@@ -1089,11 +1089,8 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
 #pragma unroll 1
         for (int q = 0; q < 5; ++q) column_async();
     }
-    Stage1Acc<T> sums;
-    // FP32: this thread's FP64 sum slots after the stress slots
+    T vmax = 0;
     T* ssm = sm + NB * 9 * PP + (OWN ? NS * SP : 0) + tid;
-    double* acc = reinterpret_cast<double*>(ssm - tid + 6 * ST_THREADS) + tid;
-    if (MODE == M_STAGE1) sums.start(acc, ST_THREADS);
     // this thread's cell in plane z0 (cell (z0, 0, 0) for threads outside the grid: in-bounds
     // loads, no stores)
     CellCtx<T> cx;
@@ -1187,7 +1184,7 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
             if (more) request();
             return true;
         };
-        stencil_cell<T, ND, MODE, VAR>(I, cx, own, tv, kc, sums, acc, sig, vac, ssm,
+        stencil_cell<T, ND, MODE, VAR>(I, cx, own, tv, kc, vmax, sig, vac, ssm,
                                        more ? cx.sig + plane : nullptr, early, ring_read);
         if (!ok) break;
         cx.sig += plane;
@@ -1204,20 +1201,12 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
         }
     }
     cp_async_wait_own();   // no copy in flight past here
-    if (!ok) {
-        // a copy did not land in time: let every copy this block issued finish (bounded), then leave
+    // a copy did not land in time: let every copy this block issued finish (bounded)
+    if (!ok)
         for (int n = max(0, issued - NB + 1); n <= issued; ++n) landed(n);
-        return;
-    }
     if (MODE == M_STAGE1) {
-        double m = block_reduce_max(sums.max_speed(), red);
-        double es = block_reduce_sum(sums.energy_sum(acc), red);
-        double zs = block_reduce_sum(sums.bzz_sum(acc, ST_THREADS), red);
-        if (tid == 0) {
-            bmax[blockIdx.x] = m;
-            bsum[2 * blockIdx.x] = es;
-            bsum[2 * blockIdx.x + 1] = zs;
-        }
+        const double m = ok ? block_reduce_max((double)vmax, red) : __longlong_as_double(0x7ff0000000000000LL);
+        step_dt(I, ii, m, dta, clk, status, red);
     }
 }
 
@@ -1225,8 +1214,7 @@ template <typename T, int MODE, int VAR>
 __global__ void __launch_bounds__(st_threads<T>(), ST_BLOCKS)
 k_stencil(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ pre,
           const T* __restrict__ bs, const T* bn, T* out, const T* __restrict__ sig,
-          T* __restrict__ speed_out, const InstClock* __restrict__ clk, double t_flux,
-          double* __restrict__ bmax, double* __restrict__ bsum, int* __restrict__ status,
+          T* __restrict__ speed_out, InstClock* clk, double t_flux, const DtArgs dta, int* __restrict__ status,
           const T* __restrict__ vac, const __grid_constant__ StencilMapSet maps) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     T* sm = reinterpret_cast<T*>(smem_raw);
@@ -1236,60 +1224,11 @@ k_stencil(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__
     const InstDev& I = insts[ii];
     const int lb = blockIdx.x - pre[ii];
     if (I.nd == 3)
-        march<T, 3, MODE, VAR>(I, ii, lb, sm, red, bars, maps, bs, bn, out, sig, speed_out, clk, t_flux, bmax, bsum,
-                          status, vac);
+        march<T, 3, MODE, VAR>(I, ii, lb, sm, red, bars, maps, bs, bn, out, sig, speed_out, clk, t_flux, dta, status,
+                          vac);
     else
-        march<T, 2, MODE, VAR>(I, ii, lb, sm, red, bars, maps, bs, bn, out, sig, speed_out, clk, t_flux, bmax, bsum,
-                          status, vac);
-}
-
-// ------------------------------------------------------------------------------------------
-// Per-instance time step: dt = cfl / (max(shape) * max speed), clamped to t_end
-// (FieldMover.py L94-111). Non-finite maxima raise ST_NONFINITE and skip the step.
-// ------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) k_dt(const InstDev* __restrict__ insts,
-                                           const int* __restrict__ pre,
-                                           const double* __restrict__ bmax,
-                                           const double* __restrict__ bsum,
-                                           InstClock* __restrict__ clk, double* __restrict__ obs,
-                                           int* __restrict__ status, int fixed, double dt_fixed) {
-    __shared__ double red[32];
-    const int ii = blockIdx.x;
-    const InstDev& I = insts[ii];
-    const int b0 = pre[ii], b1 = pre[ii + 1];
-    pdl_wait();
-    double m = 0.0, es = 0.0, zs = 0.0;
-    // one pass over the block partials, unrolled so that several loads are in flight; observable
-    // sums: fixed-order strided partial sums, then a fixed tree (deterministic)
-#pragma unroll 8
-    for (int b = b0 + threadIdx.x; b < b1; b += blockDim.x) {
-        m = fmax(m, bmax[b]);
-        es += bsum[2 * b];
-        zs += bsum[2 * b + 1];
-    }
-    m = block_reduce_max(m, red);
-    es = block_reduce_sum(es, red);
-    zs = block_reduce_sum(zs, red);
-    if (threadIdx.x == 0) {
-        obs[2 * ii] = es / (4.0 * I.mu);
-        obs[2 * ii + 1] = zs * I.inv_cells;
-        InstClock c = clk[ii];
-        c.vmax = m;
-        c.t_stage = c.t;
-        bool finite = (m <= 1.0e300);
-        if (!fixed && !finite) atomicOr(status, (int)ST_NONFINITE);
-        bool act = (c.t < c.t_end) && (fixed || finite);
-        double dt;
-        if (fixed) dt = dt_fixed;
-        else dt = act ? I.cfl / (I.nmax * m) : 0.0;
-        if (!fixed && I.dt_max > 0.0 && dt > I.dt_max) dt = I.dt_max;   // dtBound (FieldMover.py L359-360)
-        if (act && c.t + dt > c.t_end) dt = c.t_end - c.t;
-        if (!act) dt = 0.0;
-        c.dt = dt;
-        c.active = act ? 1 : 0;
-        if (act) { c.t = c.t + dt; c.steps += 1; }
-        clk[ii] = c;
-    }
+        march<T, 2, MODE, VAR>(I, ii, lb, sm, red, bars, maps, bs, bn, out, sig, speed_out, clk, t_flux, dta, status,
+                          vac);
 }
 
 // F0 = u + dt * rhs, in place on the rhs buffer, for active instances (one fused multiply-add per
@@ -1424,8 +1363,9 @@ __global__ void __launch_bounds__(256) k_obs_reduce(const InstDev* __restrict__ 
 // ------------------------------------------------------------------------------------------
 template <typename T>
 static void stencil_dispatch(const PlanCore& P, int mode, const void* bs, const void* bn, void* out,
-                             void* speed, double t, const StencilMapSet& maps, cudaStream_t st) {
+                             void* speed, double t, const StencilMapSet& maps, cudaStream_t st, int fixed, double dt_fixed) {
     const LaunchShape& L = P.stencil;
+    const DtArgs dta{L.d_pre, P.d_bmax, P.d_done, fixed, dt_fixed};
     const T* b = (const T*)bs;
     const T* n = (const T*)bn;
     T* o = (T*)out;
@@ -1435,7 +1375,7 @@ static void stencil_dispatch(const PlanCore& P, int mode, const void* bs, const 
     const int var = (P.any_glide ? 1 : 0) | (P.any_vac ? 2 : 0);
 #define CDD_LAUNCH_V(M, V, SP)                                                                           \
     launch_pdl(k_stencil<T, M, V>, L.blocks, st_threads<T>(), L.smem, st, P.d_inst, P.n_inst, L.d_pre, b, n, o, s, SP,     \
-                                                             P.d_clock, t, P.d_bmax, P.d_bsum, P.d_status,    \
+                                                             P.d_clock, t, dta, P.d_status,    \
                                                              (const T*)P.d_vac, maps)
 #define CDD_LAUNCH_ST(M, SP)                                  \
     switch (var) {                                            \
@@ -1480,9 +1420,10 @@ cudaError_t launch_vacancy_post(const PlanCore& P, const void* beta, cudaStream_
 }
 
 cudaError_t launch_stencil(const PlanCore& P, int mode, const void* bs, const void* bn, void* out,
-                           void* speed, double t_flux, const StencilMapSet& maps, cudaStream_t st) {
-    if (P.precision == CDD_F32) stencil_dispatch<float>(P, mode, bs, bn, out, speed, t_flux, maps, st);
-    else stencil_dispatch<double>(P, mode, bs, bn, out, speed, t_flux, maps, st);
+                           void* speed, double t_flux, const StencilMapSet& maps, cudaStream_t st, int fixed,
+                           double dt_fixed) {
+    if (P.precision == CDD_F32) stencil_dispatch<float>(P, mode, bs, bn, out, speed, t_flux, maps, st, fixed, dt_fixed);
+    else stencil_dispatch<double>(P, mode, bs, bn, out, speed, t_flux, maps, st, fixed, dt_fixed);
     return cudaGetLastError();
 }
 
@@ -1562,12 +1503,6 @@ cudaError_t launch_set_clock(const PlanCore& P, double t, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_dt(const PlanCore& P, int fixed, double dt_fixed, cudaStream_t st) {
-    launch_pdl(k_dt, P.n_inst, 1024, 0, st, P.d_inst, P.stencil.d_pre, P.d_bmax, P.d_bsum, P.d_clock, P.d_obs,
-                                   P.d_status, fixed, dt_fixed);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_axpy_f0(const PlanCore& P, const void* u, void* rhs_f0, cudaStream_t st) {
     const LaunchShape& L = P.cellwise;
     if (P.precision == CDD_F32)
@@ -1611,11 +1546,10 @@ cudaError_t stencil_set_attributes(int precision, size_t smem) {
     return precision == CDD_F32 ? st_attr<float>(smem) : st_attr<double>(smem);
 }
 
-// The plane boxes and columns plus the 6 stress slots of every thread (FP32: and its two FP64 sum slots).
+// The plane boxes and columns plus the 6 stress slots of every thread.
 size_t stencil_smem_bytes(int precision, bool any3d) {
     if (precision == CDD_F32)
-        return ((size_t)(any3d ? TileGeom<float>::NS : 1) * 9 * tile_pp<float>() + 6 * st_threads<float>()) * sizeof(float) +
-               2 * st_threads<float>() * sizeof(double);
+        return ((size_t)(any3d ? TileGeom<float>::NS : 1) * 9 * tile_pp<float>() + 6 * st_threads<float>()) * sizeof(float);
     return ((size_t)9 * tile_pp<double>() + ((any3d ? TileGeom<double>::NS * 9 : 0) + 6) * st_threads<double>()) * sizeof(double);
 }
 

@@ -19,9 +19,8 @@
 //   -> inverse FFT along axis 1 -> C2R rows (axis 2).
 // 2-D: R2C rows (axis 1) -> fused Green pass along axis 0 -> C2R rows.
 //
-// FP32 plans keep the k = 0 mode in FP64: the R2C pass records FP64 row sums of beta, a small
-// kernel turns their means into the mean stress -lam tr<b> d - mu (<b> + <b>^T), and the C2R pass
-// adds it after the FP32 transforms (which carry a zero k = 0 mode).
+// FP32 plans keep the k = 0 mode in FP64: the R2C pass records FP64 row sums of beta, the k-space pass's first
+// blocks form their means, and the C2R pass adds the mean stress -lam tr<b> d - mu (<b> + <b>^T) after the FP32 transforms (which carry a zero k = 0 mode).
 #include "rows_pass.cuh"
 
 #include <cooperative_groups.h>
@@ -343,57 +342,6 @@ k_plane_inv(const InstDev* __restrict__ insts, int n_inst, const int* __restrict
 }
 
 // ------------------------------------------------------------------------------------------
-// FP32 plans: FP64 mean of each beta component from the row sums. One cluster of MEAN_SPLIT blocks
-// per (instance, component): each block sums a contiguous share of the rows (fixed-order strided
-// sums and a fixed tree), block 0 of the cluster adds the shares from the blocks' shared memory
-// (distributed shared memory) in rank order, so the result is deterministic.
-// ------------------------------------------------------------------------------------------
-constexpr int MEAN_SPLIT = 8;
-__global__ void __cluster_dims__(1, 1, MEAN_SPLIT) __launch_bounds__(1024)
-k_mean_beta(const InstDev* __restrict__ insts, const double* __restrict__ rowsum, double* __restrict__ mean9) {
-    const InstDev& I = insts[blockIdx.x];
-    const int c = blockIdx.y;
-    cg::cluster_group cl = cg::this_cluster();
-    pdl_wait();
-    const int part = (int)cl.block_rank();
-    __shared__ double red[32];
-    __shared__ double share;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int chunk = (I.rows + MEAN_SPLIT - 1) / MEAN_SPLIT;
-    const int r0 = part * chunk, r1 = min(I.rows, r0 + chunk);
-    const double* rs = rowsum + I.rsoff + (long long)c * I.rows;
-    // four independent accumulators per thread keep several loads in flight; fixed order throughout
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    const int nt = blockDim.x;
-    int r = r0 + tid;
-    for (; r + 3 * nt < r1; r += 4 * nt) {
-        a0 += rs[r];
-        a1 += rs[r + nt];
-        a2 += rs[r + 2 * nt];
-        a3 += rs[r + 3 * nt];
-    }
-    for (; r < r1; r += nt) a0 += rs[r];
-    double acc = (a0 + a1) + (a2 + a3);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) red[warp] = acc;
-    __syncthreads();
-    if (tid == 0) {
-        double s = 0.0;
-        for (int w = 0; w < (nt >> 5); ++w) s += red[w];
-        share = s;
-    }
-    cl.sync();   // every block's share is written
-    if (part == 0 && tid == 0) {
-        double s = 0.0;
-        for (int k = 0; k < MEAN_SPLIT; ++k) s += *cl.map_shared_rank(&share, k);
-        mean9[9 * blockIdx.x + c] = s * I.inv_cells;
-    }
-    cl.sync();   // the shares stay in shared memory until block 0 has read them
-}
-
-
-// ------------------------------------------------------------------------------------------
 // Host launch sequence
 // ------------------------------------------------------------------------------------------
 // u != null: beta holds the stage-1 rhs and the stress is that of F0 = u + dt rhs, formed in place
@@ -420,7 +368,6 @@ static cudaError_t run_stress(const PlanCore& P, const void* beta, void* sigma, 
         launch_pdl(k_plane_fwd<float, false>, P.plane.blocks, P.plane.threads, P.plane.smem, st, 
             P.d_inst, P.n_inst, P.plane.d_pre, (const float*)beta, spec, tw, P.d_rowsum, nullptr, nullptr, nullptr);
     if (LR[PASS_R2C].blocks > 0) launch_r2c(P, LR[PASS_R2C], beta, f32 ? P.d_rowsum : nullptr, RS_SYM, 6, st);
-    if (f32) launch_pdl(k_mean_beta, dim3(P.n_inst, 6, MEAN_SPLIT), 1024, 0, st, P.d_inst, P.d_rowsum, P.d_sbar);
     launch_mid(P, LR[PASS_MID_F], false, 6, 0, st);
     launch_green(P, P.pass[PASS_GREEN], 0, f32, P.d_k, phi, nullptr, st);
     launch_mid(P, LR[PASS_MID_I], true, 6, 0, st);
