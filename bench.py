@@ -597,11 +597,11 @@ def main():
     issue_ach = FLUX_WARP_INST_PER_CELL * cells / t_stencil / 1e9
     stage_s = el32 / K / 3
     achieved = WORDS_PER_CELL_STAGE * 4 * cells / stage_s / 1e9
-    # per stage: the stress solve (fused plane passes: forward, mean, k-space, inverse; else six
-    # passes incl. the mean) and the stencil; per step: k_dt and, unless the plane passes form F0,
-    # the F0 axpy
+    # per stage: the stress solve (fused plane passes: forward, k-space, inverse; else five passes;
+    # the k-space pass forms the means) and the stencil (stage 1's last block sets dt); per step the
+    # F0 axpy, unless the plane passes form F0
     plane = p32_tuning.get("plane_fft") == 1
-    launches_per_step = 3 * ((4 if plane else 6) + 1) + (1 if plane else 2)
+    launches_per_step = 3 * ((3 if plane else 5) + 1) + (0 if plane else 1)
     line = {
         "metric": METRIC, "value": rate32, "unit": UNIT, "n_gpus": world, "steps": K, "warmup": W,
         "ms_per_step": ms32, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,

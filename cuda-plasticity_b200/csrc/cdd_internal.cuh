@@ -49,25 +49,37 @@ struct LinePlan {
     FDiv ns[MAX_STAGES];   // stage st: span of the finished sub-transforms (product of earlier radices)
     int twst[MAX_STAGES];  // stage st: offset (even, complex elements) of its twiddle rows
     int twspan;            // elements from twst[0] to the end of the last stage's rows
+    int twvalues;          // the same without the rows' padding
     // two-pass form (see pass_stages): n = A B, pass A the first sa stages, pass B the others; pa, pb index
     // CDD_PASS_A / CDD_PASS_B (0: no such form)
     int pa, pb, sa, A, B;
 };
 
-// Radix rounded up to even: the length of one twiddle row (pairs load as one 16-byte vector).
+// Radix rounded up to even: the values of one twiddle row (pairs load as one 16-byte vector).
 __host__ __device__ constexpr int tw_row(int R) { return R + (R & 1); }
+// Row pitch: for radix 8 and 16 an odd number of 16-byte vectors, so that the lanes of a warp, each reading a row of
+// its own, spread over the shared-memory banks. At the plain length these loads were 8-way conflicts: 76% of the
+// shared-load wavefronts of the FP64 C2R pass on 256-point rows. Shorter rows conflict less (radix 4: two- to
+// four-way) and stay dense. 256^3 stress solve 2278 -> 1927 us (FP64), 1156 -> 1032 us (FP32); 128^3 FP64 311 -> 286 us.
+__host__ __device__ constexpr int tw_pitch(int R, size_t velt) {
+    return R < 8 ? tw_row(R) : (velt == 16 ? (R | 1) : 2 * ((tw_row(R) / 2) | 1));
+}
+
+// (Row offsets are written j R + j (pitch - R): with one product ptxas' schedule of the spilling FP64 BIG axis-1
+// kernel takes 160 us a pass of 100x200x250, this way 141 us.)
 
 // Twiddle rows of every stage of lp in butterfly order: row jm of stage st holds
-// w_n^(r jm n / (ns R)), r < R (then (1, 0) padding), ns = lp.ns[st].d, from the length-n table
-// already at re/im[lp.tw ...]. Appends to re/im and sets lp.twst. Over all stages the rows take
-// sum_st ns_st tw_row(R_st) <= 2n entries.
-inline void append_stage_twiddles(LinePlan& lp, std::vector<double>& re, std::vector<double>& im) {
+// w_n^(r jm n / (ns R)), r < R (then (1, 0) padding up to the pitch), ns = lp.ns[st].d, from the length-n table
+// already at re/im[lp.tw ...]. Appends to re/im and sets lp.twst.
+inline void append_stage_twiddles(LinePlan& lp, std::vector<double>& re, std::vector<double>& im, size_t velt) {
     const int n = lp.n;
+    lp.twvalues = 0;
     for (int st = 0; st < lp.nst; ++st) {
         if (re.size() & 1) { re.push_back(1.0); im.push_back(0.0); }   // even start: 16-byte rows
         lp.twst[st] = (int)re.size();
-        const int R = lp.radix[st], ns = lp.ns[st].d, Rp = tw_row(R);
+        const int R = lp.radix[st], ns = lp.ns[st].d, Rp = tw_pitch(R, velt);
         const int twstep = n / (ns * R);
+        lp.twvalues += ns * tw_row(R);
         for (int jm = 0; jm < ns; ++jm)
             for (int r = 0; r < Rp; ++r) {
                 if (r < R) {
@@ -529,7 +541,7 @@ __device__ __forceinline__ void fft_stage(const V* __restrict__ src, V* __restri
             for (int r = 0; r < R; ++r) v[r] = src[lay.addr(l, j + r * nr)];
         } else {
             V w[R];
-            load_tw_row<R>(twrows + jm * tw_row(R), w);
+            load_tw_row<R>(twrows + jm * R + jm * (tw_pitch(R, sizeof(V)) - R), w);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 const V a = src[lay.addr(l, j + r * nr)];
@@ -568,7 +580,7 @@ __device__ __forceinline__ void fft_stage_c(const V* __restrict__ src, V* __rest
             for (int r = 0; r < R; ++r) v[r] = src[ld(r)];
         } else {
             V w[R];
-            load_tw_row<R>(twrows + jm * tw_row(R), w);
+            load_tw_row<R>(twrows + jm * R + jm * (tw_pitch(R, sizeof(V)) - R), w);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 const V a = src[ld(r)];
@@ -666,7 +678,7 @@ __device__ __forceinline__ void fft_stage_io(const LS& src, const LD& dst, int l
             for (int r = 0; r < R; ++r) v[r] = a.ld(r);
         } else {
             V w[R];
-            load_tw_row<R>(twrows + jm * tw_row(R), w);
+            load_tw_row<R>(twrows + jm * R + jm * (tw_pitch(R, sizeof(V)) - R), w);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 const V x = a.ld(r);
@@ -800,7 +812,7 @@ template <typename V, bool INV, bool FIRST, int R, int... Rest>
 __device__ __forceinline__ void pass_stages(V* v, const LinePlan& lp, const V* __restrict__ tws, int st, int jm, int ns) {
     constexpr int M = RadixProd<Rest...>::v;
     V w[R];
-    if constexpr (!FIRST) load_tw_row<R>(tws + (lp.twst[st] - lp.twst[0]) + jm * tw_row(R), w);
+        load_tw_row<R>(tws + (lp.twst[st] - lp.twst[0]) + jm * R + jm * (tw_pitch(R, sizeof(V)) - R), w);
 #pragma unroll
     for (int b = 0; b < M; ++b) {
         V x[R];

@@ -8,8 +8,8 @@
 // caller cannot create a cdd_plan (plan creation allocates its scratch), so this entry point
 // keeps its scratch in a fixed array inside the library instead.
 //
-// The scratch is one file-scope device array of CDD_STRESS_NOALLOC_MAX_BYTES. Every GPU that
-// loads the library holds it until the process exits. Host code may not use the array's name as a
+// The scratch is one file-scope device array of CDD_STRESS_NOALLOC_MAX_BYTES (and the twiddle rows' padding). Every GPU
+// that loads the library holds it until the process exits. Host code may not use the array's name as a
 // device address (on the host it only names a stand-in), so the first call on each device, with that
 // device current, looks the address up once with cudaGetSymbolAddress and caches it; that first
 // call should come before any stream capture. The cached address belongs to the device's primary
@@ -37,7 +37,9 @@ int report_error(int code, const char* msg);   // plan.cu
 
 using namespace cdd;
 
-static __device__ __align__(256) unsigned char g_stress_scratch[CDD_STRESS_NOALLOC_MAX_BYTES];
+// Room for the padding of the twiddle rows (tw_pitch; at most 1184 bytes a length).
+static constexpr size_t TW_PAD_MAX = 4096;
+static __device__ __align__(256) unsigned char g_stress_scratch[CDD_STRESS_NOALLOC_MAX_BYTES + TW_PAD_MAX];
 
 namespace {
 
@@ -152,6 +154,7 @@ extern "C" int cdd_stress_noalloc(const cdd_instance* d, int precision, const vo
     I.inv_cells = 1.0 / (double)I.cells;
     std::vector<double> twre, twim, ktab;
     std::map<int, LinePlan> lp_done;
+    size_t tw_pad = 0;   // padding values of the twiddle rows: not counted against the scratch
     LinePlan* lps[3] = {&I.lp_last, &I.lp_mid, &I.lp_first};
     int lens[3] = {I.nl, I.nd == 3 ? I.n1 : I.n0, I.n0};
     for (int k = 0; k < 3; ++k) {
@@ -166,7 +169,8 @@ extern "C" int cdd_stress_noalloc(const cdd_instance* d, int precision, const vo
                 twre.push_back(re);
                 twim.push_back(im);
             }
-            append_stage_twiddles(*lps[k], twre, twim);
+            append_stage_twiddles(*lps[k], twre, twim, velt);
+            tw_pad += lps[k]->twspan - lps[k]->twvalues;
             it = lp_done.emplace(lens[k], *lps[k]).first;
         }
         *lps[k] = it->second;
@@ -248,16 +252,21 @@ extern "C" int cdd_stress_noalloc(const cdd_instance* d, int precision, const vo
     const size_t off_inst = 0;
     const size_t off_pre = align256(off_inst + sizeof(InstDev));
     const size_t off_tw = align256(off_pre + sizeof(int) * 2 * NUM_PASSES);
-    const size_t off_k = align256(off_tw + velt * twre.size());
-    const size_t off_rs = align256(off_k + elt * ktab.size());
-    const size_t off_sbar = align256(off_rs + (f64 ? 0 : sizeof(double) * 9 * (size_t)I.rows));
-    const size_t off_spec = align256(off_sbar + sizeof(double) * 9);
-    const size_t total = off_spec + velt * 9 * (size_t)I.rows * I.nhp;
+    size_t off_k, off_rs, off_sbar, off_spec;
+    auto layout = [&](size_t ntw) {
+        off_k = align256(off_tw + velt * ntw);
+        off_rs = align256(off_k + elt * ktab.size());
+        off_sbar = align256(off_rs + (f64 ? 0 : sizeof(double) * 9 * (size_t)I.rows));
+        off_spec = align256(off_sbar + sizeof(double) * 9);
+        return off_spec + velt * 9 * (size_t)I.rows * I.nhp;
+    };
+    const size_t total = layout(twre.size() - tw_pad);
     if (total > (size_t)CDD_STRESS_NOALLOC_MAX_BYTES)
         return err(CDD_ERR_SHAPE, "cdd_stress_noalloc: grid needs " + std::to_string(total) +
                                       " bytes of scratch, the fixed scratch holds " +
                                       std::to_string((size_t)CDD_STRESS_NOALLOC_MAX_BYTES) +
                                       "; use a cdd_plan for this size");
+    layout(twre.size());
 
     // ---------------- once per device: the scratch array's device address ----------------
     int dev = 0;

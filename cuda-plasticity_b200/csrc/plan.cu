@@ -171,11 +171,15 @@ int build_shapes(cdd_plan* p, size_t elt) {
     pre_cw.push_back(0);
     pre_ob.push_back(0);
     size_t smem_max[NUM_PASSES] = {0, 0, 0, 0, 0};
+    // What a launch shape may need: two line buffers (one for the register-resident plans) and dense twiddle rows,
+    // so that accepting a tuning does not depend on the form that runs. (Padded rows cross the limit at no length and
+    // tuning where dense ones stay below it.)
+    size_t smem_lim[NUM_PASSES] = {0, 0, 0, 0, 0};
     int n_tma = 0;
     int thr_max[NUM_PASSES] = {0, 0, 0, 0, 0};
     std::vector<int> pre9[NUM_PASSES];   // the observables' launch shapes (9 components)
     for (int k = 0; k < NUM_PASSES; ++k) pre9[k].push_back(0);
-    size_t smem_green12 = 0, smem_green9 = 0, smem_green_lim = 0;
+    size_t smem_green12 = 0, smem_green9 = 0;
     bool lean = true;
     int rtier = 0;
     // the fused plane passes of the stress solve (3-D FP32 shapes that allow them) and the separate
@@ -202,6 +206,9 @@ int build_shapes(cdd_plan* p, size_t elt) {
             int P = rows_lines(I.lp_last, npairs, (int)velt);
             if (tu.rows_lines > 0) P = tu.rows_lines;
             if (P > npairs) P = (int)npairs;
+            const size_t lim = (((size_t)(rows_io_plan(I.lp_last, P) ? 1 : 2) * P * (I.nl + (I.nl >> 4) + 1) + 1) & ~(size_t)1) * velt +
+                               (size_t)I.lp_last.twvalues * velt + rows_table_bytes(P);
+            if (lim > smem_lim[k]) smem_lim[k] = lim;
             PassTile& t = I.tile[k];
             rtier = std::max(rtier, rows_tier(I.lp_last, P));
             t.lines = P;
@@ -221,6 +228,9 @@ int build_shapes(cdd_plan* p, size_t elt) {
             int W = (int)(128 / velt);
             while (W > 1 && 2 * (size_t)W * I.n1 * velt > 96 * 1024) W >>= 1;
             if (p->tune[i].mid_cols > 0) W = p->tune[i].mid_cols;
+            const int bufs = (line_plan_io(I.lp_mid) && I.lp_mid.nst == 2) ? 1 : 2;
+            const size_t lim = bufs * (size_t)W * I.n1 * velt + (size_t)I.lp_mid.twvalues * velt;
+            if (lim > smem_lim[k]) smem_lim[k] = lim;
             C.big_mid |= pass_big(I.lp_mid);
             t.lines = W;
             t.lgw = 0;
@@ -252,8 +262,8 @@ int build_shapes(cdd_plan* p, size_t elt) {
             t.blocks = (I.nd == 3 ? I.n1 : 1) * t.tiles_a;
             const size_t sm = green_smem_bytes(I, W, 6, velt);
             if (sm > smem_max[PASS_GREEN]) smem_max[PASS_GREEN] = sm;
-            const size_t lim = ((size_t)9 * (I.n0 * W + W) + 1) / 2 * 2 * velt + (size_t)I.lp_first.twspan * velt;
-            if (lim > smem_green_lim) smem_green_lim = lim;
+            const size_t lim = ((size_t)9 * (I.n0 * W + W) + 1) / 2 * 2 * velt + (size_t)I.lp_first.twvalues * velt;
+            if (lim > smem_lim[PASS_GREEN]) smem_lim[PASS_GREEN] = lim;
             lean &= green_plan_lean(I.lp_first);
             C.big_green |= pass_big(I.lp_first);
         }
@@ -268,7 +278,7 @@ int build_shapes(cdd_plan* p, size_t elt) {
             const int b9[NUM_PASSES] = {b_rows, b_mid, I.tile[PASS_GREEN].blocks, b_mid, b_rows};
             for (int k = 0; k < NUM_PASSES; ++k) pre9[k].push_back(pre9[k].back() + b9[k]);
             const int W = I.tile[PASS_GREEN].lines;
-            const size_t lim = ((size_t)12 * (I.n0 * W + W) + 1) / 2 * 2 * velt + (size_t)I.lp_first.twspan * velt;
+            const size_t lim = ((size_t)12 * (I.n0 * W + W) + 1) / 2 * 2 * velt + (size_t)I.lp_first.twvalues * velt;
             if (lim > smem_green12) smem_green12 = lim;
             const size_t sm = green_smem_bytes(I, W, 9, velt);
             if (sm > smem_green9) smem_green9 = sm;
@@ -311,9 +321,9 @@ int build_shapes(cdd_plan* p, size_t elt) {
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         for (int k = 0; k < NUM_PASSES; ++k)
-            if (const size_t need = (k == PASS_GREEN) ? smem_green_lim : smem_max[k]; optin > 0 && need + 1024 > (size_t)optin)
+            if (optin > 0 && smem_lim[k] + 1024 > (size_t)optin)
                 return fail(CDD_ERR_ARG, "launch shapes need %zu bytes of shared memory in FFT pass %d (limit %d)",
-                            need, k, optin);
+                            smem_lim[k], k, optin);
     }
     size_t smem_all = 0;
     for (int k = 0; k < NUM_PASSES; ++k) {
@@ -538,7 +548,7 @@ int cdd_plan_create_tuned(const cdd_instance* inst, int n_inst, int precision, c
                     twre.push_back((double)re);
                     twim.push_back((double)im);
                 }
-                append_stage_twiddles(*lps[k], twre, twim);
+                append_stage_twiddles(*lps[k], twre, twim, 2 * elt);
                 it = lp_done.emplace(key, *lps[k]).first;
             }
             *lps[k] = it->second;

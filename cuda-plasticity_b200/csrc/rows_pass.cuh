@@ -190,7 +190,7 @@ __device__ __forceinline__ void r2c_rows_io(const InstDev& I, int lb, int P, int
     for (int g = tid; g < P * R0; g += nt) {
         const int l = g / R0, j = g - l * R0;
         V w[R1], v[R1];
-        load_tw_row<R1>(tw1 + j * tw_row(R1), w);
+        load_tw_row<R1>(tw1 + j * tw_pitch(R1, sizeof(V)), w);
         const V* sl = s + l * ld + row_pad(j);
 #pragma unroll
         for (int r = 0; r < R1; ++r) {
@@ -450,7 +450,7 @@ __device__ __forceinline__ void c2r_rows_io(const InstDev& I, int lb, int P, int
     for (int g = tid; g < P * R0; g += nt) {
         const int l = g / R0, j = g - l * R0;
         V w[R1], v[R1];
-        load_tw_row<R1>(tw1 + j * tw_row(R1), w);
+        load_tw_row<R1>(tw1 + j * tw_pitch(R1, sizeof(V)), w);
         const V* sl = s + l * ld + row_pad(j);
 #pragma unroll
         for (int r = 0; r < R1; ++r) {

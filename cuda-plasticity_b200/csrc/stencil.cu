@@ -1348,6 +1348,7 @@ __global__ void __launch_bounds__(256) k_obs_reduce(const InstDev* __restrict__ 
     const int ii = blockIdx.x;
     pdl_wait();
     double es = 0.0, zs = 0.0;
+#pragma unroll 8
     for (int b = pre[ii] + threadIdx.x; b < pre[ii + 1]; b += blockDim.x) {
         es += bsum[2 * b];
         zs += bsum[2 * b + 1];
