@@ -613,7 +613,7 @@ def main():
                    "l2": "inputs larger than L2 (FP32 field %.0f MB)" % (9 * cells * 4 / 1e6),
                    "timing": "CUDA graph of whole steps, CUDA events, max over ranks",
                    "launch_shapes": p32_tuning},
-        # dominant kernel: k_stencil (≈47% of a step in the launch list), timed alone here in its
+        # dominant kernel: k_stencil (≈46% of a step in the launch list), timed alone here in its
         # flux form; algorithmic bytes per launch = 24 words per cell (read beta 9 + stress 6,
         # write rhs 9); traffic = DRAM bytes per cell from one ncu capture at 192^3, scaled by cells
         "roofline": {"bound": "hbm", "kernel": "k_stencil (flux evaluation, cdd_flux_with_stress)",

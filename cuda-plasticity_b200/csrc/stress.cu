@@ -20,7 +20,8 @@
 // 2-D: R2C rows (axis 1) -> fused Green pass along axis 0 -> C2R rows.
 //
 // FP32 plans keep the k = 0 mode in FP64: the R2C pass records FP64 row sums of beta, the k-space pass's first
-// blocks form their means, and the C2R pass adds the mean stress -lam tr<b> d - mu (<b> + <b>^T) after the FP32 transforms (which carry a zero k = 0 mode).
+// blocks form their means, and the C2R pass adds the mean stress -lam tr<b> d - mu (<b> + <b>^T) after the FP32
+// transforms (which carry a zero k = 0 mode).
 #include "rows_pass.cuh"
 
 #include <cooperative_groups.h>
