@@ -200,19 +200,26 @@ __host__ __device__ inline int rows_elems(const LinePlan& lp, int P, int velt) {
     if (!rows_io_plan(lp, P) && lp.pa) return P * lp.B * (lp.A + 1 + (velt == 8 ? 2 : 0));
     return (rows_io_plan(lp, P) ? 1 : 2) * P * (lp.n + (lp.n >> 4) + 1);
 }
-// Line pairs per block and threads of the row passes. 4096 (FP32) or 2048 (FP64) values per block; small
-// grids take fewer lines, down to two blocks per SM (24^3 FP32: 11 blocks and 28 us before, see rows_lines
-// in the plan), in the multiples that the register-resident form needs.
-inline int rows_lines(const LinePlan& lp, long long npairs, int velt) {
+// Line pairs per block and threads of the row passes. 4096 (FP32) or 2048 (FP64) values per block; plans whose
+// row passes then have fewer than two blocks per SM over all instances (`blocks` of that size on `sms` SMs) take
+// proportionally fewer lines (24^3 FP32: 11 blocks and 28 us before), in the multiples that the register-resident
+// form needs. The count is the plan's, not the instance's: single pairs per block for each of 64 grids of 96^2 and
+// 100^2 points took 541 us a FP64 stress solve, 2048 values per block 156 us.
+inline int rows_lines_full(const LinePlan& lp, int velt) {
     const int full = (velt == 8 ? 4096 : 2048) / lp.n;
+    return full < 1 ? 1 : full;
+}
+inline int rows_lines(const LinePlan& lp, long long npairs, double blocks, int sms, int velt) {
+    const int full = rows_lines_full(lp, velt);
     int step = 1;
     while (step < 8 && lp.nst == 2 && !rows_io_plan(lp, step)) step *= 2;
     if (!rows_io_plan(lp, step)) step = 1;
-    long long P = lp.pa ? npairs / (2 * 148) / step * step : full;
+    int P = full;
+    if (lp.pa && blocks < 2.0 * sms) P = (int)(full * blocks / (2.0 * sms) + 1e-9) / step * step;
     if (P < step) P = step;
     if (P > full) P = full;
-    if (P < 1) P = 1;
-    return (int)(P > npairs ? npairs : P);
+    if (P > npairs) P = npairs >= step ? (int)npairs / step * step : (int)npairs;
+    return P;
 }
 inline int rows_threads(const LinePlan& lp, int P, int velt) {
     const int big = lp.pa ? (lp.A > lp.B ? lp.A : lp.B) : lp.n / 4;
@@ -1035,6 +1042,12 @@ inline cudaError_t set_dyn_smem_limit(F* fn, size_t smem) {
     const long long v = (smem < (size_t)lim) ? (long long)smem : lim;
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v);
 }
+// SMs of the current device.
+inline int device_sms() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+    return sms > 0 ? sms : 148;
+}
 size_t stencil_smem_bytes(int precision, bool any3d);
 int stencil_default_planes(const InstDev* insts, int n, int precision, int sms);
 void stencil_geometry(InstDev& I, int precision, int planes);
@@ -1061,7 +1074,7 @@ cudaError_t r2c_set_attributes(int precision, size_t smem);
 cudaError_t mid_set_attributes(int precision, size_t smem);
 cudaError_t green_set_attributes(int precision, size_t smem);
 cudaError_t c2r_set_attributes(int precision, size_t smem);
-int green_cols(const InstDev& I, size_t velt);
+int green_cols(const InstDev& I, int sms, size_t velt);
 int green_threads(const InstDev& I, size_t velt);
 size_t green_smem_bytes(const InstDev& I, int W, int slots, size_t velt);
 bool green_plan_lean(const LinePlan& lp);

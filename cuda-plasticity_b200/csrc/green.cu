@@ -578,11 +578,11 @@ void launch_green(const PlanCore& P, const LaunchShape& L, int gmode, bool mean6
 // Columns per tile: 32-byte row segments; 64-byte ones (half the line lookups in L1 per byte; stress solve at
 // 128^3 FP64 379 -> 357 us, 100 x 200 x 250 FP32 721 -> 701 us) where the six slots stay under 50 KB, so that as
 // many blocks fit an SM, and the grid still has four blocks per SM (64^3 FP32 prefers 32 bytes, 64 us against 66).
-int green_cols(const InstDev& I, size_t velt) {
+int green_cols(const InstDev& I, int sms, size_t velt) {
     int W = (int)(32 / velt);
     while (W > 1 && (size_t)9 * (I.n0 * W + W) * velt > 100 * 1024) W >>= 1;
     const int wide = (int)(64 / velt), rows = (I.nd == 3) ? I.n1 : 1;
-    if ((size_t)6 * (I.n0 + 1) * 64 <= 50 * 1024 && rows * ((I.nh + wide - 1) / wide) >= 4 * 148) W = wide;
+    if ((size_t)6 * (I.n0 + 1) * 64 <= 50 * 1024 && rows * ((I.nh + wide - 1) / wide) >= 4 * sms) W = wide;
     return W;
 }
 // Threads: FP32 tiles of long lines (three blocks per SM) run on 256 (256^3 stress solve 1196 us against 1259 on

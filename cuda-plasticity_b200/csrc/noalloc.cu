@@ -197,12 +197,13 @@ extern "C" int cdd_stress_noalloc(const cdd_instance* d, int precision, const vo
     P.any3d = (I.nd == 3);
     P.big_mid = (I.nd == 3) && pass_big(I.lp_mid);
     P.big_green = pass_big(I.lp_first);
+    const int sms = device_sms();
     size_t smem_need = 48 * 1024;
     int blocks[NUM_PASSES] = {0, 0, 0, 0, 0};
     for (int k : {PASS_R2C, PASS_C2R}) {
         const int comps = 6;
         long long npairs = ((long long)comps * I.rows + 1) / 2;
-        const int Pl = rows_lines(I.lp_last, npairs, (int)velt);
+        const int Pl = rows_lines(I.lp_last, npairs, (double)npairs / rows_lines_full(I.lp_last, (int)velt), sms, (int)velt);
         P.rows_tier = rows_tier(I.lp_last, Pl);
         PassTile& t = I.tile[k];
         t.lines = Pl;
@@ -230,7 +231,7 @@ extern "C" int cdd_stress_noalloc(const cdd_instance* d, int precision, const vo
     }
     {
         PassTile& t = I.tile[PASS_GREEN];
-        const int W = green_cols(I, velt);
+        const int W = green_cols(I, sms, velt);
         if ((size_t)9 * (I.n0 * W + W) * velt > 220 * 1024)
             return err(CDD_ERR_SHAPE, "cdd_stress_noalloc: axis-0 length too large for the k-space pass");
         t.lines = W;

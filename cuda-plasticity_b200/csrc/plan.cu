@@ -187,14 +187,16 @@ int build_shapes(cdd_plan* p, size_t elt) {
     std::vector<int> pre_plane(1, 0), pre_rest[NUM_PASSES];
     for (int k = 0; k < NUM_PASSES; ++k) pre_rest[k].push_back(0);
     size_t smem_plane = 0;
-    int optin_dev = 0, sms = 0;
+    int optin_dev = 0;
+    const int sms = device_sms();
     {
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&optin_dev, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     }
-    const int st_planes = stencil_default_planes(p->inst.data(), n, C.precision, sms > 0 ? sms : 148);
+    const int st_planes = stencil_default_planes(p->inst.data(), n, C.precision, sms);
+    double row_blocks = 0.0;   // of the row passes at their full size
+    for (const InstDev& I : p->inst) row_blocks += (double)((6LL * I.rows + 1) / 2) / rows_lines_full(I.lp_last, (int)velt);
     for (int i = 0; i < n; ++i) {
         InstDev& I = p->inst[i];
         // rows kernels (R2C: 9 components, C2R: 6); ping-pong buffers of P padded rows
@@ -203,7 +205,7 @@ int build_shapes(cdd_plan* p, size_t elt) {
             const int comps = 6;
             long long npairs = ((long long)comps * I.rows + 1) / 2;
             const cdd_tuning& tu = p->tune[i];
-            int P = rows_lines(I.lp_last, npairs, (int)velt);
+            int P = rows_lines(I.lp_last, npairs, row_blocks, sms, (int)velt);
             if (tu.rows_lines > 0) P = tu.rows_lines;
             if (P > npairs) P = (int)npairs;
             const size_t lim = (((size_t)(rows_io_plan(I.lp_last, P) ? 1 : 2) * P * (I.nl + (I.nl >> 4) + 1) + 1) & ~(size_t)1) * velt +
@@ -246,7 +248,7 @@ int build_shapes(cdd_plan* p, size_t elt) {
         // on W and on the axis-0 length are those of 9 slots (6 components and 3 of scratch).
         {
             PassTile& t = I.tile[PASS_GREEN];
-            int W = green_cols(I, velt);
+            int W = green_cols(I, sms, velt);
             if (p->tune[i].green_cols > 0) W = p->tune[i].green_cols;
             if ((size_t)9 * (I.n0 * W + W) * velt > 220 * 1024) {
                 if (p->tune[i].green_cols > 0)

@@ -1,0 +1,29 @@
+"""Launch shapes of plans with several instances: the lines per block of the row passes come from the plan's
+whole work, and an instance's results do not depend on what it shares its plan with."""
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import cdd
+
+
+@pytest.mark.parametrize("prec,full", [("f64", 2048), ("f32", 4096)])
+def test_row_lines_of_a_batch_fill_their_blocks(prec, full):
+    """64 grids whose row passes have far more than two blocks per SM run full blocks, where one such grid
+    alone takes single lines (results: the oracle tests)."""
+    shapes = [(96, 96), (100, 100)]
+    plan = cdd.Plan([cdd.Instance(s) for s in shapes * 32], prec)
+    assert [plan.tuning(i)["rows_lines"] for i in range(2)] == [full // 96, full // 100]
+    assert cdd.Plan([cdd.Instance(shapes[0])], prec).tuning(0)["rows_lines"] == 1
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("shape", [(4, 32), (6, 32), (4, 6, 64), (10, 128), (18, 50), (24, 24, 24)])
+def test_stress_of_an_instance_does_not_depend_on_its_batch(shape, prec):
+    b = [cdd.gaussian_random_field(s, 0.1, 0.05, 5 + i) for i, s in enumerate([shape, (96, 96), (100, 100)])]
+    one = cdd.Plan([cdd.Instance(shape)], prec)
+    want = one.stress(one.pack(b[:1]))
+    many = cdd.Plan([cdd.Instance(x.shape[1:]) for x in [b[0]] + b[1:] * 32], prec)
+    got = many.stress(many.pack([b[0]] + b[1:] * 32))
+    assert torch.equal(many.stress_view(got, 0), one.stress_view(want, 0))
