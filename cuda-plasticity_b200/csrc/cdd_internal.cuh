@@ -200,6 +200,17 @@ __host__ __device__ inline int rows_elems(const LinePlan& lp, int P, int velt) {
     if (!rows_io_plan(lp, P) && lp.pa) return P * lp.B * (lp.A + 1 + (velt == 8 ? 2 : 0));
     return (rows_io_plan(lp, P) ? 1 : 2) * P * (lp.n + (lp.n >> 4) + 1);
 }
+// Shared memory of a row-pass block: line buffer, twiddle rows, row table.
+inline size_t rows_smem_bytes(const LinePlan& lp, int P, int velt) {
+    return (((size_t)rows_elems(lp, P, velt) + 1) & ~(size_t)1) * velt + (size_t)lp.twspan * velt + rows_table_bytes(P);
+}
+// A short FP32 line's two-pass form is larger than its two line buffers (B (A + 3) values a line: 25 against 22 at 10
+// points, 15 against 14 at 6): line counts that only the buffers fit in `limit` bytes run the stage engine. The passes
+// run on the instance's own copy of the plan, so the other axes keep their form.
+inline void rows_fit(LinePlan& lp, int P, int velt, size_t limit) {
+    if (rows_io_plan(lp, P) || !lp.pa || rows_smem_bytes(lp, P, velt) <= limit) return;
+    lp.pa = lp.pb = lp.sa = lp.A = lp.B = 0;
+}
 // Line pairs per block and threads of the row passes. 4096 (FP32) or 2048 (FP64) values per block; plans whose
 // row passes then have fewer than two blocks per SM over all instances (`blocks` of that size on `sms` SMs) take
 // proportionally fewer lines (24^3 FP32: 11 blocks and 28 us before), in the multiples that the register-resident

@@ -211,8 +211,7 @@ extern "C" int cdd_stress_noalloc(const cdd_instance* d, int precision, const vo
         t.blocks = (int)((npairs + Pl - 1) / Pl);
         t.tiles_a = 1;
         P.pass[k].threads = t.threads;
-        P.pass[k].smem = (((size_t)rows_elems(I.lp_last, Pl, (int)velt) + 1) & ~(size_t)1) * velt +
-                         (size_t)I.lp_last.twspan * velt + rows_table_bytes(Pl);
+        P.pass[k].smem = rows_smem_bytes(I.lp_last, Pl, (int)velt);
     }
     for (int k : {PASS_MID_F, PASS_MID_I}) {
         PassTile& t = I.tile[k];

@@ -172,8 +172,8 @@ int build_shapes(cdd_plan* p, size_t elt) {
     pre_ob.push_back(0);
     size_t smem_max[NUM_PASSES] = {0, 0, 0, 0, 0};
     // What a launch shape may need: two line buffers (one for the register-resident plans) and dense twiddle rows,
-    // so that accepting a tuning does not depend on the form that runs. (Padded rows cross the limit at no length and
-    // tuning where dense ones stay below it.)
+    // so that accepting a tuning does not depend on the form that runs (rows_fit; padded twiddle rows cross the limit
+    // at no length and tuning where dense ones stay below it). What is launched is held to the device's limit below.
     size_t smem_lim[NUM_PASSES] = {0, 0, 0, 0, 0};
     int n_tma = 0;
     int thr_max[NUM_PASSES] = {0, 0, 0, 0, 0};
@@ -211,14 +211,14 @@ int build_shapes(cdd_plan* p, size_t elt) {
             const size_t lim = (((size_t)(rows_io_plan(I.lp_last, P) ? 1 : 2) * P * (I.nl + (I.nl >> 4) + 1) + 1) & ~(size_t)1) * velt +
                                (size_t)I.lp_last.twvalues * velt + rows_table_bytes(P);
             if (lim > smem_lim[k]) smem_lim[k] = lim;
+            rows_fit(I.lp_last, P, (int)velt, optin_dev > 0 ? (size_t)optin_dev - 1024 : SIZE_MAX);
             PassTile& t = I.tile[k];
             rtier = std::max(rtier, rows_tier(I.lp_last, P));
             t.lines = P;
             t.threads = rows_threads(I.lp_last, P, (int)velt);
             t.blocks = (int)((npairs + P - 1) / P);
             t.tiles_a = 1;
-            size_t sm = (((size_t)rows_elems(I.lp_last, P, (int)velt) + 1) & ~(size_t)1) * velt +
-                        (size_t)I.lp_last.twspan * velt + rows_table_bytes(P);   // buffers + twiddle rows + row table
+            const size_t sm = rows_smem_bytes(I.lp_last, P, (int)velt);
             if (sm > smem_max[k]) smem_max[k] = sm;
             if (t.threads > thr_max[k]) thr_max[k] = t.threads;
         }
@@ -323,9 +323,9 @@ int build_shapes(cdd_plan* p, size_t elt) {
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         for (int k = 0; k < NUM_PASSES; ++k)
-            if (optin > 0 && smem_lim[k] + 1024 > (size_t)optin)
+            if (optin > 0 && std::max(smem_lim[k] + 1024, smem_max[k]) > (size_t)optin)
                 return fail(CDD_ERR_ARG, "launch shapes need %zu bytes of shared memory in FFT pass %d (limit %d)",
-                            smem_lim[k], k, optin);
+                            std::max(smem_lim[k], smem_max[k]), k, optin);
     }
     size_t smem_all = 0;
     for (int k = 0; k < NUM_PASSES; ++k) {

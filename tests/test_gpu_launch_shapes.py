@@ -1,11 +1,13 @@
 """Launch shapes of plans with several instances: the lines per block of the row passes come from the plan's
 whole work, and an instance's results do not depend on what it shares its plan with."""
+import numpy as np
 import pytest
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 import cdd
+import cdd_oracle as O
 
 
 @pytest.mark.parametrize("prec,full", [("f64", 2048), ("f32", 4096)])
@@ -27,3 +29,21 @@ def test_stress_of_an_instance_does_not_depend_on_its_batch(shape, prec):
     many = cdd.Plan([cdd.Instance(x.shape[1:]) for x in [b[0]] + b[1:] * 32], prec)
     got = many.stress(many.pack([b[0]] + b[1:] * 32))
     assert torch.equal(many.stress_view(got, 0), one.stress_view(want, 0))
+
+
+@pytest.mark.parametrize("lines", [829, 830, 850, 903])
+def test_largest_row_lines_of_a_ten_point_axis_run(lines):
+    """FP32 line counts that fit two line buffers but not the (larger) two-pass form of 10 points (FP32 2e-6
+    rel-L2 as for the other lengths)."""
+    b = np.random.default_rng(3).standard_normal((9, 320, 10)) * 0.05
+    plan = cdd.Plan([cdd.Instance((320, 10))], "f32", tuning=[{"rows_lines": lines}])
+    assert plan.tuning(0)["rows_lines"] == lines
+    got = plan.stress_view(plan.stress(plan.pack([b])), 0).cpu().numpy()
+    want = O.stress(b.astype(np.float32).astype(np.float64), 1.0, 0.3)[[0, 1, 2, 4, 5, 8]]
+    assert np.linalg.norm(got - want) < 2e-6 * np.linalg.norm(want)
+
+
+def test_row_lines_past_the_shared_memory_are_refused():
+    with pytest.raises(cdd.CDDError) as e:
+        cdd.Plan([cdd.Instance((320, 10))], "f32", tuning=[{"rows_lines": 920}])
+    assert e.value.code == 1
