@@ -511,10 +511,10 @@ __device__ __forceinline__ void vjp_cell(const InstDev& I, long long cl, bool va
 template <typename T>
 __global__ void __launch_bounds__(VJP_THREADS, sizeof(T) == 4 ? 4 : 2) k_vjp_cells(const InstDev* __restrict__ insts, int n_inst,
                                                            const int* __restrict__ pre,
-                                                           const T* __restrict__ beta, const T* __restrict__ sig,
-                                                           const T* __restrict__ gbar, double t,
-                                                           T* __restrict__ ubar, uint32_t* __restrict__ flags,
-                                                           T* __restrict__ sigbar, double* __restrict__ bload) {
+                                                           const T* beta, const T* sig,
+                                                           const T* gbar, double t,
+                                                           T* ubar, uint32_t* flags,
+                                                           T* sigbar, double* bload) {
     __shared__ double red[VJP_THREADS / 32];
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* us = reinterpret_cast<T*>(smem_raw) + threadIdx.x;
@@ -615,9 +615,9 @@ __device__ __forceinline__ void gather_cell(const InstDev& I, long long y, const
 
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_vjp_gather(const InstDev* __restrict__ insts, int n_inst,
-                                                    const int* __restrict__ pre, const T* __restrict__ ubar,
-                                                    const uint32_t* __restrict__ flags,
-                                                    const T* __restrict__ addend, const Axpy<T> ax,
+                                                    const int* __restrict__ pre, const T* ubar,
+                                                    const uint32_t* flags,
+                                                    const T* addend, const Axpy<T> ax,
                                                     T* out) {   // out may alias an x term (same element)
     const int ii = find_instance(pre, n_inst, blockIdx.x);
     const InstDev& I = insts[ii];
@@ -629,8 +629,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_vjp_gather(cons
 }
 
 // Per-instance sums of the block partials of the load cotangent, added to the caller's array.
-__global__ void __launch_bounds__(256) k_vjp_load_reduce(const int* __restrict__ pre, const double* __restrict__ bload,
-                                                         double* __restrict__ out) {
+__global__ void __launch_bounds__(256) k_vjp_load_reduce(const int* __restrict__ pre, const double* bload,
+                                                         double* out) {
     __shared__ double red[8];
     const int ii = blockIdx.x;
     pdl_wait();
@@ -648,9 +648,9 @@ __global__ void __launch_bounds__(256) k_vjp_load_reduce(const int* __restrict__
 // sigbar (load), [6..8] the same times (t - load_t0).
 // One block per instance and sum (blockIdx.y; one block for all six took 14 us at 64^3).
 __global__ void __launch_bounds__(256) k_param_reduce(const InstDev* __restrict__ insts,
-                                                      const int* __restrict__ pre_v, const double* __restrict__ bpart,
-                                                      const int* __restrict__ pre_g, const double* __restrict__ gpart,
-                                                      double c, double t, double* __restrict__ pbar) {
+                                                      const int* __restrict__ pre_v, const double* bpart,
+                                                      const int* __restrict__ pre_g, const double* gpart,
+                                                      double c, double t, double* pbar) {
     __shared__ double red[8];
     const int ii = blockIdx.x, i = blockIdx.y;
     const bool k = i == VJP_PARTS;   // the k-space sum

@@ -7,12 +7,12 @@ template <typename T, bool MEAN64, int TIER>
 __global__ void __launch_bounds__(row_threads_max(sizeof(T)), TIER == 2 ? 3 : 4)
 k_c2r_rows(const InstDev* __restrict__ insts, int n_inst,
                                                   const int* __restrict__ pre,
-                                                  const typename VecOf<T>::type* __restrict__ spec,
-                                                  T* __restrict__ out,
+                                                  const typename VecOf<T>::type* spec,
+                                                  T* out,
                                                   const typename VecOf<T>::type* __restrict__ tw,
-                                                  const double* __restrict__ sbar, int mode, int ncomp,
-                                                  const T* __restrict__ beta, int epi,
-                                                  const InstClock* __restrict__ clk) {
+                                                  const double* sbar, int mode, int ncomp,
+                                                  const T* beta, int epi,
+                                                  const InstClock* clk) {
     typedef typename VecOf<T>::type V;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V* s = reinterpret_cast<V*>(smem_raw);

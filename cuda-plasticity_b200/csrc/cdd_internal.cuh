@@ -896,6 +896,10 @@ inline int rows_tier(const LinePlan& lp, int P) { return rows_io_plan(lp, P) ? 0
 // No kernel lets its successor start before its own blocks end (griddepcontrol.launch_dependents): those blocks
 // would pile up on the SMs that drain first and hold them at the carve-out of the kernel before (measured:
 // 256^3 FP64 step 13.28 -> 13.72 ms, 512^2 FP32 226 -> 256 us).
+// Only what no kernel writes (instance table, prefix sums, twiddles, k tables) is read through __restrict__ pointers or
+// __ldg: for anything else either would allow non-coherent loads, and loads moved ahead of the wait (a __restrict__
+// pointer's target is out of reach of the asm statement's "memory"). So no other pointer parameter of a kernel, or of a
+// function that waits, is __restrict__; functions called after the wait may restrict theirs.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Find the instance that owns global block b, given prefix sums pre[0..n] of blocks.

@@ -64,7 +64,7 @@ template <typename T, bool INV, bool BIG>
 __global__ void __launch_bounds__(mid_threads(sizeof(T)), BIG ? 3 : 4)
 k_fft_mid(const InstDev* __restrict__ insts, int n_inst,
                                                  const int* __restrict__ pre,
-                                                 typename VecOf<T>::type* __restrict__ spec,
+                                                 typename VecOf<T>::type* spec,
                                                  const typename VecOf<T>::type* __restrict__ tw,
                                                  int pass, int ncomp, int vac_only) {
     typedef typename VecOf<T>::type V;

@@ -441,9 +441,9 @@ __device__ __noinline__ void mean_block(const InstDev& I, int ii, int c, const M
 template <typename T, int TIER>
 __global__ void __launch_bounds__(sizeof(T) == 4 ? 256 : 192, (TIER == 2 && sizeof(T) == 8) ? 2 : 3)
 k_green(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ pre, int gmode, int mean64, MeanArgs mean,
-        typename VecOf<T>::type* __restrict__ spec, const typename VecOf<T>::type* __restrict__ tw,
-        const T* __restrict__ ktab, typename VecOf<T>::type* __restrict__ phi, double* __restrict__ part,
-        const InstClock* __restrict__ clk) {
+        typename VecOf<T>::type* spec, const typename VecOf<T>::type* __restrict__ tw,
+        const T* __restrict__ ktab, typename VecOf<T>::type* phi, double* part,
+        const InstClock* clk) {
     typedef typename VecOf<T>::type V;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V* s = reinterpret_cast<V*>(smem_raw);

@@ -11,10 +11,10 @@ template <typename T, bool MEAN64, int TIER>
 __global__ void __launch_bounds__(row_threads_max(sizeof(T)), TIER == 2 ? 3 : 4)
 k_r2c_rows(const InstDev* __restrict__ insts, int n_inst,
                                                   const int* __restrict__ pre,
-                                                  const T* __restrict__ beta,
-                                                  typename VecOf<T>::type* __restrict__ spec,
+                                                  const T* beta,
+                                                  typename VecOf<T>::type* spec,
                                                   const typename VecOf<T>::type* __restrict__ tw,
-                                                  double* __restrict__ rowsum, int mode, int ncomp) {
+                                                  double* rowsum, int mode, int ncomp) {
     typedef typename VecOf<T>::type V;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V* s = reinterpret_cast<V*>(smem_raw);

@@ -11,19 +11,10 @@ __host__ __device__ inline int rows_ld(int n) { return n + (n >> 4) + 1; }
 
 // Four consecutive reals: one 16-byte access for float, two for double (16-byte aligned).
 __device__ __forceinline__ void load4(const float* p, float* v) {
-    float4 q = __ldg(reinterpret_cast<const float4*>(p));
-    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-}
-__device__ __forceinline__ void load4(const double* p, double* v) {
-    double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p) + 1);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-// The same through the coherent path (data the kernel also writes).
-__device__ __forceinline__ void load4c(const float* p, float* v) {
     float4 q = *reinterpret_cast<const float4*>(p);
     v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
 }
-__device__ __forceinline__ void load4c(const double* p, double* v) {
+__device__ __forceinline__ void load4(const double* p, double* v) {
     double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
     v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
 }
@@ -395,8 +386,8 @@ __device__ __forceinline__ void dst_rows(const InstDev& I, T* base, int mode, lo
 template <typename T>
 __device__ __forceinline__ void epilogue4(const T* beta, const RowPtr& e, T coef, int idx, T* v) {
     T a[4], b[4] = {0, 0, 0, 0};
-    load4c(beta + e.p + idx, a);
-    if (e.q >= 0) load4c(beta + e.q + idx, b);
+    load4(beta + e.p + idx, a);
+    if (e.q >= 0) load4(beta + e.q + idx, b);
 #pragma unroll
     for (int q = 0; q < 4; ++q) v[q] -= coef * (a[q] - b[q]);
 }

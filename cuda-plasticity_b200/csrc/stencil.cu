@@ -990,10 +990,10 @@ __device__ __forceinline__ void box_async(T* dst, const BoxGeomT<T>& g, int zp) 
 template <typename T, int ND, int MODE, int VAR>
 __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, double* red, uint64_t* bars,
                                       const StencilMapSet& maps,
-                                      const T* __restrict__ bs, const T* bn, T* out,
-                                      const T* __restrict__ sig, T* __restrict__ speed_out,
+                                      const T* bs, const T* bn, T* out,
+                                      const T* sig, T* speed_out,
                                       InstClock* clk, double t_flux, const DtArgs& dta,
-                                      int* __restrict__ status, const T* __restrict__ vac) {
+                                      int* status, const T* vac) {
     constexpr int RX = TileGeom<T>::RX, OX = TileGeom<T>::OX, PP = tile_pp<T>();
     constexpr int TYS = TileGeom<T>::TY, RY = tile_ry<T>(), ST_THREADS = st_threads<T>();
     constexpr bool OWN = own_columns<T, ND>();
@@ -1213,9 +1213,9 @@ __device__ __forceinline__ void march(const InstDev& I, int ii, int lb, T* sm, d
 template <typename T, int MODE, int VAR>
 __global__ void __launch_bounds__(st_threads<T>(), ST_BLOCKS)
 k_stencil(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ pre,
-          const T* __restrict__ bs, const T* bn, T* out, const T* __restrict__ sig,
-          T* __restrict__ speed_out, InstClock* clk, double t_flux, const DtArgs dta, int* __restrict__ status,
-          const T* __restrict__ vac, const __grid_constant__ StencilMapSet maps) {
+          const T* bs, const T* bn, T* out, const T* sig,
+          T* speed_out, InstClock* clk, double t_flux, const DtArgs dta, int* status,
+          const T* vac, const __grid_constant__ StencilMapSet maps) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     T* sm = reinterpret_cast<T*>(smem_raw);
     __shared__ double red[st_threads<T>() / 32];
@@ -1235,8 +1235,8 @@ k_stencil(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__
 // value). Instances with the fused plane passes form F0 in their forward pass instead.
 template <typename T>
 __global__ void __launch_bounds__(256) k_axpy_f0(const InstDev* __restrict__ insts, int n_inst,
-                                                 const int* __restrict__ pre, const T* __restrict__ u,
-                                                 T* __restrict__ f0, const InstClock* __restrict__ clk) {
+                                                 const int* __restrict__ pre, const T* u,
+                                                 T* f0, const InstClock* clk) {
     const int ii = find_instance(pre, n_inst, blockIdx.x);
     const InstDev& I = insts[ii];
     pdl_wait();
@@ -1283,8 +1283,8 @@ __global__ void __launch_bounds__(256) k_axpy_f0(const InstDev* __restrict__ ins
 // xx + yy, then zz, as the reference does.
 template <typename T>
 __global__ void __launch_bounds__(256) k_vac_trace(const InstDev* __restrict__ insts, int n_inst,
-                                                   const int* __restrict__ pre, const T* __restrict__ beta,
-                                                   T* __restrict__ tr) {
+                                                   const int* __restrict__ pre, const T* beta,
+                                                   T* tr) {
     const int ii = find_instance(pre, n_inst, blockIdx.x);
     const InstDev& I = insts[ii];
     pdl_wait();
@@ -1297,9 +1297,9 @@ __global__ void __launch_bounds__(256) k_vac_trace(const InstDev* __restrict__ i
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_vac_update(const InstDev* __restrict__ insts, int n_inst,
-                                                    const int* __restrict__ pre, const T* __restrict__ beta,
-                                                    const T* __restrict__ tr, T* __restrict__ c,
-                                                    const InstClock* __restrict__ clk) {
+                                                    const int* __restrict__ pre, const T* beta,
+                                                    const T* tr, T* c,
+                                                    const InstClock* clk) {
     const int ii = find_instance(pre, n_inst, blockIdx.x);
     const InstDev& I = insts[ii];
     pdl_wait();
@@ -1316,9 +1316,9 @@ __global__ void __launch_bounds__(256) k_vac_update(const InstDev* __restrict__ 
 template <typename T>
 __global__ void __launch_bounds__(256) k_observe(const InstDev* __restrict__ insts, int n_inst,
                                                         const int* __restrict__ pre,
-                                                        const T* __restrict__ beta,
-                                                        const T* __restrict__ sig,
-                                                        double* __restrict__ bsum) {
+                                                        const T* beta,
+                                                        const T* sig,
+                                                        double* bsum) {
     __shared__ double red[8];
     const int ii = find_instance(pre, n_inst, blockIdx.x);
     const InstDev& I = insts[ii];
@@ -1342,8 +1342,8 @@ __global__ void __launch_bounds__(256) k_observe(const InstDev* __restrict__ ins
 
 __global__ void __launch_bounds__(256) k_obs_reduce(const InstDev* __restrict__ insts,
                                                     const int* __restrict__ pre,
-                                                    const double* __restrict__ bsum,
-                                                    double* __restrict__ obs) {
+                                                    const double* bsum,
+                                                    double* obs) {
     __shared__ double red[8];
     const int ii = blockIdx.x;
     pdl_wait();
@@ -1490,7 +1490,7 @@ bool encode_stencil_maps(const PlanCore& P, const InstDev* insts, const void* ba
 }
 
 // Start every instance's clock at t with no end time (fixed-dt steps at a caller-given time).
-__global__ void k_set_clock(InstClock* __restrict__ clk, int n_inst, double t) {
+__global__ void k_set_clock(InstClock* clk, int n_inst, double t) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     pdl_wait();
     if (i < n_inst) {

@@ -204,8 +204,8 @@ template <typename V> struct PlaneRowOut {
 template <typename T, bool F0>
 __global__ void __cluster_dims__(PLANE_C, 1, 1) __launch_bounds__(ROW_THREADS, 3)
 k_plane_fwd(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ pre, const T* beta,
-            typename VecOf<T>::type* __restrict__ spec, const typename VecOf<T>::type* __restrict__ tw,
-            double* __restrict__ rowsum, T* f0w, const T* __restrict__ u, const InstClock* __restrict__ clk) {
+            typename VecOf<T>::type* spec, const typename VecOf<T>::type* __restrict__ tw,
+            double* rowsum, T* f0w, const T* u, const InstClock* clk) {
     typedef typename VecOf<T>::type V;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cg::cluster_group cl = cg::this_cluster();
@@ -281,8 +281,8 @@ k_plane_fwd(const InstDev* __restrict__ insts, int n_inst, const int* __restrict
 template <typename T>
 __global__ void __cluster_dims__(PLANE_C, 1, 1) __launch_bounds__(ROW_THREADS, 3)
 k_plane_inv(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ pre,
-            const typename VecOf<T>::type* __restrict__ spec, T* __restrict__ out,
-            const typename VecOf<T>::type* __restrict__ tw, const double* __restrict__ sbar) {
+            const typename VecOf<T>::type* spec, T* out,
+            const typename VecOf<T>::type* __restrict__ tw, const double* sbar) {
     typedef typename VecOf<T>::type V;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cg::cluster_group cl = cg::this_cluster();
