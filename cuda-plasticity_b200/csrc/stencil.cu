@@ -25,6 +25,7 @@
 #include <cudaTypedefs.h>
 
 #include "cdd_internal.cuh"
+#include "fp64_math.cuh"
 
 namespace cdd {
 
@@ -467,7 +468,8 @@ __device__ __forceinline__ void flux_f32(const TileView<float, ND>& tv, float ih
 // by 8 resident warps per SM to hide its latency. All 54 derivatives stay in registers (246, no spills), formed
 // once: forming them again for the rhs, with the five-compare minmod, 8 square roots and 8 + 4 divisions
 // of the form before it, took 4272 us per 256^3 flux, this 2704 us; with the plane copies under the cell's own
-// work (march) and 20 planes per block, 1796 us; with own columns and Newton's rsqrt and reciprocal, 1649 us.
+// work (march) and 20 planes per block, 1796 us; with own columns and Newton's rsqrt and reciprocal, 1649 us; with their
+// values at 0 and infinity (fp64_math.cuh), 1658 us.
 // d + h minmod(e, m) for h = -1/2 or 1/2: the factor is 0 unless the signs of e and m agree (an integer test),
 // and times the smaller magnitude otherwise, so the FP64 pipe sees one compare and one multiply-add. A NaN in
 // e (two cells away) leaves m, as minmod's 0 leaves d: only the cells whose d or m is NaN become NaN.
@@ -482,23 +484,6 @@ __device__ __forceinline__ void derivs5_f64(const double* v, double& up, double&
     const double e0 = d1 - d0, em1 = d0 - dm1, em2 = dm1 - dm2;
     up = limited_f64(d0, e0, em1, -0.5);
     um = limited_f64(dm1, em2, em1, 0.5);
-}
-
-// 1 / sqrt(x) and 1 / x of normal positive x: the hardware's approximations (about 2^-22) and Newton's iteration,
-// y <- y + y (1 - x y^2) / 2 and y <- y + y (1 - x y), twice: no branches, unlike the library's, whose special
-// cases cannot occur here (x >= ME Dx^2, x >= ME; 0 or NaN results for infinite or NaN x as NaN).
-__device__ __forceinline__ double rsqrt_f64(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double h = 0.5 * y, e = fma(-x * y, y, 1.0);
-    y = fma(h, e, y);
-    return fma(0.5 * y, fma(-x * y, y, 1.0), y);
-}
-__device__ __forceinline__ double rcp_f64(double x) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    y = fma(y, fma(-x, y, 1.0), y);
-    return fma(y, fma(-x, y, 1.0), y);
 }
 
 // meh: ME Dx^2. ring_read(): called once the thread has read all it needs of the ring but its cell's own
