@@ -468,14 +468,17 @@ __device__ __forceinline__ void flux_f32(const TileView<float, ND>& tv, float ih
 // by 8 resident warps per SM to hide its latency. All 54 derivatives stay in registers (246, no spills), formed
 // once: forming them again for the rhs, with the five-compare minmod, 8 square roots and 8 + 4 divisions
 // of the form before it, took 4272 us per 256^3 flux, this 2704 us; with the plane copies under the cell's own
-// work (march) and 20 planes per block, 1796 us; with own columns and Newton's rsqrt and reciprocal, 1649 us; with their
-// values at 0 and infinity (fp64_math.cuh), 1658 us.
-// d + h minmod(e, m) for h = -1/2 or 1/2: the factor is 0 unless the signs of e and m agree (an integer test),
-// and times the smaller magnitude otherwise, so the FP64 pipe sees one compare and one multiply-add. A NaN in
-// e (two cells away) leaves m, as minmod's 0 leaves d: only the cells whose d or m is NaN become NaN.
+// work (march) and 20 planes per block, 1796 us; with own columns and Newton's rsqrt and reciprocal, 1649 us; with the
+// values of NaN, zero and infinite arguments (limited_f64, fp64_math.cuh), 1693 us.
+// d + h minmod(e, m) for h = -1/2 or 1/2: the factor is 0 unless the signs of e and m agree (an integer test), and
+// times the smaller magnitude otherwise, so the FP64 pipe sees one compare and one multiply-add. A NaN in e (two cells
+// away) leaves d, as minmod's 0 does: only the cells whose d or m is NaN become NaN. (A result of arithmetic is a quiet
+// NaN: adding its quiet bit to the upper word carries into the sign bit, and for no other value. This test costs 2% of
+// a 256^3 flux, 1658 -> 1694 us; forming the rare cells with a NaN again at the end of the march cost as much.)
 __device__ __forceinline__ double limited_f64(double d, double e, double m, double h) {
     const double v = fabs(e) < fabs(m) ? e : m;
-    const bool same = (__double2hiint(e) ^ __double2hiint(m)) >= 0;
+    const int he = __double2hiint(e);
+    const bool same = ((he ^ __double2hiint(m)) | (he ^ (int)((unsigned)he + 0x00080000u))) >= 0;
     return fma(__hiloint2double(same ? __double2hiint(h) : 0, 0), v, d);
 }
 // (u+, u-) times Dx from u_{-2} .. u_{+2}.

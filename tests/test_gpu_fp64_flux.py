@@ -1,4 +1,4 @@
-"""The FP64 flux at the edges of its number range: its reciprocals against long double, and
+"""The FP64 flux at the edges of its number range: its reciprocals against long double, NaN neighbours and
 overflowing gradients."""
 import os
 import shutil
@@ -11,6 +11,7 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 import cdd
+import cdd_oracle as O
 
 REPO = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(REPO, "cuda-plasticity_b200", "csrc")
@@ -68,6 +69,33 @@ def test_reciprocals_against_long_double(tmp_path):
     out = subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout.split()
     assert int(out[1]) == 1
     assert float(out[2]) < 1.0 and float(out[3]) < 1.0, out
+
+
+@pytest.mark.parametrize("shape,at", [((16, 40), (7, 20)), ((8, 12, 72), (3, 5, 40)), ((8, 6, 18), (0, 1, 0))])
+def test_nan_reaches_the_nearest_cells_only(shape, at, monkeypatch):
+    """A NaN two cells away leaves the limited derivative at its difference, whatever the NaN's sign bit: every cell
+    that is not the NaN's own or its nearest neighbour along an axis has the finite value of a limiter that takes
+    no part of it (FP64 1e-12 as for the other fluxes)."""
+    minmod3 = O.minmod3
+    monkeypatch.setattr(O, "minmod3", lambda a, b, c: np.where(np.isnan(a) | np.isnan(c), 0.0,
+                                                               minmod3(*(np.nan_to_num(v) for v in (a, b, c)))))
+    b = cdd.gaussian_random_field(shape, 0.08, 0.05, 13)
+    plan = cdd.Plan([cdd.Instance(shape)], "f64")
+    sigma = plan.stress(plan.pack([b]))
+    far = np.ones(shape, bool)
+    for d in range(len(shape)):
+        for k in (-1, 0, 1):
+            far[at[:d] + ((at[d] + k) % shape[d],) + at[d + 1:]] = False
+    total = O.stress(b, 1.0, 0.3)
+    for sign in (1.0, -1.0):
+        bad = b.copy()
+        bad[(4,) + at] = np.copysign(np.nan, sign)
+        rhs, speed = plan.flux(plan.pack([bad]), 0.0, sigma=sigma)
+        ref, ref_speed = O.flux(bad, total)
+        got, got_speed = plan.field_view(rhs, 0).cpu().numpy(), speed.cpu().numpy().reshape(shape)
+        assert np.isnan(got_speed[at]) and np.isfinite(got[:, far]).all()
+        assert np.linalg.norm(got[:, far] - ref[:, far]) < 1e-12 * np.linalg.norm(ref[:, far])
+        assert np.linalg.norm(got_speed[far] - ref_speed[far]) < 1e-12 * np.linalg.norm(ref_speed[far])
 
 
 def test_overflowing_gradients_stand_still():
