@@ -405,8 +405,7 @@ struct MeanArgs {
     const double* rowsum;
     double* mean9;           // 9 per instance
 };
-__device__ __noinline__ void mean_block(const InstDev& I, int ii, int c, const MeanArgs& a) {
-    __shared__ double red[8];
+__device__ __noinline__ void mean_block(const InstDev& I, int ii, int c, const MeanArgs& a, double* red) {
     const int tid = threadIdx.x, nt = blockDim.x;
     pdl_wait();
     const double* rs = a.rowsum + I.rsoff + (long long)c * I.rows;
@@ -436,6 +435,9 @@ __device__ __noinline__ void mean_block(const InstDev& I, int ii, int c, const M
 //   pass A global -> slots, pass B in place (its outputs m + A r are the positions it read), contraction,
 //   inverse pass A in place (j + B q, natural order in; output m stays at j + B m), inverse pass B from
 //   the B consecutive values at m B -> global.
+// No static shared memory: the slots and twiddle rows of some lengths fill an SM's share to within 300 bytes (three
+// blocks of 256 points at radix 8, two of 288 points with 12 slots; a 320-byte array made the latter's passes take 468
+// us instead of 332).
 // Four block barriers, no scratch slots and one butterfly per thread and pass at 256 (12 lines FP64, 24 FP32,
 // on 192 threads). Bound by the latency of its phases and, at FP64, the FP64 pipe.
 template <typename T, int TIER>
@@ -448,7 +450,7 @@ k_green(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ p
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V* s = reinterpret_cast<V*>(smem_raw);
     if ((int)blockIdx.x < mean.blocks) {
-        mean_block(insts[blockIdx.x / 6], blockIdx.x / 6, blockIdx.x % 6, mean);
+        mean_block(insts[blockIdx.x / 6], blockIdx.x / 6, blockIdx.x % 6, mean, reinterpret_cast<double*>(smem_raw));
         return;
     }
     const int blk = blockIdx.x - mean.blocks;
@@ -523,8 +525,8 @@ k_green(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ p
 #undef CDD_CONTRACT
     }
     if (gmode == 1 && part) {
-        // fixed-order block reduction (deterministic)
-        __shared__ double red[32];
+        // fixed-order block reduction (deterministic), in the bytes that this mode's launch adds (launch_green)
+        double* red = reinterpret_cast<double*>(tws + ((lp.twspan + 1) & ~1));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) pacc += __shfl_xor_sync(0xffffffffu, pacc, o);
         if ((tid & 31) == 0) red[tid >> 5] = pacc;
@@ -559,9 +561,10 @@ static void green_t(const PlanCore& P, const LaunchShape& L, int gmode, bool mea
                     cudaStream_t st) {
     typedef typename VecOf<T>::type V;
     const int tier = (P.green_lean && gmode <= 1) ? 0 : (P.big_green ? 2 : 1);
+    const size_t smem = L.smem + (gmode == 1 ? 96 : 0);   // the block sums of the adjoint mode
     const MeanArgs mean{mean64 ? 6 * P.n_inst : 0, P.d_rowsum, P.d_sbar};
 #define CDD_LAUNCH_G(TIER)                                                                                               \
-    launch_pdl(k_green<T, TIER>, L.blocks + mean.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, gmode, mean64, \
+    launch_pdl(k_green<T, TIER>, L.blocks + mean.blocks, L.threads, smem, st, P.d_inst, P.n_inst, L.d_pre, gmode, mean64, \
                mean, (V*)P.d_spec, (const V*)P.d_tw, (const T*)ktab, (V*)phi, part, P.d_clock)
     if (tier == 0) CDD_LAUNCH_G(0);
     else if (tier == 1) CDD_LAUNCH_G(1);
