@@ -609,8 +609,11 @@ __device__ __forceinline__ void gather_cell(const InstDev& I, long long y, const
 #pragma unroll
         for (int k = 0; k < 3; ++k)
             if (ax.x[k]) v += ax.a[k] * ax.x[k][o];
-        out[o] = v;
+        acc[c] = v;
     }
+    // all loads before the first store: out may be an x term (same element), and no load can pass a store
+#pragma unroll
+    for (int c = 0; c < 9; ++c) out[I.foff + (long long)c * cells + y] = acc[c];
 }
 
 template <typename T>
