@@ -211,27 +211,34 @@ inline void rows_fit(LinePlan& lp, int P, int velt, size_t limit) {
     if (rows_io_plan(lp, P) || !lp.pa || rows_smem_bytes(lp, P, velt) <= limit) return;
     lp.pa = lp.pb = lp.sa = lp.A = lp.B = 0;
 }
-// Line pairs per block and threads of the row passes. 4096 (FP32) or 2048 (FP64) values per block; plans whose
-// row passes then have fewer than two blocks per SM over all instances (`blocks` of that size on `sms` SMs) take
-// proportionally fewer lines (24^3 FP32: 11 blocks and 28 us before), in the multiples that the register-resident
-// form needs. The count is the plan's, not the instance's: single pairs per block for each of 64 grids of 96^2 and
-// 100^2 points took 541 us a FP64 stress solve, 2048 values per block 156 us.
-inline int rows_lines_full(const LinePlan& lp, int velt) {
-    const int full = (velt == 8 ? 4096 : 2048) / lp.n;
-    return full < 1 ? 1 : full;
-}
-inline int rows_lines(const LinePlan& lp, long long npairs, double blocks, int sms, int velt) {
-    const int full = rows_lines_full(lp, velt);
+// Line pairs per block and threads of the row passes. 4096 (FP32) or 2048 (FP64) values per block; an instance with fewer
+// than two such blocks per SM takes fewer lines, down to two blocks per SM (24^3 FP32: 11 blocks and 28 us before), in
+// the multiples that the register-resident form needs. The instances of a plan together get four blocks per SM that
+// way, and `scale` times the lines where they would have more: single pairs per block for each of 64 grids of 96^2 and
+// 100^2 points took 541 us a FP64 stress solve, 2048 values per block 156 us; four grids of 32^3 to 100^3 points in
+// FP32 want the smaller blocks of the small ones (278 us against 302).
+inline int rows_step(const LinePlan& lp) {
     int step = 1;
     while (step < 8 && lp.nst == 2 && !rows_io_plan(lp, step)) step *= 2;
-    if (!rows_io_plan(lp, step)) step = 1;
+    return rows_io_plan(lp, step) ? step : 1;
+}
+inline int rows_lines(const LinePlan& lp, long long npairs, double scale, int sms, int velt) {
+    int full = (velt == 8 ? 4096 : 2048) / lp.n;
+    if (full < 1) full = 1;
+    const int step = rows_step(lp);
+    const double want = (double)(npairs / (2 * sms) / step * step);
     int P = full;
-    if (lp.pa && blocks < 2.0 * sms) P = (int)(full * blocks / (2.0 * sms) + 1e-9) / step * step;
-    if (P < step) P = step;
+    if (lp.pa && (want < step ? step : want) * scale < full) P = (int)((want < step ? step : want) * scale) / step * step;
     if (P > full) P = full;
     if (P > npairs) P = npairs >= step ? (int)npairs / step * step : (int)npairs;
     return P;
 }
+// Blocks of an instance with fewer lines than a full block's (0: full blocks).
+inline double rows_small_blocks(const LinePlan& lp, long long npairs, int sms, int velt) {
+    const int P = rows_lines(lp, npairs, 1.0, sms, velt);
+    return lp.pa && P < (velt == 8 ? 4096 : 2048) / lp.n ? (double)npairs / P : 0.0;
+}
+inline double rows_scale(double small_blocks, int sms) { return small_blocks > 4.0 * sms ? small_blocks / (4.0 * sms) : 1.0; }
 inline int rows_threads(const LinePlan& lp, int P, int velt) {
     const int big = lp.pa ? (lp.A > lp.B ? lp.A : lp.B) : lp.n / 4;
     return (velt == 8 && P * big > 192) ? 256 : 128;

@@ -203,7 +203,7 @@ extern "C" int cdd_stress_noalloc(const cdd_instance* d, int precision, const vo
     for (int k : {PASS_R2C, PASS_C2R}) {
         const int comps = 6;
         long long npairs = ((long long)comps * I.rows + 1) / 2;
-        const int Pl = rows_lines(I.lp_last, npairs, (double)npairs / rows_lines_full(I.lp_last, (int)velt), sms, (int)velt);
+        const int Pl = rows_lines(I.lp_last, npairs, 1.0, sms, (int)velt);
         P.rows_tier = rows_tier(I.lp_last, Pl);
         PassTile& t = I.tile[k];
         t.lines = Pl;

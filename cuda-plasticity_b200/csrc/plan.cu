@@ -195,8 +195,9 @@ int build_shapes(cdd_plan* p, size_t elt) {
         cudaDeviceGetAttribute(&optin_dev, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     }
     const int st_planes = stencil_default_planes(p->inst.data(), n, C.precision, sms);
-    double row_blocks = 0.0;   // of the row passes at their full size
-    for (const InstDev& I : p->inst) row_blocks += (double)((6LL * I.rows + 1) / 2) / rows_lines_full(I.lp_last, (int)velt);
+    double small_blocks = 0.0;
+    for (const InstDev& I : p->inst) small_blocks += rows_small_blocks(I.lp_last, (6LL * I.rows + 1) / 2, sms, (int)velt);
+    const double row_scale = rows_scale(small_blocks, sms);
     for (int i = 0; i < n; ++i) {
         InstDev& I = p->inst[i];
         // rows kernels (R2C: 9 components, C2R: 6); ping-pong buffers of P padded rows
@@ -205,7 +206,7 @@ int build_shapes(cdd_plan* p, size_t elt) {
             const int comps = 6;
             long long npairs = ((long long)comps * I.rows + 1) / 2;
             const cdd_tuning& tu = p->tune[i];
-            int P = rows_lines(I.lp_last, npairs, row_blocks, sms, (int)velt);
+            int P = rows_lines(I.lp_last, npairs, row_scale, sms, (int)velt);
             if (tu.rows_lines > 0) P = tu.rows_lines;
             if (P > npairs) P = (int)npairs;
             const size_t lim = (((size_t)(rows_io_plan(I.lp_last, P) ? 1 : 2) * P * (I.nl + (I.nl >> 4) + 1) + 1) & ~(size_t)1) * velt +

@@ -1,5 +1,7 @@
 """Launch shapes of plans with several instances: the lines per block of the row passes come from the plan's
 whole work, and an instance's results do not depend on what it shares its plan with."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -11,12 +13,14 @@ import cdd_oracle as O
 
 
 @pytest.mark.parametrize("prec,full", [("f64", 2048), ("f32", 4096)])
-def test_row_lines_of_a_batch_fill_their_blocks(prec, full):
-    """64 grids whose row passes have far more than two blocks per SM run full blocks, where one such grid
-    alone takes single lines (results: the oracle tests)."""
-    shapes = [(96, 96), (100, 100)]
-    plan = cdd.Plan([cdd.Instance(s) for s in shapes * 32], prec)
-    assert [plan.tuning(i)["rows_lines"] for i in range(2)] == [full // 96, full // 100]
+def test_row_lines_come_from_the_whole_plan(prec, full):
+    """64 grids together take lines for about four blocks per SM, or whole blocks, where one such grid alone takes
+    single lines (results: the oracle tests)."""
+    shapes = [(96, 96), (100, 100)] * 32
+    plan = cdd.Plan([cdd.Instance(s) for s in shapes], prec)
+    lines = [plan.tuning(i)["rows_lines"] for i in range(len(shapes))]
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert all(n == full // s[1] for n, s in zip(lines, shapes)) or sum(3 * s[0] / n for n, s in zip(lines, shapes)) < 4.4 * sms
     assert cdd.Plan([cdd.Instance(shapes[0])], prec).tuning(0)["rows_lines"] == 1
 
 
@@ -47,3 +51,29 @@ def test_row_lines_past_the_shared_memory_are_refused():
     with pytest.raises(cdd.CDDError) as e:
         cdd.Plan([cdd.Instance((320, 10))], "f32", tuning=[{"rows_lines": 920}])
     assert e.value.code == 1
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_a_plan_of_every_fft_form(prec):
+    """One plan whose axes take one-stage passes, passes of up to 16 and of more values, and lengths without a two-pass
+    form: each instance has the stress, its adjoint and the observables of its own plan."""
+    shapes = [(64, 64, 8), (36, 54, 8), (100, 20, 8), (20, 100, 8), (288, 6, 8), (6, 288, 8), (512, 4, 8), (4, 4, 4)]
+    fields = [np.random.default_rng(i).standard_normal((9,) + s) * 0.05 for i, s in enumerate(shapes)]
+    many = cdd.Plan([cdd.Instance(s) for s in shapes], prec)
+
+    def results(plan, b):
+        beta = plan.pack(b)
+        sig = plan.stress(beta)
+        back = plan.empty_field()
+        ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+        assert plan.lib.cdd_stress_adjoint(plan.handle, ptr(sig), ptr(back), ctypes.c_void_p(0)) == 0
+        return sig, back, plan.observe("rho", beta), plan.observe("rotation", beta)
+
+    got = results(many, fields)
+    for i, s in enumerate(shapes):
+        one = cdd.Plan([cdd.Instance(s)], prec)
+        want = results(one, [fields[i]])
+        views = (many.stress_view(got[0], i), many.field_view(got[1], i), many.observable_view(got[2], i, "rho"),
+                 many.observable_view(got[3], i, "rotation"))
+        for a, w in zip(views, want):
+            assert torch.equal(a.reshape(-1), w), s
