@@ -120,7 +120,7 @@ __device__ __forceinline__ void tile_async_load(V* dst, const V* src, long long 
     int valid = wv - w;
     valid = valid < 0 ? 0 : (valid > PER ? PER : valid);
     const int rstep = nt >> cl;
-    if (rstep <= 0) return;   // launches use 256 threads and at most 64 columns: never taken
+    if (rstep <= 0) return;   // launches use 128 threads or more and at most 64 columns: never taken
     int e = tid >> cl;
     const V* g = valid ? src + (long long)e * stride + w : src;
     const long long gstep = valid ? (long long)rstep * stride : 0;
@@ -938,6 +938,7 @@ struct PlanCore {
     bool any_vac = false;            // some instance has vacancy coupling
     int rows_tier = 1;               // row passes: 0 every instance register-resident (rows_io_plan), 2 some BIG passes, else 1
     bool big_mid = false, big_green = false;   // some instance's middle / first axis takes BIG passes
+    bool engine_mid = false, engine_green = false;   // or is one of mid_engine's / green_engine's
     bool green_lean = false;         // every instance's k-space pass can run its lean form (green_plan_lean)
     void* d_vac = nullptr;           // caller's vacancy concentrations (cdd_set_vacancy), field_elems / 9
     void* d_vtr = nullptr;           // trace of beta^P at the step start (vacancy instances), field_elems / 9
@@ -1074,8 +1075,20 @@ size_t stencil_smem_bytes(int precision, bool any3d);
 int stencil_default_planes(const InstDev* insts, int n, int precision, int sms);
 void stencil_geometry(InstDev& I, int precision, int planes);
 cudaError_t stress_set_attributes(int precision, size_t max_smem);
-// Axis-1 pass: 128-byte row segments (16 columns FP32, 8 FP64), one radix-16 butterfly per thread at 256.
-__host__ __device__ constexpr int mid_threads(size_t elt) { return elt == 4 ? 256 : 128; }
+// Axis-1 pass: 128-byte row segments (16 columns FP32, 8 FP64), one radix-16 butterfly per thread at 256. engine: an FP64
+// plan with an axis-1 length of the runtime stage engine (see k_fft_mid).
+__host__ __device__ constexpr int mid_threads(size_t elt, bool engine) { return elt == 4 || engine ? 256 : 128; }
+// Lengths of the stage engine (no two-pass form: 288, 512, 576, 640, 768, 800, 864, 972, 1000, 1024; others at radix 4 and
+// 8) that the axis-1 and the k-space pass run on kernels of their own, long ones, whose tiles leave an SM few blocks;
+// see k_fft_mid and k_green.
+__host__ __device__ inline bool line_512(const LinePlan& lp) { return lp.nst == 3 && lp.radix[0] == 16 && lp.radix[1] == 8 && lp.radix[2] == 4; }
+inline bool line_1024(const LinePlan& lp) {
+    return lp.nst == 3 && lp.radix[0] == 16 && lp.radix[1] == 16 && lp.radix[2] == 4;
+}
+inline bool mid_engine(const LinePlan& lp, size_t elt) {
+    return elt == 8 && !lp.pa && lp.n > 256 && !line_512(lp) && !line_1024(lp);
+}
+inline bool green_engine(const LinePlan& lp, size_t elt) { return !lp.pa && (elt == 8 ? lp.n > 256 : line_512(lp)); }
 __host__ __device__ constexpr int row_threads_max(size_t elt) { return elt == 4 ? 256 : 128; }   // row passes
 __host__ __device__ inline int mid_buffers(const LinePlan& lp) { return (line_plan_io(lp) || lp.pa) ? 1 : 2; }
 // Component counts of the k-space pass per mode (see contract_tile).
@@ -1100,6 +1113,7 @@ int green_cols(const InstDev& I, int sms, size_t velt);
 int green_threads(const InstDev& I, size_t velt);
 size_t green_smem_bytes(const InstDev& I, int W, int slots, size_t velt);
 bool green_plan_lean(const LinePlan& lp);
+inline bool green_tier3(const PlanCore& P) { return P.engine_green && !P.big_green; }
 // Fused plane passes of the stress solve (stress.cu): whether instance I can take them and their
 // shared memory per block.
 bool plane_eligible(const InstDev& I, int precision, size_t smem_limit);

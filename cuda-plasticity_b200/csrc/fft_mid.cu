@@ -10,7 +10,7 @@ namespace cdd {
 // One column tile: W = 2^lgw columns of N = n1 elements from base (row pitch nhp), wv of them valid.
 // The kernel calls it with lgw as a literal for the usual tile widths, so that every shared-memory
 // offset of the stages folds to a constant.
-template <typename T, bool INV, bool BIG>
+template <typename T, bool INV, int TIER>
 __device__ __forceinline__ void fft_mid_tile(const InstDev& I, typename VecOf<T>::type* s,
                                              typename VecOf<T>::type* base,
                                              const typename VecOf<T>::type* __restrict__ tws, int lgw, int wv,
@@ -30,8 +30,8 @@ __device__ __forceinline__ void fft_mid_tile(const InstDev& I, typename VecOf<T>
         const LinePlan& lp = I.lp_mid;
         __syncthreads();
         const Cols<V> g{base, 0, wv}, t{s, 0, W};
-        col_pass_a<V, INV, BIG ? 2 : 1>(g, nhp, (long long)lp.B * nhp, t, (long long)lp.A << lgw, W, W, lgw, lp, tws, tid, nt);
-        col_pass_b<V, INV, BIG ? 2 : 1>(t, W, (long long)lp.A << lgw, g, nhp, (long long)lp.A * nhp, W, lgw, lp, tws, tid, nt);
+        col_pass_a<V, INV, TIER == 1 ? 1 : 2>(g, nhp, (long long)lp.B * nhp, t, (long long)lp.A << lgw, W, W, lgw, lp, tws, tid, nt);
+        col_pass_b<V, INV, TIER == 1 ? 1 : 2>(t, W, (long long)lp.A << lgw, g, nhp, (long long)lp.A * nhp, W, lgw, lp, tws, tid, nt);
         return;
     }
     if (W * (int)sizeof(V) >= 16) {
@@ -60,8 +60,11 @@ __device__ __forceinline__ void fft_mid_tile(const InstDev& I, typename VecOf<T>
     }
 }
 
-template <typename T, bool INV, bool BIG>
-__global__ void __launch_bounds__(mid_threads(sizeof(T)), BIG ? 3 : 4)
+// TIER 1: two-pass forms of at most 16 values a pass; 2: all of them; 3 (FP64): the same on 256 threads instead of 128,
+// for plans with long axis-1 lines of the runtime stage engine (mid_engine), whose tiles of two buffers leave room for few blocks (288
+// points, 64x288x256: 198 -> 178 us a pass; the compile-time stages of 512 points prefer 128: 270 us against 279).
+template <typename T, bool INV, int TIER>
+__global__ void __launch_bounds__(mid_threads(sizeof(T), TIER == 3), TIER == 1 ? 4 : (TIER == 2 ? 3 : 2))
 k_fft_mid(const InstDev* __restrict__ insts, int n_inst,
                                                  const int* __restrict__ pre,
                                                  typename VecOf<T>::type* spec,
@@ -88,21 +91,26 @@ k_fft_mid(const InstDev* __restrict__ insts, int n_inst,
     if (c >= ncomp) return;   // launch sized for more components than this pass carries
     if (vac_only && !I.vacancy) return;
     V* base = spec + I.spoff + ((long long)c * I.n0 + i0) * (long long)N * nhp + col0;
-    if (lgw == 4) fft_mid_tile<T, INV, BIG>(I, s, base, tws, 4, wv, tid, nt);
-    else if (lgw == 3) fft_mid_tile<T, INV, BIG>(I, s, base, tws, 3, wv, tid, nt);
-    else fft_mid_tile<T, INV, BIG>(I, s, base, tws, lgw, wv, tid, nt);
+    if (lgw == 4) fft_mid_tile<T, INV, TIER>(I, s, base, tws, 4, wv, tid, nt);
+    else if (lgw == 3) fft_mid_tile<T, INV, TIER>(I, s, base, tws, 3, wv, tid, nt);
+    else fft_mid_tile<T, INV, TIER>(I, s, base, tws, lgw, wv, tid, nt);
 }
 
 template <typename T, bool INV>
 static void mid_t(const PlanCore& P, const LaunchShape& L, int ncomp, int vac_only, cudaStream_t st) {
     typedef typename VecOf<T>::type V;
     const int pass = INV ? PASS_MID_I : PASS_MID_F;
-    if (P.big_mid)
-        launch_pdl(k_fft_mid<T, INV, true>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, (V*)P.d_spec, (const V*)P.d_tw,
-                                                                     pass, ncomp, vac_only);
-    else
-        launch_pdl(k_fft_mid<T, INV, false>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, (V*)P.d_spec, (const V*)P.d_tw,
-                                                                      pass, ncomp, vac_only);
+#define CDD_LAUNCH_M(TIER) launch_pdl(k_fft_mid<T, INV, TIER>, L.blocks, L.threads, L.smem, st, P.d_inst, P.n_inst, L.d_pre, \
+        (V*)P.d_spec, (const V*)P.d_tw, pass, ncomp, vac_only)
+    if constexpr (sizeof(T) == 8) {
+        if (P.engine_mid) {
+            CDD_LAUNCH_M(3);
+            return;
+        }
+    }
+    if (P.big_mid) CDD_LAUNCH_M(2);
+    else CDD_LAUNCH_M(1);
+#undef CDD_LAUNCH_M
 }
 
 void launch_mid(const PlanCore& P, const LaunchShape& L, bool inv, int ncomp, int vac_only, cudaStream_t st) {
@@ -119,10 +127,14 @@ void launch_mid(const PlanCore& P, const LaunchShape& L, bool inv, int ncomp, in
 template <typename T>
 static cudaError_t mid_attr(size_t smem) {
     cudaError_t e;
-    if ((e = set_dyn_smem_limit(k_fft_mid<T, true, false>, smem))) return e;
-    if ((e = set_dyn_smem_limit(k_fft_mid<T, false, false>, smem))) return e;
-    if ((e = set_dyn_smem_limit(k_fft_mid<T, true, true>, smem))) return e;
-    return set_dyn_smem_limit(k_fft_mid<T, false, true>, smem);
+#define CDD_ATTR_M(TIER)                                                               \
+    if ((e = set_dyn_smem_limit(k_fft_mid<T, true, TIER>, smem))) return e;            \
+    if ((e = set_dyn_smem_limit(k_fft_mid<T, false, TIER>, smem))) return e;
+    CDD_ATTR_M(1)
+    CDD_ATTR_M(2)
+    if constexpr (sizeof(T) == 8) { CDD_ATTR_M(3) }
+#undef CDD_ATTR_M
+    return cudaSuccess;
 }
 cudaError_t mid_set_attributes(int precision, size_t smem) {
     return precision == CDD_F32 ? mid_attr<float>(smem) : mid_attr<double>(smem);

@@ -440,8 +440,12 @@ __device__ __noinline__ void mean_block(const InstDev& I, int ii, int c, const M
 // us instead of 332).
 // Four block barriers, no scratch slots and one butterfly per thread and pass at 256 (12 lines FP64, 24 FP32,
 // on 192 threads). Bound by the latency of its phases and, at FP64, the FP64 pipe.
+// TIER 0: every instance's passes are one stage each; 1: of at most 16 values; 2: all two-pass forms; 3: as 1, for plans
+// with long lines of the stage engine (green_engine): FP64 on 256 threads instead of 192 (their slots leave an SM one or
+// two blocks), and 512-point lines leave by their last stage (288 points, 288x64x256 FP64: 484 -> 438 us; 512 points,
+// 512x128x128: FP64 964 -> 786, FP32 441 -> 390).
 template <typename T, int TIER>
-__global__ void __launch_bounds__(sizeof(T) == 4 ? 256 : 192, (TIER == 2 && sizeof(T) == 8) ? 2 : 3)
+__global__ void __launch_bounds__(sizeof(T) == 4 || TIER == 3 ? 256 : 192, (TIER >= 2 && sizeof(T) == 8) ? 2 : 3)
 k_green(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ pre, int gmode, int mean64, MeanArgs mean,
         typename VecOf<T>::type* spec, const typename VecOf<T>::type* __restrict__ tw,
         const T* __restrict__ ktab, typename VecOf<T>::type* phi, double* part,
@@ -477,6 +481,7 @@ k_green(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ p
     const int nin = green_nin(gmode), nout = green_nout(gmode), slots = nin > nout ? nin : nout;
     const LinePlan& lp = I.lp_first;
     const bool two = TIER == 0 || lp.pa != 0;
+    constexpr int PT = TIER == 3 ? 1 : TIER;   // the two-pass forms compiled in
     V* scratch = s + slots * cs;
     V* tws = s + (((two ? slots : slots + 3) * cs + 1) & ~1);   // twiddle rows after the slots
     stage_tw_to_smem(lp, tw, tws, tid, nt);
@@ -484,17 +489,21 @@ k_green(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ p
     const Cols<V> glob{base, cstride, wv}, slot{s, cs, W};
     if (two) {
         __syncthreads();
-        col_pass_a<V, false, TIER>(glob, estride, lp.B * estride, slot, (long long)lp.A << lgw, W, nin << lgw, lgw, lp, tws,
+        col_pass_a<V, false, PT>(glob, estride, lp.B * estride, slot, (long long)lp.A << lgw, W, nin << lgw, lgw, lp, tws,
                                    tid, nt);
-        col_pass_b<V, false, TIER>(slot, W, (long long)lp.A << lgw, slot, W, (long long)lp.A << lgw, nin << lgw, lgw, lp, tws,
+        col_pass_b<V, false, PT>(slot, W, (long long)lp.A << lgw, slot, W, (long long)lp.A << lgw, nin << lgw, lgw, lp, tws,
                                    tid, nt);
     } else if constexpr (TIER != 0) {
         if (W * (int)sizeof(V) >= 16) {
 #pragma unroll 1
             for (int c = 0; c < nin; ++c) tile_async_load(s + c * cs, base + c * cstride, estride, N, lgw, wv, tid, nt);
         } else {
+            // 8-byte columns (W = 1, FP32)
 #pragma unroll 1
-            for (int i = tid; i < nin * N; i += nt) s[(i / N) * cs + i % N] = base[(i / N) * cstride + (i % N) * estride];
+            for (int c = 0; c < nin; ++c) {
+#pragma unroll 8
+                for (int i = tid; i < N; i += nt) s[c * cs + i] = base[c * cstride + i * estride];
+            }
         }
         cp_async_wait_all();
         __syncthreads();
@@ -539,11 +548,25 @@ k_green(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ p
     }
     __syncthreads();
     if (two) {
-        col_pass_a<V, true, TIER>(slot, W, (long long)lp.B << lgw, slot, W, (long long)lp.B << lgw, nout << lgw, lgw, lp, tws,
+        col_pass_a<V, true, PT>(slot, W, (long long)lp.B << lgw, slot, W, (long long)lp.B << lgw, nout << lgw, lgw, lp, tws,
                                   tid, nt);
-        col_pass_b<V, true, TIER>(slot, (long long)lp.B << lgw, W, glob, estride, lp.A * estride, nout << lgw, lgw, lp, tws,
+        col_pass_b<V, true, PT>(slot, (long long)lp.B << lgw, W, glob, estride, lp.A * estride, nout << lgw, lgw, lp, tws,
                                   tid, nt);
     } else if constexpr (TIER != 0) {
+        if constexpr (TIER == 3) {
+            if (nout > 1 && line_512(lp)) {
+                // 512 points: the last stage writes global memory (an odd stage count would end in the scratch slots)
+                const SColT<V, 3> x{scratch, lgw, cs};
+#pragma unroll 1
+                for (int c = 0; c < nout; c += 3) {
+                    const SColT<V, 3> slots3{s + c * cs, lgw, cs};
+                    const GColT<V, 3> out{base + c * cstride, estride, cstride, lgw, wv};
+                    fft_io_c<V, true, 3, SColT<V, 3>, GColT<V, 3>, 1, 16, 8, 4>(slots3, x, slots3, out, lgw, lp, tws, tid, nt,
+                                                                               lp.twst[0], 0);
+                }
+                return;
+            }
+        }
         if (nout == 1) fft_slots<V, true, 1>(s, nout, scratch, lgw, cs, lp, tws, tid, nt);
         else fft_slots<V, true, 3>(s, nout, scratch, lgw, cs, lp, tws, tid, nt);
         if (W * (int)sizeof(V) >= 16) {
@@ -551,7 +574,10 @@ k_green(const InstDev* __restrict__ insts, int n_inst, const int* __restrict__ p
             for (int c = 0; c < nout; ++c) tile_store(base + c * cstride, s + c * cs, estride, N, lgw, wv, tid, nt);
         } else {
 #pragma unroll 1
-            for (int i = tid; i < nout * N; i += nt) base[(i / N) * cstride + (i % N) * estride] = s[(i / N) * cs + i % N];
+            for (int c = 0; c < nout; ++c) {
+#pragma unroll 4
+                for (int i = tid; i < N; i += nt) base[c * cstride + i * estride] = s[c * cs + i];
+            }
         }
     }
 }
@@ -560,7 +586,7 @@ template <typename T>
 static void green_t(const PlanCore& P, const LaunchShape& L, int gmode, bool mean64, const void* ktab, void* phi, double* part,
                     cudaStream_t st) {
     typedef typename VecOf<T>::type V;
-    const int tier = (P.green_lean && gmode <= 1) ? 0 : (P.big_green ? 2 : 1);
+    const int tier = green_tier3(P) ? 3 : (P.green_lean && gmode <= 1) ? 0 : (P.big_green ? 2 : 1);
     const size_t smem = L.smem + (gmode == 1 ? 96 : 0);   // the block sums of the adjoint mode
     const MeanArgs mean{mean64 ? 6 * P.n_inst : 0, P.d_rowsum, P.d_sbar};
 #define CDD_LAUNCH_G(TIER)                                                                                               \
@@ -568,7 +594,8 @@ static void green_t(const PlanCore& P, const LaunchShape& L, int gmode, bool mea
                mean, (V*)P.d_spec, (const V*)P.d_tw, (const T*)ktab, (V*)phi, part, P.d_clock)
     if (tier == 0) CDD_LAUNCH_G(0);
     else if (tier == 1) CDD_LAUNCH_G(1);
-    else CDD_LAUNCH_G(2);
+    else if (tier == 2) CDD_LAUNCH_G(2);
+    else CDD_LAUNCH_G(3);
 #undef CDD_LAUNCH_G
 }
 
@@ -589,7 +616,7 @@ int green_cols(const InstDev& I, int sms, size_t velt) {
     return W;
 }
 // Threads: FP32 tiles of long lines (three blocks per SM) run on 256 (256^3 stress solve 1196 us against 1259 on
-// 192), others on 192 (64^3 64 us against 79).
+// 192), others on 192 (64^3 64 us against 79). TIER 3 runs on 256.
 int green_threads(const InstDev& I, size_t velt) { return velt == 8 && I.n0 >= 192 ? 256 : 192; }
 
 size_t green_smem_bytes(const InstDev& I, int W, int slots, size_t velt) {
@@ -603,6 +630,7 @@ static cudaError_t green_attr(size_t smem) {
     cudaError_t e;
     if ((e = set_dyn_smem_limit(k_green<T, 0>, smem))) return e;
     if ((e = set_dyn_smem_limit(k_green<T, 1>, smem))) return e;
+    if ((e = set_dyn_smem_limit(k_green<T, 3>, smem))) return e;
     return set_dyn_smem_limit(k_green<T, 2>, smem);
 }
 cudaError_t green_set_attributes(int precision, size_t smem) {

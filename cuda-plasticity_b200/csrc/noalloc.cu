@@ -197,6 +197,8 @@ extern "C" int cdd_stress_noalloc(const cdd_instance* d, int precision, const vo
     P.any3d = (I.nd == 3);
     P.big_mid = (I.nd == 3) && pass_big(I.lp_mid);
     P.big_green = pass_big(I.lp_first);
+    P.engine_mid = I.nd == 3 && mid_engine(I.lp_mid, elt);
+    P.engine_green = green_engine(I.lp_first, elt);
     const int sms = device_sms();
     size_t smem_need = 48 * 1024;
     int blocks[NUM_PASSES] = {0, 0, 0, 0, 0};
@@ -215,14 +217,14 @@ extern "C" int cdd_stress_noalloc(const cdd_instance* d, int precision, const vo
     }
     for (int k : {PASS_MID_F, PASS_MID_I}) {
         PassTile& t = I.tile[k];
-        P.pass[k].threads = mid_threads(elt);
+        P.pass[k].threads = mid_threads(elt, P.engine_mid);
         if (I.nd != 3) continue;
         const int comps = 6;
         int W = (int)(128 / velt);
         while (W > 1 && 2 * (size_t)W * I.n1 * velt > 96 * 1024) W >>= 1;
         t.lines = W;
         while ((1 << t.lgw) < W) ++t.lgw;
-        t.threads = mid_threads(elt);
+        t.threads = mid_threads(elt, P.engine_mid);
         t.tiles_a = (I.nh + W - 1) / W;
         t.blocks = comps * I.n0 * t.tiles_a;
         P.pass[k].smem = mid_buffers(I.lp_mid) * (size_t)W * I.n1 * velt +
@@ -235,7 +237,7 @@ extern "C" int cdd_stress_noalloc(const cdd_instance* d, int precision, const vo
             return err(CDD_ERR_SHAPE, "cdd_stress_noalloc: axis-0 length too large for the k-space pass");
         t.lines = W;
         while ((1 << t.lgw) < W) ++t.lgw;
-        t.threads = green_threads(I, velt);
+        t.threads = green_tier3(P) ? 256 : green_threads(I, velt);
         t.tiles_a = (I.nh + W - 1) / W;
         t.blocks = (I.nd == 3 ? I.n1 : 1) * t.tiles_a;
         P.pass[PASS_GREEN].threads = t.threads;

@@ -235,10 +235,11 @@ int build_shapes(cdd_plan* p, size_t elt) {
             const size_t lim = bufs * (size_t)W * I.n1 * velt + (size_t)I.lp_mid.twvalues * velt;
             if (lim > smem_lim[k]) smem_lim[k] = lim;
             C.big_mid |= pass_big(I.lp_mid);
+            C.engine_mid |= mid_engine(I.lp_mid, elt);
             t.lines = W;
             t.lgw = 0;
             while ((1 << t.lgw) < W) ++t.lgw;
-            t.threads = mid_threads(elt);
+            t.threads = mid_threads(elt, mid_engine(I.lp_mid, elt));
             t.tiles_a = (I.nh + W - 1) / W;
             t.blocks = comps * I.n0 * t.tiles_a;
             size_t sm = mid_buffers(I.lp_mid) * (size_t)W * I.n1 * velt + (size_t)I.lp_mid.twspan * velt;
@@ -269,6 +270,7 @@ int build_shapes(cdd_plan* p, size_t elt) {
             if (lim > smem_lim[PASS_GREEN]) smem_lim[PASS_GREEN] = lim;
             lean &= green_plan_lean(I.lp_first);
             C.big_green |= pass_big(I.lp_first);
+            C.engine_green |= green_engine(I.lp_first, elt);
         }
         for (int k = 0; k < NUM_PASSES; ++k) pre[k].push_back(pre[k].back() + I.tile[k].blocks);
         {
@@ -328,11 +330,12 @@ int build_shapes(cdd_plan* p, size_t elt) {
                 return fail(CDD_ERR_ARG, "launch shapes need %zu bytes of shared memory in FFT pass %d (limit %d)",
                             std::max(smem_lim[k], smem_max[k]), k, optin);
     }
+    if (green_tier3(C)) thr_max[PASS_GREEN] = 256;
     size_t smem_all = 0;
     for (int k = 0; k < NUM_PASSES; ++k) {
         LaunchShape& L = C.pass[k];
         L.blocks = pre[k].back();
-        L.threads = (k == PASS_MID_F || k == PASS_MID_I) ? mid_threads(elt) : thr_max[k];
+        L.threads = (k == PASS_MID_F || k == PASS_MID_I) ? mid_threads(elt, C.engine_mid) : thr_max[k];
         L.smem = smem_max[k];
         if (L.smem > smem_all) smem_all = L.smem;
         CDD_CUDA(dalloc(p, (void**)&L.d_pre, sizeof(int) * (n + 1)));
