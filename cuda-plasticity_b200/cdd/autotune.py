@@ -5,9 +5,12 @@ For one grid shape and precision it builds plans with candidate ``cdd_tuning`` v
 keeps the fastest. The search is a coordinate descent from the built-in rule: one knob at a time,
 the others held at their current best, over a few sweeps until nothing improves. Results are cached
 in a JSON file (``CDD_TUNE_CACHE``, default ``~/.cache/cdd_tune.json``) keyed by GPU name,
-precision and shape, so a shape is tuned once per GPU model. No knob changes the mathematics:
+precision, the kernels' variant (glide-only, vacancies, Lambda), shape and library build, so a shape is
+tuned once per GPU model and build: shapes timed with other kernels are not used. No knob changes the mathematics:
 results agree with the built-in shapes to rounding (different radix orders round differently).
 """
+import functools
+import hashlib
 import json
 import os
 
@@ -24,6 +27,19 @@ def cache_path():
 
 def cache_key(gpu, precision, shape):
     return "%s|%s|%s" % (gpu, precision, "x".join(str(int(n)) for n in shape))
+
+
+@functools.lru_cache(maxsize=None)
+def library_tag():
+    """A short digest of the built library, the kernels that a cached timing belongs to."""
+    with open(_lib.LIB_PATH, "rb") as f:
+        return hashlib.blake2b(f.read(), digest_size=8).hexdigest()
+
+
+def variant(inst):
+    """The parts of an instance that select other kernels, as a suffix of the key's precision."""
+    return ("-glide" if inst.glide_only else "") + ("-vacancy" if inst.vacancy is not None else "") + \
+        ("-lambda" if inst.Lambda != 0.0 else "")
 
 
 def load_cache(path=None):
@@ -89,7 +105,7 @@ def tune(inst, precision, reps=5, sweeps=2, verbose=False):
     from .engine import Instance, Plan
     from .initial import gaussian_random_field_torch
     one = Instance(tuple(inst.shape), mu=inst.mu, nu=inst.nu, Lambda=inst.Lambda, cfl=inst.cfl,
-                   load_rate=inst.load_rate, glide_only=inst.glide_only)
+                   load_rate=inst.load_rate, glide_only=inst.glide_only, vacancy=inst.vacancy)
     field = gaussian_random_field_torch(tuple(inst.shape), 0.04, 0.05, 7, device="cuda")
     tried = {}
 
@@ -103,6 +119,8 @@ def tune(inst, precision, reps=5, sweeps=2, verbose=False):
             tried[key] = (None, None)
             return tried[key]
         beta = plan.pack([field])
+        if one.vacancy is not None:
+            plan.set_vacancy(plan.empty_vacancy())
         ms = _time_steps(plan, beta, reps)
         eff = plan.tuning(0)
         plan.close()
@@ -135,13 +153,15 @@ def best(inst, precision, use_cache=True, verbose=False):
     """The tuned launch shapes of inst (a cdd.Instance) at precision, from the cache or by tuning."""
     import torch
     gpu = torch.cuda.get_device_name()
-    key = cache_key(gpu, precision + ("-glide" if inst.glide_only else ""), inst.shape)
+    stem = cache_key(gpu, precision + variant(inst), inst.shape)
+    key = "%s|%s" % (stem, library_tag())
     cache = load_cache() if use_cache else {}
     if key in cache:
         return dict(cache[key]["tuning"])
     t, ms, base_ms, _ = tune(inst, precision, verbose=verbose)
     if use_cache:
-        cache = load_cache()
+        # the entries of other builds for this shape go
+        cache = {k: v for k, v in load_cache().items() if k != stem and not k.startswith(stem + "|")}
         cache[key] = {"tuning": t, "ms_per_step": ms, "builtin_ms_per_step": base_ms}
         try:
             save_cache(cache)

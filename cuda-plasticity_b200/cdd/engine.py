@@ -74,7 +74,7 @@ class Plan:
     tuning: None (built-in launch shapes), a list with one dict per instance (keys of
     ``_lib.cdd_tuning``: fft_radix, rows_lines, mid_cols, green_cols, stencil_planes; missing or 0
     keeps the built-in rule), or "auto" (``cdd.autotune`` picks them by timing, cached per GPU,
-    precision and shape).
+    precision, kernel variant, shape and library build).
     """
 
     def __init__(self, instances, precision="f64", device=None, tuning=None):
