@@ -719,7 +719,7 @@ __device__ __forceinline__ void fft_stage_io(const LS& src, const LD& dst, int l
 }
 
 // Stages st, st+1, ... (remaining radices R, Rs..., span NS so far) from `in` to `out`; stage k
-// writes the shared tile x when k is even and y when odd, the last stage writes `out`.
+// writes the shared tile x when k is even and y when odd, the last stage writes `out` (two stages: y unused).
 template <typename V, bool INV, int K, class LIn, class LOut, int NS, int R, int... Rs>
 __device__ __forceinline__ void fft_io_c(const LIn& in, const SColT<V, K>& x, const SColT<V, K>& y, const LOut& out,
                                          int lgw, const LinePlan& lp, const V* __restrict__ twbase, int tid, int nt,
@@ -746,26 +746,22 @@ __device__ __forceinline__ void fft_io_c(const LIn& in, const SColT<V, K>& x, co
 
 // True when lp runs through fft_io (the host sizes shared memory with this).
 __host__ __device__ inline bool line_plan_io(const LinePlan& lp) {
-    const int nst = lp.nst, r0 = lp.radix[0], r1 = lp.radix[1], r2 = lp.radix[2];
-    (void)r2;
+    const int nst = lp.nst, r0 = lp.radix[0], r1 = lp.radix[1];
 #define CDD_IO_TEST(COND, ...) if (COND) return true;
     CDD_IO_SEQS(CDD_IO_TEST)
 #undef CDD_IO_TEST
     return false;
 }
 
-// All stages of lp from `in` to `out` through the shared tiles x, y (y unused by two-stage plans).
-// Returns false, doing nothing, when lp has no compile-time sequence. Every thread of the block
-// must call this; it ends synchronised.
+// Both stages of lp from `in` to `out` through the shared tile x. Returns false, doing nothing, when lp has no
+// compile-time sequence. Every thread of the block must call this; it ends synchronised.
 template <typename V, bool INV, int K, class LIn, class LOut>
-__device__ __forceinline__ bool fft_io(const LIn& in, const SColT<V, K>& x, const SColT<V, K>& y, const LOut& out,
-                                       int lgw, const LinePlan& lp, const V* __restrict__ twbase, int tid, int nt,
-                                       int rebase) {
-    const int nst = lp.nst, r0 = lp.radix[0], r1 = lp.radix[1], r2 = lp.radix[2];
-    (void)r2;
+__device__ __forceinline__ bool fft_io(const LIn& in, const SColT<V, K>& x, const LOut& out, int lgw, const LinePlan& lp,
+                                       const V* __restrict__ twbase, int tid, int nt, int rebase) {
+    const int nst = lp.nst, r0 = lp.radix[0], r1 = lp.radix[1];
 #define CDD_IO_RUN(COND, ...)                                                                               \
     if (COND) {                                                                                             \
-        fft_io_c<V, INV, K, LIn, LOut, 1, __VA_ARGS__>(in, x, y, out, lgw, lp, twbase, tid, nt, rebase, 0); \
+        fft_io_c<V, INV, K, LIn, LOut, 1, __VA_ARGS__>(in, x, x, out, lgw, lp, twbase, tid, nt, rebase, 0); \
         return true;                                                                                        \
     }
     CDD_IO_SEQS(CDD_IO_RUN)

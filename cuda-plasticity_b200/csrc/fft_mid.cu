@@ -21,8 +21,8 @@ __device__ __forceinline__ void fft_mid_tile(const InstDev& I, typename VecOf<T>
     if (line_plan_io(I.lp_mid)) {
         // both stages' other ends in global memory, one shared tile
         const GColT<V, 1> g{base, nhp, 0, lgw, wv};
-        const SColT<V, 1> x{s, lgw, 0}, y{s + N * W, lgw, 0};
-        fft_io<V, INV, 1>(g, x, y, g, lgw, I.lp_mid, tws, tid, nt, I.lp_mid.twst[0]);
+        const SColT<V, 1> x{s, lgw, 0};
+        fft_io<V, INV, 1>(g, x, g, lgw, I.lp_mid, tws, tid, nt, I.lp_mid.twst[0]);
         return;
     }
     if (I.lp_mid.pa) {

@@ -37,7 +37,7 @@ int report_error(int code, const char* msg);   // plan.cu
 
 using namespace cdd;
 
-// Room for the padding of the twiddle rows (tw_pitch; at most 1184 bytes a length).
+// Room for the padding of the twiddle rows (tw_pitch; at most 288 bytes a length at the default radices, 1184 at 8).
 static constexpr size_t TW_PAD_MAX = 4096;
 static __device__ __align__(256) unsigned char g_stress_scratch[CDD_STRESS_NOALLOC_MAX_BYTES + TW_PAD_MAX];
 

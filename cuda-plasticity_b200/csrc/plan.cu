@@ -231,7 +231,7 @@ int build_shapes(cdd_plan* p, size_t elt) {
             int W = (int)(128 / velt);
             while (W > 1 && 2 * (size_t)W * I.n1 * velt > 96 * 1024) W >>= 1;
             if (p->tune[i].mid_cols > 0) W = p->tune[i].mid_cols;
-            const int bufs = (line_plan_io(I.lp_mid) && I.lp_mid.nst == 2) ? 1 : 2;
+            const int bufs = line_plan_io(I.lp_mid) ? 1 : 2;
             const size_t lim = bufs * (size_t)W * I.n1 * velt + (size_t)I.lp_mid.twvalues * velt;
             if (lim > smem_lim[k]) smem_lim[k] = lim;
             C.big_mid |= pass_big(I.lp_mid);
@@ -331,20 +331,17 @@ int build_shapes(cdd_plan* p, size_t elt) {
                             std::max(smem_lim[k], smem_max[k]), k, optin);
     }
     if (green_tier3(C)) thr_max[PASS_GREEN] = 256;
-    size_t smem_all = 0;
     for (int k = 0; k < NUM_PASSES; ++k) {
         LaunchShape& L = C.pass[k];
         L.blocks = pre[k].back();
         L.threads = (k == PASS_MID_F || k == PASS_MID_I) ? mid_threads(elt, C.engine_mid) : thr_max[k];
         L.smem = smem_max[k];
-        if (L.smem > smem_all) smem_all = L.smem;
         CDD_CUDA(dalloc(p, (void**)&L.d_pre, sizeof(int) * (n + 1)));
         CDD_CUDA(cudaMemcpy(L.d_pre, pre[k].data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
         LaunchShape& L9 = C.pass9[k];
         L9.blocks = pre9[k].back();
         L9.threads = L.threads;
         L9.smem = (k == PASS_GREEN) ? smem_green9 : L.smem;
-        if (L9.smem > smem_all) smem_all = L9.smem;
         CDD_CUDA(dalloc(p, (void**)&L9.d_pre, sizeof(int) * (n + 1)));
         CDD_CUDA(cudaMemcpy(L9.d_pre, pre9[k].data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
     }
@@ -371,7 +368,6 @@ int build_shapes(cdd_plan* p, size_t elt) {
         C.rows_tier = rtier;
     }
     C.stencil.blocks = pre_st.back();
-    C.stencil.threads = 256;
     C.stencil.smem = stencil_smem_bytes(C.precision, C.any3d);
     CDD_CUDA(stencil_set_attributes(C.precision, SIZE_MAX));   // device limit (see set_dyn_smem_limit)
     {
@@ -393,7 +389,6 @@ int build_shapes(cdd_plan* p, size_t elt) {
     CDD_CUDA(dalloc(p, (void**)&C.cellwise.d_pre, sizeof(int) * (n + 1)));
     CDD_CUDA(cudaMemcpy(C.cellwise.d_pre, pre_cw.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
     CDD_CUDA(stress_set_attributes(C.precision, SIZE_MAX));   // device limit (see set_dyn_smem_limit)
-    (void)smem_all;
     return CDD_OK;
 }
 

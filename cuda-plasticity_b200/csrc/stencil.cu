@@ -21,7 +21,7 @@
 // into per-axis terms P[d][s] and pair terms C_de[s_d][s_e]. The corner-weighted sum of H
 // contracts to 6 scalars G[d][s] and 18 scalars Q[i][s][l] (sums of w V over the corners with a
 // given sign on one axis). No per-corner H or derivative tensor is formed. The derivatives are
-// computed one tensor column (j) at a time, twice: pass 1 accumulates A, P, C; pass 2 forms rhs.
+// computed once and stay in registers: pass 1 accumulates A, P, C from them, pass 2 forms rhs.
 #include <cudaTypedefs.h>
 
 #include "cdd_internal.cuh"
@@ -733,7 +733,7 @@ template <int MODE>
 __device__ __forceinline__ StageConst stage_const(const InstDev& I, const InstClock& ck, double t_flux) {
     StageConst k;
     // load time: the step-start time in all three stages (FieldMover.py L62, L123, L133); stage 1
-    // runs before the dt kernel advances t, stages 2 and 3 after it (t_stage holds the start).
+    // runs before its last block advances t (step_dt), stages 2 and 3 after it (t_stage holds the start).
     const double tload = (MODE == M_FLUX) ? t_flux : ((MODE == M_STAGE1) ? ck.t : ck.t_stage);
     applied_load(I, tload, k.ld);
     k.dt = ck.dt;
@@ -1442,7 +1442,7 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 // 5-D map per run of consecutive same-shape instances: (x = last axis, y, z = axis 0 (3-D), component,
 // instance of the run); box = one staged plane of all 9 components of one instance, RX x RY cells;
-// out-of-grid coordinates read zeros (patched by the kernel).
+// no copy leaves the grid (tiles whose box does are staged by the threads: march).
 bool encode_stencil_maps(const PlanCore& P, const InstDev* insts, const void* base, StencilMapSet& maps) {
     maps.enabled = 0;
     PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
@@ -1552,8 +1552,8 @@ static int stencil_tiles(const InstDev& I, int precision) {
 // Planes per block (one value for all 3-D instances of a plan). A block costs its planes and about c0 planes'
 // time for its start (flux form at 256^3, planes per block 1 / 2 / 4 / 8 / 24: FP64 2565 / 2107 / 1837 / 1712 /
 // 1649 us, FP32 1589 / 1180 / 982 / 894 / 851 us); two blocks per SM run at once, and a block alone on its SM takes
-// about 0.7 of the time. Many short blocks pay c0 often, few long ones leave SMs idle (small grids) or a tail
-// (a share of a block): the estimate is minimised. At least 8 planes per block whatever the grid, the rule
+// about 0.7 of the time (128 blocks of 4, 8 and 16 planes against 256: FP32 0.72, 0.68, 0.65, FP64 0.83, 0.82, 0.81). Many short blocks pay c0 often, few long ones leave SMs idle (small grids) or a tail
+// (a share of a block, chosen with c0, not measured by itself): the estimate is minimised. At least 8 planes per block whatever the grid, the rule
 // before, gave one 32^3 FP64 flux 32 blocks and 50 us, against 25 us at one plane per block.
 int stencil_default_planes(const InstDev* insts, int n, int precision, int sms) {
     const double c0 = precision == CDD_F32 ? 0.9 : 0.55, tail = precision == CDD_F32 ? 0.2 : 0.4;

@@ -102,7 +102,7 @@ bool plane_eligible(const InstDev& I, int precision, size_t smem_limit) {
     if (I.n1 % (2 * PLANE_C) != 0 || (I.nl / 2) % (2 * PLANE_C) != 0) return false;
     const PlaneGeom g = plane_geom(I, sizeof(float2));
     if (!rows_io_plan(I.lp_last, g.P)) return false;
-    if (!(line_plan_io(I.lp_mid) && I.lp_mid.nst == 2)) return false;
+    if (!line_plan_io(I.lp_mid)) return false;
     return g.total + 1024 <= smem_limit;
 }
 
@@ -256,7 +256,7 @@ k_plane_fwd(const InstDev* __restrict__ insts, int n_inst, const int* __restrict
     }
     cl.sync();   // every half-spectrum bin of the plane is in its owner's S_col
     SColT<V, 1> col{s_col, lgw, 0}, scr{s_line, lgw, 0};
-    fft_io<V, false, 1>(col, scr, scr, col, lgw, I.lp_mid, tw, tid, nt, 0);
+    fft_io<V, false, 1>(col, scr, col, lgw, I.lp_mid, tw, tid, nt, 0);
     V* dst = spec + I.spoff + plane_row * I.nhp;
     for (int e = tid; e < n1 * W; e += nt) {
         const int ky = e >> lgw, w = e & (W - 1);
@@ -325,7 +325,7 @@ k_plane_inv(const InstDev* __restrict__ insts, int n_inst, const int* __restrict
         const PlaneSpecIn<V> in{spec + I.spoff + plane_row * I.nhp + rank * g.W, I.nhp, n1, N / 2, rank == 0};
         const PlaneRowOut<V> rows{s_own, rank * g.W, 31 - __clz(g.Rc), ldo, N / 2, rank == 0};
         SColT<V, 1> scr{s_buf, lgw, 0};
-        fft_io<V, true, 1>(in, scr, scr, rows, lgw, I.lp_mid, tw, tid, nt, 0);
+        fft_io<V, true, 1>(in, scr, rows, lgw, I.lp_mid, tw, tid, nt, 0);
     }
     cl.sync();   // every row of every block's S_own is complete; no block reads the scratch tiles
     {
