@@ -1552,9 +1552,10 @@ static int stencil_tiles(const InstDev& I, int precision) {
 // Planes per block (one value for all 3-D instances of a plan). A block costs its planes and about c0 planes'
 // time for its start (flux form at 256^3, planes per block 1 / 2 / 4 / 8 / 24: FP64 2565 / 2107 / 1837 / 1712 /
 // 1649 us, FP32 1589 / 1180 / 982 / 894 / 851 us); two blocks per SM run at once, and a block alone on its SM takes
-// about 0.7 of the time (128 blocks of 4, 8 and 16 planes against 256: FP32 0.72, 0.68, 0.65, FP64 0.83, 0.82, 0.81). Many short blocks pay c0 often, few long ones leave SMs idle (small grids) or a tail
-// (a share of a block, chosen with c0, not measured by itself): the estimate is minimised. At least 8 planes per block whatever the grid, the rule
-// before, gave one 32^3 FP64 flux 32 blocks and 50 us, against 25 us at one plane per block.
+// about 0.7 of the time (128 blocks of 4, 8 and 16 planes against 256: FP32 0.72, 0.68, 0.65, FP64 0.83, 0.82,
+// 0.81). Many short blocks pay c0 often, few long ones leave SMs idle (small grids) or a tail (a share of a block,
+// chosen with c0, not measured by itself): the estimate is minimised. At least 8 planes per block whatever the grid,
+// the rule before, gave one 32^3 FP64 flux 32 blocks and 50 us, against 25 us at one plane per block.
 int stencil_default_planes(const InstDev* insts, int n, int precision, int sms) {
     const double c0 = precision == CDD_F32 ? 0.9 : 0.55, tail = precision == CDD_F32 ? 0.2 : 0.4;
     const int resident = ST_BLOCKS * sms;
